@@ -829,8 +829,8 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   if (d_logits_in == nullptr && route_fixup_applies(h)) {
     // logits from the tensor-core product: tokens whose pick its rounding could have changed are re-routed
     // from exactly recomputed logits, so the routing is that of correctly rounded fp32 logits
-    rc = launch_route_topk_fixup(h, d_x, d_gate_w, logits, d_bias, T, idx, w,
-                                 reinterpret_cast<int32_t*>(ws + L.off[WS_FIX]), st, &launches);
+    rc = launch_route_fused(h, d_x, d_gate_w, logits, d_bias, T, idx, w,
+                            reinterpret_cast<int32_t*>(ws + L.off[WS_FIX]), st, &launches);
   } else {
     rc = launch_route_topk(h, logits, d_bias, T, idx, w, st);
     launches += 1;

@@ -115,6 +115,8 @@ int launch_route_topk(const Handle* h, const float* logits, const float* bias, i
 size_t route_fix_bytes(int64_t T);
 int launch_route_topk_fixup(const Handle* h, const void* x, const void* gate_w, float* logits, const float* bias,
                             int64_t T, int32_t* idx, float* w, int32_t* fix, cudaStream_t st, int* launches);
+int launch_route_fused(const Handle* h, const void* x, const void* gate_w, float* logits, const float* bias, int64_t T,
+                       int32_t* idx, float* w, int32_t* fix, cudaStream_t st, int* launches);
 size_t plan_ws_bytes(const Handle* h, int64_t T);
 int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expert_lo, int n_exp,
                         int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,

@@ -97,10 +97,14 @@ __device__ __forceinline__ float kth_best_value(const float (&c0)[P], uint32_t g
   return from_ordered_bits(best);
 }
 
-template <int P>
-__device__ __forceinline__ void route_token(const float* __restrict__ logits, const float* __restrict__ bias,
-                                            int64_t t, const RouteParams& rp, int32_t* __restrict__ out_idx,
-                                            float* __restrict__ out_w, int32_t* __restrict__ fix) {
+// Near-ties are listed in `fix` when it is given (route_topk_kernel) or, with FIX_INLINE, returned as this lane's
+// experts in play (route_fused_kernel recomputes them in the same warp; groups are runs of lanes there).
+template <int P, bool FIX_INLINE = false>
+__device__ __forceinline__ uint32_t route_token(const float* logits, const float* __restrict__ bias,
+                                                int64_t t, const RouteParams& rp, int32_t* __restrict__ out_idx,
+                                                float* __restrict__ out_w, int32_t* __restrict__ fix) {
+  const bool detect = FIX_INLINE || fix != nullptr;
+  uint32_t found = 0;
   const int lane = threadIdx.x & 31;
   const int E = rp.E;
   const float NEG_INF = __int_as_float(0xff800000);
@@ -213,7 +217,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
       const uint32_t win = __reduce_min_sync(0xFFFFFFFFu, (open && gkey == best) ? static_cast<uint32_t>(my_g) : 0xFFFFFFFFu);
       gmask |= 1u << win;
     }
-    if (fix != nullptr) {
+    if (detect) {
       const bool kept = my_g >= 0 && ((gmask >> my_g) & 1u);
       group_kept_min = -warp_max_f(kept ? -my_gs : NEG_INF);
       group_open_max = warp_max_f(my_g >= 0 && !kept ? my_gs : NEG_INF);
@@ -255,7 +259,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
     last_owner = owner;
     if (lane == r) { my_idx = static_cast<int>(e_win); my_w = wv; }
   }
-  if (fix != nullptr) {
+  if (detect) {
     last_c = __shfl_sync(0xFFFFFFFFu, last_c, last_owner);
     float next_c = NEG_INF, amax = 0.f;
 #pragma unroll
@@ -307,11 +311,12 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
             if (band || scores) in_play |= 1u << i;
           }
         }
+        if (FIX_INLINE) found = in_play;
         bool full = false;
-        int32_t* pairs = fix + 4 + 2 * rp.T;
+        int32_t* pairs = FIX_INLINE ? nullptr : fix + 4 + 2 * rp.T;
 #pragma unroll
         for (int i = 0; i < P; ++i) {
-          if ((in_play >> i) & 1u) {
+          if (!FIX_INLINE && ((in_play >> i) & 1u)) {
             const int pos = atomicAdd(fix + 2, 1);
             if (pos < rp.pair_cap) {
               pairs[2 * pos] = static_cast<int32_t>(t);
@@ -323,7 +328,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
         }
         whole_row = __any_sync(0xFFFFFFFFu, full);
       }
-      if (lane == 0) {
+      if (!FIX_INLINE && lane == 0) {
         fix[4 + atomicAdd(fix, 1)] = static_cast<int32_t>(t);
         if (whole_row) fix[4 + rp.T + atomicAdd(fix + 1, 1)] = static_cast<int32_t>(t);
       }
@@ -346,6 +351,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
     out_idx[t * rp.k + lane] = my_idx;
     out_w[t * rp.k + lane] = my_w;
   }
+  return found;
 }
 
 template <int P>
@@ -467,7 +473,31 @@ __global__ void __launch_bounds__(256) route_fix_logits_kernel(const __nv_bfloat
   }
 }
 
-// Single logits, the same way: one warp per (token, expert) pair, lanes across H.
+// One logit by one warp, lanes across H: the exact products summed in fp64.
+__device__ __forceinline__ double exact_logit(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                              int vecs, int lane) {
+  const uint4* xr = reinterpret_cast<const uint4*>(x);
+  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+#pragma unroll 4
+  for (int v = lane; v < vecs; v += 32) {
+    const uint4 xv = __ldg(xr + v), wv = __ldg(wr + v);
+    a0 = fma(bf16_lo_f64(xv.x), bf16_lo_f64(wv.x), a0);
+    a1 = fma(bf16_hi_f64(xv.x), bf16_hi_f64(wv.x), a1);
+    a2 = fma(bf16_lo_f64(xv.y), bf16_lo_f64(wv.y), a2);
+    a3 = fma(bf16_hi_f64(xv.y), bf16_hi_f64(wv.y), a3);
+    a0 = fma(bf16_lo_f64(xv.z), bf16_lo_f64(wv.z), a0);
+    a1 = fma(bf16_hi_f64(xv.z), bf16_hi_f64(wv.z), a1);
+    a2 = fma(bf16_lo_f64(xv.w), bf16_lo_f64(wv.w), a2);
+    a3 = fma(bf16_hi_f64(xv.w), bf16_hi_f64(wv.w), a3);
+  }
+  double a = (a0 + a1) + (a2 + a3);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+  return a;
+}
+
+// Single logits, the same way: one warp per (token, expert) pair.
 __global__ void __launch_bounds__(256) route_fix_pairs_kernel(const __nv_bfloat16* __restrict__ x,
                                                               const __nv_bfloat16* __restrict__ gate_w, int H, int E,
                                                               const int32_t* __restrict__ fix, int64_t T, int pair_cap,
@@ -480,25 +510,47 @@ __global__ void __launch_bounds__(256) route_fix_pairs_kernel(const __nv_bfloat1
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
     const int64_t t = pairs[2 * i];
     const int e = pairs[2 * i + 1];
-    const uint4* xr = reinterpret_cast<const uint4*>(x + t * H);
-    const uint4* wr = reinterpret_cast<const uint4*>(gate_w + static_cast<int64_t>(e) * H);
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    for (int v = lane; v < vecs; v += 32) {
-      const uint4 xv = xr[v], wv = wr[v];
-      a0 = fma(bf16_lo_f64(xv.x), bf16_lo_f64(wv.x), a0);
-      a1 = fma(bf16_hi_f64(xv.x), bf16_hi_f64(wv.x), a1);
-      a2 = fma(bf16_lo_f64(xv.y), bf16_lo_f64(wv.y), a2);
-      a3 = fma(bf16_hi_f64(xv.y), bf16_hi_f64(wv.y), a3);
-      a0 = fma(bf16_lo_f64(xv.z), bf16_lo_f64(wv.z), a0);
-      a1 = fma(bf16_hi_f64(xv.z), bf16_hi_f64(wv.z), a1);
-      a2 = fma(bf16_lo_f64(xv.w), bf16_lo_f64(wv.w), a2);
-      a3 = fma(bf16_hi_f64(xv.w), bf16_hi_f64(wv.w), a3);
-    }
-    double a = (a0 + a1) + (a2 + a3);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+    const double a = exact_logit(x + t * H, gate_w + static_cast<int64_t>(e) * H, vecs, lane);
     if (lane == 0) logits[t * E + e] = static_cast<float>(a);
   }
+}
+
+// Routing and the near-tie fix-up in one pass: a block routes 8 tokens, recomputes the logits in play of its close
+// tokens (a warp per logit) and routes those tokens again.  Same logits, picks and weights as the listing kernels
+// above; no lists in memory.  Bound by launches and latency at decode sizes: V2-Lite at 8 tokens spent 23 us in
+// memset, top-k, two fix-up kernels and the second top-k, 8 us now; V3 at 4096 skewed tokens 0.13 -> 0.05 ms, at
+// 65536 tokens beside the de-quantisation 1.30 -> 0.65 ms.
+constexpr int kRouteWarps = 8;
+template <int P>
+__global__ void __launch_bounds__(kRouteWarps * 32) route_fused_kernel(float* logits, const float* __restrict__ bias,
+                                                                       RouteParams rp,
+                                                                       const __nv_bfloat16* __restrict__ x,
+                                                                       const __nv_bfloat16* __restrict__ gate_w, int H,
+                                                                       int32_t* __restrict__ out_idx,
+                                                                       float* __restrict__ out_w) {
+  __shared__ uint16_t pairs[kRouteWarps * kMaxExperts];       // token of the block << 9 | expert
+  __shared__ int n_pairs;
+  static_assert(kMaxExperts == 1 << 9, "pairs are packed for 512 experts");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kRouteWarps, t = t0 + warp;
+  if (threadIdx.x == 0) n_pairs = 0;
+  __syncthreads();
+  uint32_t in_play = 0;
+  if (t < rp.T) in_play = route_token<P, true>(logits, bias, t, rp, out_idx, out_w, nullptr);
+#pragma unroll
+  for (int i = 0; i < P; ++i)
+    if ((in_play >> i) & 1u) pairs[atomicAdd(&n_pairs, 1)] = static_cast<uint16_t>(warp << 9 | (lane * P + i));
+  __syncthreads();
+  const int n = n_pairs;
+  if (n == 0) return;
+  for (int i = warp; i < n; i += kRouteWarps) {
+    const int64_t tok = t0 + (pairs[i] >> 9);
+    const int e = pairs[i] & (kMaxExperts - 1);
+    const double a = exact_logit(x + tok * H, gate_w + static_cast<int64_t>(e) * H, H >> 3, lane);
+    if (lane == 0) logits[tok * rp.E + e] = static_cast<float>(a);
+  }
+  __syncthreads();
+  if (__any_sync(0xFFFFFFFFu, in_play != 0u)) route_token<P>(logits, bias, t, rp, out_idx, out_w, nullptr);
 }
 
 static int route_P(int n_experts) {
@@ -548,6 +600,40 @@ int launch_route_topk_fixup(const Handle* h, const void* x, const void* gate_w, 
 #undef MG_ROUTE_CASE
   MG_CUDA(cudaGetLastError());
   if (launches) *launches += 4;
+  return MG_OK;
+}
+
+// groups (if any) are power-of-two runs of whole lanes, as route_token's fast reduction wants them
+static bool groups_are_lane_runs(const mg_layer_desc& d, int P) {
+  if (d.gating != MG_GATE_SOFTMAX_GROUP_MAX && d.gating != MG_GATE_SIGMOID_NOAUX_TC) return true;
+  const int size = d.n_experts / d.n_group, lanes = size / P;
+  return size % P == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0;
+}
+
+// The same routing for a caller that does not want the lists: one launch instead of five.  Layers whose groups
+// are not lane runs recompute whole rows for a close group selection, which one warp would take too long over;
+// they keep the listing kernels (`fix`: their scratch).
+int launch_route_fused(const Handle* h, const void* x, const void* gate_w, float* logits, const float* bias, int64_t T,
+                       int32_t* idx, float* w, int32_t* fix, cudaStream_t st, int* launches) {
+  if (T == 0) return MG_OK;
+  const mg_layer_desc& d = h->d;
+  const int P = route_P(d.n_experts);
+  if (P == 0 || !groups_are_lane_runs(d, P))
+    return launch_route_topk_fixup(h, x, gate_w, logits, bias, T, idx, w, fix, st, launches);
+  if (T > (0x7fffffff - 64) / 8) { set_error("token count beyond the fix-up list's index range"); return MG_ERR_SHAPE; }
+  const RouteParams rp{d.n_experts, d.top_k, d.n_group, d.topk_group, d.gating, d.norm_topk_prob,
+                       d.routed_scale, route_fix_err(d.hidden), 0, T};
+  const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
+  const __nv_bfloat16* wb = static_cast<const __nv_bfloat16*>(gate_w);
+  const unsigned grid = static_cast<unsigned>((T + kRouteWarps - 1) / kRouteWarps);
+#define MG_ROUTE_CASE(PP) \
+  case PP: route_fused_kernel<PP><<<grid, kRouteWarps * 32, 0, st>>>(logits, bias, rp, xb, wb, d.hidden, idx, w); break
+  switch (P) {
+    MG_ROUTE_CASE(1); MG_ROUTE_CASE(2); MG_ROUTE_CASE(4); MG_ROUTE_CASE(5); MG_ROUTE_CASE(8); MG_ROUTE_CASE(16);
+  }
+#undef MG_ROUTE_CASE
+  MG_CUDA(cudaGetLastError());
+  if (launches) *launches += 1;
   return MG_OK;
 }
 
@@ -685,6 +771,80 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
   }
 }
 
+// The whole plan in one block, for batches of up to kPlanSmallTokens tokens: a bitmap per (32 tokens, expert) gives
+// the counts and the stable ranks, one block scan the offsets.  Same results as the four kernels above, which cost a
+// launch each: 20 -> 8 us at 8 tokens, 23 -> 10 us at 512.  The limit is one token per thread of the block.
+constexpr int kPlanSmallTokens = 1024;
+__global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restrict__ idx, int T, int k, int lo, int n,
+                                                          int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
+                                                          int32_t* __restrict__ pad_offsets,
+                                                          int32_t* __restrict__ dst_row) {
+  extern __shared__ int32_t sm[];
+  __shared__ int32_t warp_o[32], warp_p[32];
+  const int W = (T + 31) >> 5;
+  uint32_t* bm = reinterpret_cast<uint32_t*>(sm);  // [W][n] tokens of the run of 32 that picked e
+  int32_t* wbase = sm + W * n;                     // [W][n] first row of the run's tokens
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < W * n; i += blockDim.x) bm[i] = 0u;
+  __syncthreads();
+  if (tid < T) {
+    for (int j = 0; j < k; ++j) {
+      const int e = idx[tid * k + j] - lo;
+      if (e >= 0 && e < n) atomicOr(&bm[warp * n + e], 1u << lane);
+    }
+  }
+  __syncthreads();
+  int32_t c = 0;
+  if (tid < n) {
+    for (int w = 0; w < W; ++w) {
+      wbase[w * n + tid] = c;
+      c += __popc(bm[w * n + tid]);
+    }
+  }
+  const int32_t cp = (c + kTileM - 1) / kTileM * kTileM;
+  int32_t io = c, ip = cp;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t vo = __shfl_up_sync(0xFFFFFFFFu, io, o), vp = __shfl_up_sync(0xFFFFFFFFu, ip, o);
+    if (lane >= o) { io += vo; ip += vp; }
+  }
+  if (lane == 31) { warp_o[warp] = io; warp_p[warp] = ip; }
+  __syncthreads();
+  if (tid < n) {
+    int32_t bo = 0, bp = 0;
+    for (int i = 0; i < warp; ++i) { bo += warp_o[i]; bp += warp_p[i]; }
+    const int32_t first = bp + ip - cp;
+    counts[tid] = c;
+    offsets[tid] = bo + io - c;
+    pad_offsets[tid] = first;
+    if (tid == n - 1) { offsets[n] = bo + io; pad_offsets[n] = bp + ip; }
+    for (int w = 0; w < W; ++w) wbase[w * n + tid] += first;
+  }
+  __syncthreads();
+  if (tid < T) {
+    const uint32_t lt = (1u << lane) - 1u;
+    for (int j = 0; j < k; ++j) {
+      const int e = idx[tid * k + j] - lo;
+      dst_row[tid * k + j] = e >= 0 && e < n ? wbase[warp * n + e] + __popc(bm[warp * n + e] & lt) : -1;
+    }
+  }
+}
+
+static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo, int n, int32_t* counts,
+                             int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row, cudaStream_t st) {
+  const size_t smem = static_cast<size_t>(2) * ((T + 31) / 32) * n * sizeof(int32_t);
+  static bool done[64];
+  if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[h->device])) {
+    MG_CUDA(cudaFuncSetAttribute(plan_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 2 * (kPlanSmallTokens / 32) * kMaxExperts * static_cast<int>(sizeof(int32_t))));
+    if (h->device >= 0 && h->device < 64) done[h->device] = true;
+  }
+  const int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;
+  plan_small_kernel<<<1, threads, smem, st>>>(idx, T, h->d.top_k, lo, n, counts, offsets, pad_offsets, dst_row);
+  MG_CUDA(cudaGetLastError());
+  return MG_OK;
+}
+
 size_t plan_ws_bytes(const Handle* h, int64_t T) {
   int64_t nblk = (T + kPlanTokens - 1) / kPlanTokens;
   if (nblk < 1) nblk = 1;
@@ -696,6 +856,10 @@ int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expe
                         int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,
                         void* ws, cudaStream_t st, int* launches) {
   const int k = h->d.top_k;
+  if (T > 0 && T <= kPlanSmallTokens) {
+    if (launches) *launches += 1;
+    return launch_plan_small(h, idx, static_cast<int>(T), expert_lo, n_exp, counts, offsets, pad_offsets, dst_row, st);
+  }
   int nblk = static_cast<int>((T + kPlanTokens - 1) / kPlanTokens);
   int32_t* bc = static_cast<int32_t*>(ws);
   if (nblk > 0) {

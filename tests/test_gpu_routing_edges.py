@@ -1,0 +1,59 @@
+"""GPU: the one-block permute plan and the one-pass routing at the edges of their ranges."""
+
+import pytest
+import torch
+
+from oracle import moe_oracle as O
+from tests.util import make_layer
+
+pytestmark = pytest.mark.gpu
+
+
+def _router_only(E, k, H=256, gating=O.GATE_SOFTMAX_GREEDY, n_group=1, topk_group=1):
+    spec = O.LayerSpec(H, 128, E, k, 0, n_group, topk_group, gating, True, 1.0, O.WEIGHT_BF16, O.COMBINE_FP32)
+    g = torch.Generator().manual_seed(3)
+    bias = torch.randn(E, generator=g) * 0.01 if gating == O.GATE_SIGMOID_NOAUX_TC else None
+    return spec, make_layer(spec, O.LayerWeights((torch.randn(E, H, generator=g) * 0.02).to(torch.bfloat16), bias))
+
+
+@pytest.mark.parametrize("E,k", [(8, 2), (64, 6), (512, 16)])
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 256, 1023, 1024, 1025])
+def test_permute_plan_at_the_one_block_limit(built_lib, T, E, k):
+    _, layer = _router_only(E, k)
+    idx = torch.rand(T, E, generator=torch.Generator().manual_seed(T)).topk(k, dim=1).indices
+    counts, offsets, pad, dst = layer.permute_plan(idx.int().cuda())
+    rc, roff, order, _ = O.permute_plan(idx, E)
+    assert torch.equal(counts.cpu().long(), rc) and torch.equal(offsets.cpu().long(), roff)
+    padc = pad.cpu().long()
+    assert torch.equal(padc[1:] - padc[:-1], (rc + 127) // 128 * 128)
+    rank = torch.arange(T * k) - roff[:-1].repeat_interleave(rc)
+    want = torch.empty(T * k, dtype=torch.int64)
+    want[order] = padc[:-1].repeat_interleave(rc) + rank
+    assert torch.equal(dst.cpu().long().view(-1), want)
+
+
+@pytest.mark.parametrize("gating,E,k,n_group,topk_group", [
+    (O.GATE_SOFTMAX_GREEDY, 64, 6, 1, 1), (O.GATE_SOFTMAX_GROUP_MAX, 160, 6, 8, 3),
+    (O.GATE_SIGMOID_NOAUX_TC, 256, 8, 8, 4), (O.GATE_SOFTMAX_GROUP_MAX, 96, 4, 3, 2)])
+@pytest.mark.parametrize("T", [1, 8, 9, 700])
+def test_forward_routes_as_the_staged_call(built_lib, gating, E, k, n_group, topk_group, T):
+    """The forward's picks, weights and recomputed logits are those of the listing kernels, bit for bit; the last
+    configuration's groups are not runs of lanes."""
+    spec = O.LayerSpec(512, 128, E, k, 0, n_group, topk_group, gating, True, 1.0, O.WEIGHT_BF16, O.COMBINE_FP32)
+    _, W = O.make_inputs(spec, 1, 7)
+    layer = make_layer(spec, W)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, 512, generator=g, device="cuda").to(torch.bfloat16)
+    x[T // 2:] = x[0]                                   # repeated tokens, and a few rows that nearly tie
+    x[::3, 1:] = 0
+    idx, w, logits, _ = layer.gate_route(x)
+    layer.forward(x)
+    torch.cuda.synchronize()
+
+    def view(which, shape, dtype):
+        off = layer.workspace_view(which, T) - layer._ws.data_ptr()
+        n = torch.Size(shape).numel() * 4
+        return layer._ws[off:off + n].view(dtype).view(shape)
+    assert torch.equal(view(1, (T, k), torch.int32), idx)
+    assert torch.equal(view(2, (T, k), torch.float32), w)
+    assert torch.equal(view(0, (T, E), torch.float32), logits)
