@@ -30,7 +30,7 @@ def build_sanitized_library(force: bool = False) -> str:
     (-O1 -g).  It is loaded only by the host-side tests, in a process that preloads the sanitizer
     runtimes (select it with MOEGEN_B200_LIB); device code is not instrumented."""
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
-    deps = srcs + [os.path.join(CSRC, "common.cuh"), os.path.join(ROOT, "include", "moegen_b200.h")]
+    deps = srcs + [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "tc.cuh"), os.path.join(ROOT, "include", "moegen_b200.h")]
     if force or _stale(LIB_SANITIZED, deps):
         nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
         cmd = [nvcc, "-std=c++17", "-O1", "-g", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler",
@@ -47,7 +47,7 @@ def build_library(force: bool = False, verbose: bool = False, checked: bool = Fa
     and return kernels read from a table is compared with the buffer's declared rows; a violation is
     recorded in the device status word and the access skipped (select it with MOEGEN_B200_LIB)."""
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
-    deps = srcs + [os.path.join(CSRC, "common.cuh"), os.path.join(ROOT, "include", "moegen_b200.h")]
+    deps = srcs + [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "tc.cuh"), os.path.join(ROOT, "include", "moegen_b200.h")]
     target = LIB_CHECKED if checked else LIB
     if force or _stale(target, deps):
         nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

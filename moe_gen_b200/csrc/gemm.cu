@@ -18,9 +18,7 @@
 //     layout TMA would have produced, then hand it to the MMA warp through an mbarrier;
 //   * every mbarrier wait is bounded; on expiry the kernel records MG_DEV_WAIT_TIMEOUT, all
 //     roles leave their loops, TMEM is freed and the kernel returns.
-#include <cuda_fp8.h>
-
-#include "common.cuh"
+#include "tc.cuh"
 
 namespace mg {
 
@@ -36,16 +34,22 @@ constexpr int GEMM_THREADS = 192;
 constexpr int CONVERT_THREADS = 256;
 constexpr int NUM_BARS = 2 * STAGES + 4 + 2 * B_SLOTS;
 
-template <bool F8B>
+// NARROW: tiles of 32 columns for the router product of few tokens, which is a chain of load latencies: more CTAs
+// and a deeper ring of smaller stages.
+constexpr int BN_NARROW = 32;
+template <bool F8B, bool NARROW = false>
 struct Cfg {
-  static constexpr int STAGE_BYTES = A_BYTES + (F8B ? B8_BYTES : B_BYTES);
-  static constexpr int NS = F8B ? 3 : STAGES;       // W8A16: a stage less, a converted-tile slot more
+  static constexpr int STAGE_BYTES = A_BYTES + (F8B ? B8_BYTES : NARROW ? BN_NARROW * BK * 2 : B_BYTES);
+  static constexpr int NS = F8B ? 3 : NARROW ? 10 : STAGES;       // W8A16: a stage less, a converted-tile slot more
+  static constexpr int BAR_STAGES = NARROW ? NS : STAGES;
+  static constexpr int BARS = 2 * BAR_STAGES + 4 + 2 * B_SLOTS;
   static constexpr int RING_BYTES = NS * STAGE_BYTES + (F8B ? B_SLOTS * B_BYTES : 0);
+  static constexpr size_t CTRL_BYTES = 8 * BARS + 16 + 4 * (2 * kMaxExperts + 2);
+  static constexpr size_t SMEM_BYTES = 1024 + RING_BYTES + CTRL_BYTES + 1024 + 4 * 2 * 2048;
   static constexpr int THREADS = GEMM_THREADS + (F8B ? CONVERT_THREADS : 0);
 };
 constexpr int TMEM_COLS = 512;
 constexpr int ACC_COLS = 256;
-constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
 struct GemmArgs {
   const int32_t* pad_offsets;   // nullptr => dense
@@ -65,144 +69,6 @@ struct GemmArgs {
   int32_t* status;
 };
 
-constexpr size_t SMEM_CTRL_BYTES = 8 * NUM_BARS + 16 + 4 * (2 * kMaxExperts + 2);
-template <bool F8B>
-constexpr size_t gemm_smem_bytes() { return 1024 + Cfg<F8B>::RING_BYTES + SMEM_CTRL_BYTES + 1024 + 4 * 2 * 2048; }
-
-// ---- PTX wrappers ---------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok;
-}
-// nanoseconds; the two halves are read separately and the high half checked, so that a carry of the low
-// half between the reads cannot produce a value that is off by 2^32 ns
-__device__ __forceinline__ unsigned long long global_timer() {
-  uint32_t hi, lo, hi2;
-  do {
-    asm volatile("mov.u32 %0, %%globaltimer_hi;" : "=r"(hi));
-    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(lo));
-    asm volatile("mov.u32 %0, %%globaltimer_hi;" : "=r"(hi2));
-  } while (hi != hi2);
-  return (static_cast<unsigned long long>(hi) << 32) | lo;
-}
-// The limit of a bounded wait has run out.  The 64-bit timer is read as two halves; a read that straddles
-// a carry of the low half can come out far too small or too large, so the difference is taken as a
-// signed number (a reading below t0 never counts) and an expiry must be seen by two readings in a row.
-__device__ __forceinline__ bool timed_out(unsigned long long t0, unsigned long long limit_ns) {
-  const long long d1 = static_cast<long long>(global_timer() - t0);
-  if (d1 <= static_cast<long long>(limit_ns)) return false;
-  const long long d2 = static_cast<long long>(global_timer() - t0);
-  return d2 > static_cast<long long>(limit_ns) && d2 >= d1;
-}
-// Bounded wait.  Returns false if the wait ran out or another role already gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int32_t* status, int where,
-                                          unsigned long long limit_ns = WAIT_LIMIT_NS) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_timer();
-  uint32_t spins = 0;
-  while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 63u) == 0u) {
-      if (*abort_flag) return false;
-      if (timed_out(t0, limit_ns)) {
-        *abort_flag = 1;
-        if (atomicCAS(status, MG_DEV_OK, MG_DEV_WAIT_TIMEOUT) == MG_DEV_OK) status[1] = where;
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-// L2 residency hints for data that is written once and read many times before it is overwritten
-__device__ __forceinline__ uint64_t policy_evict_last() {
-  uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
-}
-__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar,
-                                                 uint64_t pol) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(pol)
-      : "memory");
-}
-__device__ __forceinline__ void st_global_hint16(void* ptr, const uint4& v, uint64_t pol) {
-  asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(ptr), "r"(v.x), "r"(v.y), "r"(v.z),
-               "r"(v.w), "l"(pol)
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                            uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tc_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// K-major, 128B-swizzled operand tile: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);        // start address, 16-byte units
-  d |= static_cast<uint64_t>(1) << 16;                        // leading byte offset (unused here)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                // stride byte offset between 8-row groups
-  d |= static_cast<uint64_t>(1) << 46;                        // descriptor version (Blackwell)
-  d |= static_cast<uint64_t>(2) << 61;                        // SWIZZLE_128B
-  return d;
-}
 
 // ---- tile scheduler -------------------------------------------------------------------
 struct Tile {
@@ -240,23 +106,6 @@ __device__ __forceinline__ Tile locate_tile(int tile, const int* s_pad, const in
   return t;
 }
 
-__device__ __forceinline__ float silu_f(float g) { return __fdividef(g, 1.0f + __expf(-g)); }
-
-// 16 FP8 values -> 16 bf16 (two 16-byte chunks), each bf16(float(q) * s)
-__device__ __forceinline__ void convert16(const uint4& q, float s, uint4& lo, uint4& hi) {
-  const __nv_fp8x2_storage_t* p = reinterpret_cast<const __nv_fp8x2_storage_t*>(&q);
-  uint32_t o[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[i], __NV_E4M3);
-    float2 f = __half22float2(*reinterpret_cast<__half2*>(&hr));
-    __nv_bfloat162 b = __floats2bfloat162_rn(__fmul_rn(f.x, s), __fmul_rn(f.y, s));
-    o[i] = *reinterpret_cast<uint32_t*>(&b);
-  }
-  lo = make_uint4(o[0], o[1], o[2], o[3]);
-  hi = make_uint4(o[4], o[5], o[6], o[7]);
-}
-
 // ---- epilogue ---------------------------------------------------------------------------
 // bf16 outputs leave through shared memory: each epilogue warp owns 32 rows, writes a 32-row x
 // 32-column piece (2 KiB) into one of its two staging buffers and one lane hands it to TMA
@@ -264,13 +113,6 @@ __device__ __forceinline__ void convert16(const uint4& q, float s, uint4& lo, ui
 // instead of 64-byte runs per thread.  Rows of a piece that lie in an expert's padding are
 // written too (they belong to nobody); rows beyond the tensor are clipped by TMA.
 constexpr int EPI_PIECE_BYTES = 32 * 64;                 // 32 rows x 32 bf16
-
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int c0, int c1, uint32_t src) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(c0),
-               "r"(c1), "r"(src)
-               : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
 
 struct EpiWarp {
   uint8_t* stage;      // this warp's staging buffers
@@ -340,16 +182,17 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, const GemmArgs& g,
       send_piece(w, tmC, packed, n_idx * g.bn + c, row_first, warp_live);
     }
   } else {
-    // fp32 output, N = n_per_group columns in one tile (the router logits): direct stores
-    float* orow = static_cast<float*>(g.out) + row * g.ldo;
-    for (int c = 0; c < g.n_per_group; c += 32) {
+    // fp32 output, up to n_per_group columns (the router logits): direct stores
+    const int col0 = n_idx * g.bn, cols = min(g.bn, g.n_per_group - col0);
+    float* orow = static_cast<float*>(g.out) + row * g.ldo + col0;
+    for (int c = 0; c < cols; c += 32) {
       uint32_t r[32];
       tc_ld32(taddr + c, r);
       tc_ld_wait();
       if (live) {
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          if (c + i < g.n_per_group) {
+          if (c + i < cols) {
             float4 v;
             v.x = __uint_as_float(r[i]); v.y = __uint_as_float(r[i + 1]);
             v.z = __uint_as_float(r[i + 2]); v.w = __uint_as_float(r[i + 3]);
@@ -389,27 +232,28 @@ struct TileScales {
   }
 };
 
-template <int EPI, bool F8B>
-__global__ void __launch_bounds__(Cfg<F8B>::THREADS, 1)
+template <int EPI, bool F8B, bool NARROW = false>
+__global__ void __launch_bounds__(Cfg<F8B, NARROW>::THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const GemmArgs g) {
-  constexpr int STAGE_BYTES = Cfg<F8B>::STAGE_BYTES;
-  constexpr int NS = Cfg<F8B>::NS;
+  constexpr int STAGE_BYTES = Cfg<F8B, NARROW>::STAGE_BYTES;
+  constexpr int NS = Cfg<F8B, NARROW>::NS;
+  constexpr int BS = Cfg<F8B, NARROW>::BAR_STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg<F8B>::RING_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg<F8B, NARROW>::RING_BYTES);
   uint64_t* full = bars;
-  uint64_t* empty = bars + STAGES;
-  uint64_t* tfull = bars + 2 * STAGES;
-  uint64_t* tempty = bars + 2 * STAGES + 2;
-  uint64_t* bready = bars + 2 * STAGES + 4;            // converted B tile ready (W8A16)
-  uint64_t* bfree = bars + 2 * STAGES + 4 + B_SLOTS;   // converted B tile consumed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
+  uint64_t* empty = bars + BS;
+  uint64_t* tfull = bars + 2 * BS;
+  uint64_t* tempty = bars + 2 * BS + 2;
+  uint64_t* bready = bars + 2 * BS + 4;            // converted B tile ready (W8A16)
+  uint64_t* bfree = bars + 2 * BS + 4 + B_SLOTS;   // converted B tile consumed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg<F8B, NARROW>::BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* s_pad = reinterpret_cast<int*>(tmem_slot + 4);
   int* s_cnt = s_pad + kMaxExperts + 1;
   uint8_t* epi_stage = reinterpret_cast<uint8_t*>(
-      (reinterpret_cast<uintptr_t>(smem + Cfg<F8B>::RING_BYTES + SMEM_CTRL_BYTES) + 1023) & ~uintptr_t(1023));
+      (reinterpret_cast<uintptr_t>(smem + Cfg<F8B, NARROW>::RING_BYTES + Cfg<F8B, NARROW>::CTRL_BYTES) + 1023) & ~uintptr_t(1023));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -445,7 +289,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       const uint32_t tx_bytes = A_BYTES + static_cast<uint32_t>(g.bn) * BK * (F8B ? 1 : 2);
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
@@ -463,7 +307,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, tcount = 0;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
         const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
@@ -604,45 +448,6 @@ constexpr size_t SMEM2_CTRL_BYTES = 8 * NUM_BARS2 + 16 + 4 * (3 * kMaxExperts + 
 template <bool F8B>
 constexpr size_t gemm2_smem_bytes() { return 1024 + Cfg2<F8B>::RING_BYTES + SMEM2_CTRL_BYTES + 1024 + 4 * 2 * 2048; }
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// both CTAs of the pair issue it; the completion bytes are counted on the leader's barrier
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar & 0xFEFFFFFFu), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-__device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 struct Tile2 {
   int row0;       // first of the pair's 256 rows
   int rows_left;  // rows of the expert from row0 on (may exceed 256)
@@ -753,7 +558,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs) {
         const Tile2 t = locate_tile2(tile, s_pad, s_cnt, s_pp, g.n_groups, g.n_tiles, g.n_per_group);
@@ -776,7 +581,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       uint32_t it = 0, tcount = 0;
       for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs, ++tcount) {
         const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
@@ -996,7 +801,7 @@ grouped_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   if (warp == 0) {
     // ---------------- TMA producer: TM rows of A per k-block, one box ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
         const Tile2 t = locate_w8<TM>(tile, s_pad, s_cnt, s_pp, g);
@@ -1011,7 +816,7 @@ grouped_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, tcount = 0;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
         // a 256-row tile with at most 128 live rows needs its first half only
@@ -1320,7 +1125,7 @@ grouped_gemm_ring_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 
   if (warp == 0) {
     // ---------------- TMA producer: A from the rows, B from the ring ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       int have = -1;                                    // granule already known to be in the ring
       const uint64_t keep = policy_evict_last();
@@ -1347,7 +1152,7 @@ grouped_gemm_ring_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, tcount = 0;
       for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
         const RingTile t = locate_ring(tile, s_pad, s_cnt, s_gb, g, r);
@@ -1554,14 +1359,11 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// bf16 operands land 128B-swizzled (what the UMMA descriptor expects); FP8 bytes land as plain
-// rows of 64 bytes for the converter warps
-// `out_piece`: the 32 x 32 bf16 pieces the epilogue stores (rows of 64 bytes, SWIZZLE_64B in shared memory)
 // A layer calls the same few (pointer, shape) combinations on every forward, so the encoded maps
 // are kept in the handle: a forward at decode sizes is short enough for ~60 driver calls to show.
-static int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
-                     uint32_t box_rows, bool fp8 = false, bool out_piece = false) {
-  const uint32_t kind = (fp8 ? 1u : 0u) | (out_piece ? 2u : 0u);
+int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
+              TensorMapKind kind) {
+  const bool fp8 = kind == TM_FP8_ROWS || kind == TM_FP8_SW128;
   TensorMapCache& c = h->tmaps;
   for (int i = 0; i < c.used; ++i) {
     const TensorMapCache::Entry& e = c.e[i];
@@ -1574,12 +1376,12 @@ static int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64
   MG_REQUIRE(fn != nullptr, MG_ERR_DRIVER, "cuTensorMapEncodeTiled not available from the driver");
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * (fp8 ? 1 : 2)};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(out_piece ? 32 : BK), box_rows};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(kind == TM_OUT_PIECE ? 32 : kind == TM_OUT_16 ? 16 : kind == TM_FP8_SW128 ? 128 : BK), box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  out_piece ? CU_TENSOR_MAP_SWIZZLE_64B
-                            : fp8 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                  kind == TM_OUT_PIECE ? CU_TENSOR_MAP_SWIZZLE_64B
+                  : kind == TM_FP8_ROWS || kind == TM_OUT_16 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   MG_REQUIRE(r == CUDA_SUCCESS, MG_ERR_DRIVER, "cuTensorMapEncodeTiled failed (%d) rows=%llu cols=%llu box=%u",
              static_cast<int>(r), static_cast<unsigned long long>(rows), static_cast<unsigned long long>(cols),
@@ -1601,14 +1403,14 @@ static int allow_smem(K kernel, size_t bytes, int device, bool (&done)[64]) {
   return MG_OK;
 }
 
-template <int EPI, bool F8B>
+template <int EPI, bool F8B, bool NARROW = false>
 static int launch_epi(const Handle* h, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                       const GemmArgs& args, int grid, cudaStream_t st) {
-  constexpr size_t smem = gemm_smem_bytes<F8B>();
+  constexpr size_t smem = Cfg<F8B, NARROW>::SMEM_BYTES;
   static bool done[64];
-  int rc = allow_smem(grouped_gemm_kernel<EPI, F8B>, smem, h->device, done);
+  int rc = allow_smem(grouped_gemm_kernel<EPI, F8B, NARROW>, smem, h->device, done);
   if (rc != MG_OK) return rc;
-  grouped_gemm_kernel<EPI, F8B><<<grid, Cfg<F8B>::THREADS, smem, st>>>(ta, tb, tc, args);
+  grouped_gemm_kernel<EPI, F8B, NARROW><<<grid, Cfg<F8B, NARROW>::THREADS, smem, st>>>(ta, tb, tc, args);
   MG_CUDA(cudaGetLastError());
   return MG_OK;
 }
@@ -1678,12 +1480,12 @@ static int launch_ring_gemm(const Handle* h, const GemmProblem& p, cudaStream_t 
              static_cast<long long>(p.ring_counter_ints), rp.ring_bytes, static_cast<long long>(2 * rp.max_granules));
   MG_REQUIRE(static_cast<long long>(rp.pg) * BN_MAX * (p.K / 16) < (1ll << 31), MG_ERR_LIMIT, "granule too large");
   CUtensorMap ta, tb, tc;
-  int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), BM);
+  int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), BM, TM_BF16);
   if (rc != MG_OK) return rc;
-  rc = encode_2d(h, &tb, p.ring, static_cast<uint64_t>(rp.slots) * rp.pg * BN_MAX, static_cast<uint64_t>(p.K), BN_MAX);
+  rc = encode_2d(h, &tb, p.ring, static_cast<uint64_t>(rp.slots) * rp.pg * BN_MAX, static_cast<uint64_t>(p.K), BN_MAX, TM_BF16);
   if (rc != MG_OK) return rc;
   MG_REQUIRE(p.ldo % 8 == 0, MG_ERR_SHAPE, "output row length %lld must be a multiple of 8", static_cast<long long>(p.ldo));
-  rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32, false, true);
+  rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32, TM_OUT_PIECE);
   if (rc != MG_OK) return rc;
   GemmArgs a;
   a.pad_offsets = p.pad_offsets;
@@ -1728,9 +1530,13 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   MG_REQUIRE(p.n_groups >= 1 && p.n_groups <= kMaxExperts, MG_ERR_SHAPE, "n_groups=%d out of range", p.n_groups);
   int bn;
   const bool f32_out = p.epilogue == EPI_PLAIN_F32 || p.epilogue == EPI_ROUND_BF16_F32;
+  // The router product of few tokens in 32-column tiles while those fit in one wave: at up to 128 tokens one CTA read
+  // all of the router (V3: 3.7 MB) alone.  Same bits; V3 at 64 tokens 53 -> 25 us together with the elected issue.
+  const bool narrow = f32_out && dense && p.n_per_group > BN_NARROW &&
+                      (p.dense_rows + BM - 1) / BM * ((p.n_per_group + BN_NARROW - 1) / BN_NARROW) <= h->sm_count;
   if (f32_out) {
-    bn = static_cast<int>(round_up(p.n_per_group, 16));
-    MG_REQUIRE(bn <= BN_MAX && p.n_groups == 1 && p.n_per_group % 4 == 0, MG_ERR_SHAPE,
+    bn = narrow ? BN_NARROW : static_cast<int>(round_up(p.n_per_group, 16));
+    MG_REQUIRE(p.n_per_group <= BN_MAX && p.n_groups == 1 && p.n_per_group % 4 == 0, MG_ERR_SHAPE,
                "fp32-output GEMM needs one group of <=256 columns (multiple of 4), got %d", p.n_per_group);
   } else {
     bn = BN_MAX;
@@ -1739,7 +1545,7 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   }
   // SM pairs (2-CTA tiles of 256 x 256) for the bf16 expert GEMMs when switched on
   const bool pair = h->opt_pair_gemm && !f32_out;
-  // FP8 weights converted in the kernel (one CTA per SM): 256-row tiles once experts average 120
+  // FP8 weights converted in the kernel, tokens on the lanes (on request): 256-row tiles once experts average 120
   // live rows (a_rows also counts up to 127 rows of padding per expert); below that most tall tiles
   // would be half empty, the layer is bound by streaming the weights from HBM, and the 128-row
   // kernel, whose FP8 bytes arrive by TMA, streams them faster than register loads do
@@ -1747,16 +1553,16 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
                     p.a_rows >= static_cast<int64_t>(p.n_groups) * (h->opt_fp8_m256 == 2 ? 0 : 120 + 127);
   if (p.ring != nullptr) return launch_ring_gemm(h, p, st);
   CUtensorMap ta, tb;
-  int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), m256 ? 2 * BM : BM);
+  int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), m256 ? 2 * BM : BM, TM_BF16);
   if (rc != MG_OK) return rc;
   rc = encode_2d(h, &tb, p.b, static_cast<uint64_t>(p.n_groups) * p.n_per_group, static_cast<uint64_t>(p.K),
-                 pair ? 128 : bn, p.b_fp8);
+                 pair ? 128 : bn, p.b_fp8 ? TM_FP8_ROWS : TM_BF16);
   if (rc != MG_OK) return rc;
   CUtensorMap tc = ta;   // unused by the fp32 epilogue
   if (!f32_out) {
     // output tensor [a_rows, ldo] bf16, written in 32 x 32 pieces
     MG_REQUIRE(p.ldo % 8 == 0, MG_ERR_SHAPE, "output row length %lld must be a multiple of 8", static_cast<long long>(p.ldo));
-    rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32, false, true);
+    rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32, TM_OUT_PIECE);
     if (rc != MG_OK) return rc;
   }
   if (p.b_fp8) {
@@ -1769,7 +1575,7 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   a.counts = p.counts;
   a.n_groups = p.n_groups;
   a.dense_rows = static_cast<int>(p.dense_rows);
-  a.n_tiles = f32_out ? 1 : p.n_per_group / bn;
+  a.n_tiles = (p.n_per_group + bn - 1) / bn;
   a.bn = bn;
   a.n_per_group = p.n_per_group;
   a.k_blocks = p.K / BK;
@@ -1829,8 +1635,12 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
     switch (p.epilogue) {
       case EPI_SWIGLU_BF16: return launch_epi<EPI_SWIGLU_BF16, false>(h, ta, tb, tc, a, grid, st);
       case EPI_PLAIN_BF16: return launch_epi<EPI_PLAIN_BF16, false>(h, ta, tb, tc, a, grid, st);
-      case EPI_PLAIN_F32: return launch_epi<EPI_PLAIN_F32, false>(h, ta, tb, tc, a, grid, st);
-      case EPI_ROUND_BF16_F32: return launch_epi<EPI_ROUND_BF16_F32, false>(h, ta, tb, tc, a, grid, st);
+      case EPI_PLAIN_F32:
+        return narrow ? launch_epi<EPI_PLAIN_F32, false, true>(h, ta, tb, tc, a, grid, st)
+                      : launch_epi<EPI_PLAIN_F32, false>(h, ta, tb, tc, a, grid, st);
+      case EPI_ROUND_BF16_F32:
+        return narrow ? launch_epi<EPI_ROUND_BF16_F32, false, true>(h, ta, tb, tc, a, grid, st)
+                      : launch_epi<EPI_ROUND_BF16_F32, false>(h, ta, tb, tc, a, grid, st);
     }
   }
   set_error("bad epilogue");
