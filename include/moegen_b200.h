@@ -498,9 +498,9 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
 /* MG_OPT_PAIR_GEMM: 1 = the bf16 expert GEMMs run on SM pairs (clusters of two CTAs,
  * tcgen05 cta_group::2, 256x256 tiles); 0 = one CTA per SM, 128x256 tiles. */
 #define MG_OPT_PAIR_GEMM   2
-/* MG_OPT_FP8_M256: tile height of the convert-in-the-GEMM kernels: 0 = 128 rows, 1 (default) =
- * 256 rows (one converted weight tile feeds two MMAs) when experts average at least 120 rows,
- * 2 = always 256. */
+/* MG_OPT_FP8_M256: form of the convert-in-the-GEMM kernels: 1 (default) = weights on the accumulator's
+ * lanes, up to 384 tokens per converted weight; 0 = tokens on the lanes, 128-row tiles; 2 = tokens on the
+ * lanes, 256-row tiles.  Same results. */
 #define MG_OPT_FP8_M256    4
 /* MG_OPT_BATCH_TOKENS: a caller that feeds one batch through mg_moe_forward in chunks sets the
  * batch's total token count here (0 = off, the default); MG_FP8_AUTO then decides on the larger

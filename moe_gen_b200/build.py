@@ -13,7 +13,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libmoegen_b200.so")
 LIB_CHECKED = os.path.join(PKG, "libmoegen_b200_checked.so")     # the same sources with -DMG_BOUNDS_CHECK
 LIB_SANITIZED = os.path.join(PKG, "libmoegen_b200_asan.so")      # host code under ASan + UBSan (tests only)
-SOURCES = ["api.cu", "route.cu", "pack.cu", "gemm.cu", "ep.cu"]
+SOURCES = ["api.cu", "route.cu", "pack.cu", "gemm.cu", "gemm_wl.cu", "ep.cu"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
               "-Xcompiler", "-fPIC", "-shared", "-cudart", "static", "-ldl"]
 

@@ -65,9 +65,9 @@ static size_t dequant_ws(const Handle* h) {
 //               through a ring of a few tens of MB (gemm.cu: grouped_gemm_ring_kernel): 58 MB of scratch
 //               instead of 2 bytes per weight.
 // AUTO: converting in the kernel re-does the work for every row tile of an expert; de-quantising first
-// moves every weight through HBM three more times.  On the DeepSeek-V3 shape the two cost the same near
-// 1024 rows per expert (256-row tiles), measured; below that converting wins by up to 2.7x, above it
-// de-quantising first by up to 12 %.  The ring was built to take the large batches without the HBM round
+// moves every weight through HBM three more times.  On the DeepSeek-V3 shape converting (weights on the lanes,
+// gemm_wl.cu) wins below 1024 rows per expert (512 rows: 13.7 against 16.9 ms a forward); at 2048 rows the two
+// are equal within a box's drift (53.0 and 52.7 ms).  The ring was built to take the large batches without the HBM round
 // trip of the bf16 copy, but L2 does not hold it (measured at the benchmark size: 21.6 GB written to and
 // 35.2 GB read from DRAM by the gate/up launch, i.e. the ring goes through HBM like the separate pass's
 // copy does), and it ends 5 % behind pre-dequantise there; it is chosen only on request.

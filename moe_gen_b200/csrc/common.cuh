@@ -225,6 +225,7 @@ struct RingPlan {
 };
 RingPlan ring_plan(int n_per_group, int K, int64_t a_rows, int n_groups, size_t budget_bytes);
 int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st);
+int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st);     // weights on the lanes (gemm_wl.cu)
 int launch_wait_probe(const Handle* h, int limit_ms, cudaStream_t st);
 
 // the expert FFN with the expert-parallel return pushed from inside it (api.cu)

@@ -1552,6 +1552,11 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   const bool m256 = p.b_fp8 && !pair && !f32_out && !dense && h->opt_fp8_m256 &&
                     p.a_rows >= static_cast<int64_t>(p.n_groups) * (h->opt_fp8_m256 == 2 ? 0 : 120 + 127);
   if (p.ring != nullptr) return launch_ring_gemm(h, p, st);
+  // FP8 weights converted in the kernel, by default with the weights on the lanes: one conversion per 384 tokens of
+  // an expert and MMAs as wide as its rows.  V3 shape, gate/up + down, ms before (128- or 256-row tiles) and now:
+  // 64 tokens 3.3 and 2.3, 4096 skewed tokens 6.9 and 4.9, 16384 tokens 14.1 and 11.6.  MG_OPT_FP8_M256 = 0 or 2
+  // asks for the tiles with tokens on the lanes.
+  if (p.b_fp8 && !dense && !f32_out && !pair && h->opt_fp8_m256 == 1) return launch_gemm_wl(h, p, st);
   CUtensorMap ta, tb;
   int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), m256 ? 2 * BM : BM, TM_BF16);
   if (rc != MG_OK) return rc;

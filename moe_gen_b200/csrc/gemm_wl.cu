@@ -1,0 +1,502 @@
+// W8A16 grouped GEMM with the weights on the accumulator's lanes: D[weight row, token] = W_e[N, K] . X_e[rows, K]^T.
+//
+// A cluster of two CTAs (one SM pair, tcgen05 cta_group::2, M = 256) computes 256 weight rows against up to
+// 384 tokens of one expert.  Compared with tokens on the lanes (gemm.cu):
+//   * the token side is the MMA's N, a multiple of 32 chosen per job, so an expert with few rows costs what it
+//     has and an expert with 130 rows is one job, not two 128-row tiles;
+//   * an FP8 weight is converted once per 384 tokens, by the SM whose lane holds it, and the bf16 operand goes
+//     straight into tensor memory (tcgen05.st; the A operand of the MMA is read from there).  Shared memory
+//     carries the FP8 bytes and the tokens only: per 64-element K step and SM 8 KiB + 8 KiB FP8 in and out and
+//     N/2 * 128 B of tokens in and out, where a bf16 tile built in shared memory adds 16-32 KiB each way.
+//
+// Measured on the DeepSeek-V3 shape, gate/up + down products, tokens on the lanes before and now: 64 tokens 3.3 and
+// 2.3 ms, 333 skewed 3.0 and 2.1, 4096 skewed 6.9 and 4.9, 16384 tokens 14.2 and 11.6; the same bits.  Decode reads
+// 10.0 GB in 2.3 ms, 4.3 TB/s of the measured 6.5: the bound there is the hand-over between converters and MMA
+// issuer, not HBM.  Jobs of 192, 256 and 320 tokens were up to 25 % slower at 2048 rows per expert (more
+// conversions), sixteen converter warps no faster than eight.
+//
+// Roles per CTA: warp 0 = weight TMA, warp 1 = token TMA, warp 2 = MMA issuer (leader CTA), warp 3 = job table and
+// TMEM owner, warps 4-11 = epilogue (two per lane quarter, alternate 32-token chunks), warps 12-19 = converters: a
+// thread owns one lane = one weight row; warps 12-15 take the even 64-element K steps, 16-19 the odd ones.
+//
+// Barriers (per CTA unless said otherwise):
+//   wfull/wempty   weight ring, stages of 128 rows x 128 K bytes, released by the converter warps
+//   tfull/tempty   token ring; leader's tfull counts both CTAs' bytes, tempty by commit to both
+//   aready/afree   the four 32-column slots of converted weights in TMEM; aready on the leader counts the
+//                  four warps of both CTAs, afree by commit to both
+//   dfull/dempty   accumulator halves; a job of more than HALF tokens takes both
+// Every wait is bounded (mbar_wait); on expiry the roles leave their loops and the kernel ends.
+#include "tc.cuh"
+
+namespace mg {
+
+namespace {
+
+constexpr int WL_MAX_TOKENS = 384;             // tokens per job: 384 accumulator columns
+constexpr int WL_GROUP_T = 8;                  // token tiles per L2 reuse group (weight tiles vary slower inside)
+constexpr int WL_K = 64;                       // K elements per MMA step (one 128-byte swizzle row of bf16)
+constexpr int WL_T_STAGE = WL_MAX_TOKENS / 2 * WL_K * 2;      // 24 KiB: this CTA's half of the tokens
+constexpr int WL_W_STAGE = 128 * 128;          // 16 KiB: 128 rows of 64 bf16 or of 128 FP8
+constexpr int WL_A_SLOTS = 4;
+constexpr int WL_A_COLS = 32;                  // 64 bf16 per lane
+
+constexpr int WL_SW = 6, WL_ST = 4;            // weight and token stages
+constexpr int WL_EPI_WARPS = 8, WL_CONV_WARPS = 8;
+constexpr int WL_THREADS = (4 + WL_EPI_WARPS + WL_CONV_WARPS) * 32;
+constexpr int WL_HALF = WL_MAX_TOKENS / 2;     // columns of an accumulator half
+constexpr int WL_A_COL0 = WL_MAX_TOKENS;       // converted weights above the accumulator
+constexpr int WL_RING_BYTES = WL_SW * WL_W_STAGE + WL_ST * WL_T_STAGE;
+constexpr int WL_PIECE = 2048;                 // epilogue staging per warp: 32 tokens x 32 outputs
+constexpr int WL_BARS = 2 * WL_SW + 2 * WL_ST + 2 * WL_A_SLOTS + 4;
+constexpr size_t WL_SMEM = 1024 + WL_RING_BYTES + WL_EPI_WARPS * WL_PIECE + 8 * WL_BARS + 16 + 4 * (3 * kMaxExperts + 3);
+static_assert(WL_SMEM <= 232448, "shared memory exceeds the 227 KiB a CTA may have");
+
+struct WlArgs {
+  const int32_t* pad_offsets;
+  const int32_t* counts;
+  int n_groups;
+  int n_tiles;                  // 256-row weight tiles per group
+  int n_per_group;
+  int k_steps;                  // K / 64
+  const float* scales;          // [rows / 128][K / 128]
+  int scale_cols;
+  int32_t* status;
+};
+
+struct Ring {
+  uint32_t i = 0, ph = 0;
+  __device__ __forceinline__ void next(uint32_t n) {
+    if (++i == n) { i = 0; ph ^= 1u; }
+  }
+};
+
+struct Job {
+  int row0;      // first token row
+  int left;      // live tokens
+  int n_tok;     // left rounded up to 32: the MMA's N
+  int b_row;     // first of the 256 weight rows
+  int n_idx;
+};
+
+// K steps that share one token stage: a job of few tokens packs several, so that the ring holds as many bytes in
+// flight as a job of many
+__device__ __forceinline__ int steps_per_stage(int n_tok) {
+  const int h = n_tok >> 1;
+  return h <= 24 ? 8 : h <= 48 ? 4 : h <= 96 ? 2 : 1;
+}
+__device__ __forceinline__ int round32(int v) { return (v + 31) & ~31; }
+
+// s_jp[e] = token tiles of the experts before e
+__device__ __forceinline__ Job locate_job(int job, const int* s_pad, const int* s_cnt, const int* s_jp, const WlArgs& g) {
+  int lo = 0, hi = g.n_groups;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (s_jp[mid] * g.n_tiles <= job) lo = mid; else hi = mid;
+  }
+  const int e = lo;
+  const int local = job - s_jp[e] * g.n_tiles;
+  const int nt = s_jp[e + 1] - s_jp[e];
+  const int per_group = WL_GROUP_T * g.n_tiles;
+  const int grp = local / per_group;
+  const int rem = local - grp * per_group;
+  const int gt = min(WL_GROUP_T, nt - grp * WL_GROUP_T);
+  const int n = rem / gt;
+  const int m = grp * WL_GROUP_T + (rem - n * gt);
+  const int size = round32((s_cnt[e] + nt - 1) / nt);      // tiles of one expert are equally long
+  Job j;
+  j.row0 = s_pad[e] + m * size;
+  j.left = min(size, s_cnt[e] - m * size);
+  j.n_tok = round32(j.left);
+  j.b_row = e * g.n_per_group + n * 256;
+  j.n_idx = n;
+  return j;
+}
+
+// D += A(tensor memory) * B(shared memory) on the SM pair
+__device__ __forceinline__ void tc_mma_pair_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
+      "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
+      "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Arrival on the leader CTA's barrier with the default semantics (release at CTA scope).  What it announces is tensor
+// memory, ordered by tcgen05 fences; at cluster scope the release would first wait until every global store of
+// the warp has reached L2, microseconds per tile in the epilogue.
+__device__ __forceinline__ void arrive_at_leader(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(smem_u32(bar), 0)) : "memory");
+}
+
+// 32 accumulator columns (tokens) of this thread's lane -> rows of the warp's staging piece, [token][output].
+// SwiGLU: lanes 0-15 of a warp hold gate rows, lanes 16-31 the up rows of the same 16 outputs; two tokens at a
+// time the halves trade values, lanes 0-15 finish token t and lanes 16-31 token t + 1.  The pieces are what the
+// TMA store's box wants: 32 rows of 16 outputs, or of 32 outputs with 64-byte swizzle; either way a warp's
+// 2-byte stores of one instruction fall into one run of 64 bytes.
+template <int EPI>
+__device__ __forceinline__ void stage_columns(const uint32_t (&v)[32], int lane, uint8_t* piece) {
+  if (EPI == EPI_SWIGLU_BF16) {
+    const bool up = lane >= 16;
+    uint8_t* dst = piece + (lane >> 4) * 32 + (lane & 15) * 2;
+#pragma unroll
+    for (int t = 0; t < 32; t += 2) {
+      const float a = __uint_as_float(v[t]), b = __uint_as_float(v[t + 1]);
+      const float got = __shfl_xor_sync(0xFFFFFFFFu, up ? a : b, 16);
+      const float h = up ? silu_f(got) * b : silu_f(a) * got;
+      *reinterpret_cast<__nv_bfloat16*>(dst + t * 32) = __float2bfloat16_rn(h);
+    }
+  } else {
+    const uint32_t chunk = lane >> 3, in_chunk = (lane & 7) * 2;
+#pragma unroll
+    for (int t = 0; t < 32; ++t)
+      *reinterpret_cast<__nv_bfloat16*>(piece + t * 64 + ((chunk ^ ((t >> 1) & 3)) << 4) + in_chunk) =
+          __float2bfloat16_rn(__uint_as_float(v[t]));
+  }
+}
+
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WL_THREADS, 1)
+grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmT64,
+                       const __grid_constant__ CUtensorMap tmT16, const __grid_constant__ CUtensorMap tmC, const WlArgs g) {
+  constexpr bool SWIGLU = EPI == EPI_SWIGLU_BF16;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* pieces = smem + WL_RING_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(pieces + WL_EPI_WARPS * WL_PIECE);
+  uint64_t* wfull = bars;
+  uint64_t* wempty = wfull + WL_SW;
+  uint64_t* tfull = wempty + WL_SW;
+  uint64_t* tempty = tfull + WL_ST;
+  uint64_t* aready = tempty + WL_ST;
+  uint64_t* afree = aready + WL_A_SLOTS;
+  uint64_t* dfull = afree + WL_A_SLOTS;
+  uint64_t* dempty = dfull + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + WL_BARS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* s_pad = reinterpret_cast<int*>(tmem_slot + 4);
+  int* s_cnt = s_pad + kMaxExperts + 1;
+  int* s_jp = s_cnt + kMaxExperts + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();           // 0 = leader
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < WL_SW; ++s) { mbar_init(smem_u32(&wfull[s]), 1); mbar_init(smem_u32(&wempty[s]), WL_CONV_WARPS); }
+    for (int s = 0; s < WL_ST; ++s) { mbar_init(smem_u32(&tfull[s]), 1); mbar_init(smem_u32(&tempty[s]), 1); }
+    for (int s = 0; s < WL_A_SLOTS; ++s) { mbar_init(smem_u32(&aready[s]), 8); mbar_init(smem_u32(&afree[s]), 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&dfull[s]), 1); mbar_init(smem_u32(&dempty[s]), 2 * WL_EPI_WARPS); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) { s_pad[i] = g.pad_offsets[i]; s_cnt[i] = g.counts[i]; }
+  __syncthreads();
+  if (warp == 3) {
+    // token tiles before each expert: lane sums of runs of 16 experts, warp scan, runs written out
+    constexpr int RUN = kMaxExperts / 32;
+    int sum = 0;
+    for (int i = 0; i < RUN; ++i) {
+      const int e = lane * RUN + i;
+      if (e < g.n_groups) sum += (s_cnt[e] + WL_MAX_TOKENS - 1) / WL_MAX_TOKENS;
+    }
+    int inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    int run = inc - sum;
+    for (int i = 0; i < RUN; ++i) {
+      const int e = lane * RUN + i;
+      if (e < g.n_groups) {
+        s_jp[e] = run;
+        run += (s_cnt[e] + WL_MAX_TOKENS - 1) / WL_MAX_TOKENS;
+        if (e == g.n_groups - 1) s_jp[g.n_groups] = run;
+      }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();      // barriers of both CTAs initialised, TMEM allocated on both SMs
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int total_jobs = s_jp[g.n_groups] * g.n_tiles;
+  const uint32_t w_base = smem_u32(smem);
+  const uint32_t t_base = w_base + WL_SW * WL_W_STAGE;
+
+  if (warp == 0) {
+    // ---------------- weight TMA (both CTAs, own 128 rows) ----------------
+    if (elect_one()) {
+      Ring r;
+      for (int job = pair; job < total_jobs && !*abort_flag; job += n_pairs) {
+        const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+        // SwiGLU rows come in blocks of 128 gate then 128 up; this CTA takes 64 of each
+        const int row_a = SWIGLU ? j.b_row + static_cast<int>(rank) * 64 : j.b_row + static_cast<int>(rank) * 128;
+        const int row_b = row_a + (SWIGLU ? 128 : 64);
+        for (int kb = 0; kb < g.k_steps / 2; ++kb, r.next(WL_SW)) {
+          if (!mbar_wait(smem_u32(&wempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 51)) break;
+          const uint32_t fb = smem_u32(&wfull[r.i]);
+          const uint32_t dst = w_base + r.i * WL_W_STAGE;
+          mbar_expect_tx(fb, WL_W_STAGE);
+          tma_load_2d(dst, &tmW, kb * 128, row_a, fb);
+          tma_load_2d(dst + 64 * 128, &tmW, kb * 128, row_b, fb);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- token TMA (both CTAs, own half of each MMA's N) ----------------
+    if (elect_one()) {
+      Ring r;
+      for (int job = pair; job < total_jobs && !*abort_flag; job += n_pairs) {
+        const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+        const int h1 = min(j.n_tok, 256) >> 1, h2 = (j.n_tok >> 1) - h1;
+        const int row1 = j.row0 + static_cast<int>(rank) * h1, row2 = j.row0 + 256 + static_cast<int>(rank) * h2;
+        const int kpt = steps_per_stage(j.n_tok);
+        for (int kb0 = 0; kb0 < g.k_steps; kb0 += kpt, r.next(WL_ST)) {
+          if (!mbar_wait(smem_u32(&tempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 52)) break;
+          const int kbs = min(kpt, g.k_steps - kb0);
+          const uint32_t fb = smem_u32(&tfull[r.i]);
+          if (rank == 0) mbar_expect_tx(fb, kbs * j.n_tok * 128);
+          for (int i = 0; i < kbs; ++i) {
+            const uint32_t dst = t_base + r.i * WL_T_STAGE + i * (h1 + h2) * 128;
+            const int kx = (kb0 + i) * WL_K;
+            int o = 0;
+            for (; o + 64 <= h1; o += 64) tma_load_2d_pair(dst + o * 128, &tmT64, kx, row1 + o, fb);
+            for (; o < h1; o += 16) tma_load_2d_pair(dst + o * 128, &tmT16, kx, row1 + o, fb);
+            o = 0;
+            for (; o + 64 <= h2; o += 64) tma_load_2d_pair(dst + (h1 + o) * 128, &tmT64, kx, row2 + o, fb);
+            for (; o < h2; o += 16) tma_load_2d_pair(dst + (h1 + o) * 128, &tmT16, kx, row2 + o, fb);
+          }
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ---------------- MMA issuer (leader CTA only) ----------------
+    if (rank == 0 && elect_one()) {
+      Ring rt, ra;
+      uint32_t used0 = 0u, used1 = 0u, turn = 0u;      // uses of the accumulator halves
+      // kind::f16: D fp32 (bit 4), A bf16 (bit 7), B bf16 (bit 10), both K-major, N>>3 at 17, M>>4 at 24
+      const uint32_t id0 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(256 >> 4) << 24);
+      bool ok = true;
+      for (int job = pair; job < total_jobs && ok && !*abort_flag; job += n_pairs) {
+        const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+        const bool wide = j.n_tok > WL_HALF;
+        const uint32_t h = wide ? 0u : turn;
+        if (!wide) turn ^= 1u;
+        const bool take0 = wide || h == 0u, take1 = wide || h == 1u;
+        ok = (!take0 || mbar_wait(smem_u32(&dempty[0]), (used0 & 1u) ^ 1u, abort_flag, g.status, 53)) &&
+             (!take1 || mbar_wait(smem_u32(&dempty[1]), (used1 & 1u) ^ 1u, abort_flag, g.status, 53));
+        if (!ok) break;
+        used0 += take0;
+        used1 += take1;
+        tc_fence_after();
+        const int n1 = min(j.n_tok, 256), n2 = j.n_tok - n1;
+        const uint32_t id1 = id0 | (static_cast<uint32_t>(n1 >> 3) << 17), id2 = id0 | (static_cast<uint32_t>(n2 >> 3) << 17);
+        const uint32_t d = tmem_base + h * WL_HALF;
+        const int kpt = steps_per_stage(j.n_tok), step_bytes = j.n_tok * 64;
+        int in_stage = 0;
+        for (int kb = 0; kb < g.k_steps; ++kb) {
+          ok = (in_stage != 0 || mbar_wait(smem_u32(&tfull[rt.i]), rt.ph, abort_flag, g.status, 54)) &&
+               mbar_wait(smem_u32(&aready[ra.i]), ra.ph, abort_flag, g.status, 55);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t tb = t_base + rt.i * WL_T_STAGE + in_stage * step_bytes;
+          const uint64_t db = make_smem_desc(tb);
+          const uint64_t db2 = make_smem_desc(tb + n1 * 64);
+          const uint32_t a = tmem_base + WL_A_COL0 + ra.i * WL_A_COLS;
+#pragma unroll
+          for (int k = 0; k < WL_K / 16; ++k) {
+            // 16 bf16 = 32 bytes = 2 sixteen-byte units inside the swizzle row, or 8 columns of tensor memory
+            const uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
+            tc_mma_pair_ts(d, a + 8 * k, db + 2 * k, id1, accumulate);
+            if (n2 > 0) tc_mma_pair_ts(d + 256, a + 8 * k, db2 + 2 * k, id2, accumulate);
+          }
+          tc_commit_pair(smem_u32(&afree[ra.i]));
+          if (++in_stage == kpt || kb + 1 == g.k_steps) {
+            tc_commit_pair(smem_u32(&tempty[rt.i]));
+            rt.next(WL_ST);
+            in_stage = 0;
+          }
+          ra.next(WL_A_SLOTS);
+        }
+        if (!ok) break;
+        if (take0) tc_commit_pair(smem_u32(&dfull[0]));
+        if (take1) tc_commit_pair(smem_u32(&dfull[1]));
+      }
+    }
+  } else if (warp >= 4 && warp < 4 + WL_EPI_WARPS) {
+    // ---------------- epilogue (both CTAs, own 128 lanes) ----------------
+    const int quarter = warp & 3;
+    uint8_t* piece = pieces + (warp - 4) * WL_PIECE;
+    uint32_t used0 = 0u, used1 = 0u, turn = 0u;
+    for (int job = pair; job < total_jobs && !*abort_flag; job += n_pairs) {
+      const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+      const bool wide = j.n_tok > WL_HALF;
+      const uint32_t h = wide ? 0u : turn;
+      if (!wide) turn ^= 1u;
+      const bool take0 = wide || h == 0u, take1 = wide || h == 1u;
+      bool ok;
+      ok = (!take0 || mbar_wait(smem_u32(&dfull[0]), used0 & 1u, abort_flag, g.status, 56)) &&
+           (!take1 || mbar_wait(smem_u32(&dfull[1]), used1 & 1u, abort_flag, g.status, 56));
+      ok = __all_sync(0xFFFFFFFFu, ok);
+      if (!ok) break;
+      used0 += take0;
+      used1 += take1;
+      __syncwarp();
+      tc_fence_after();
+      const int col0 = SWIGLU ? j.n_idx * 128 + static_cast<int>(rank) * 64 + quarter * 16
+                              : j.n_idx * 256 + static_cast<int>(rank) * 128 + quarter * 32;
+      const uint32_t taddr = tmem_base + h * WL_HALF + (static_cast<uint32_t>(quarter * 32) << 16);
+      for (int c = (warp - 4) / 4 * 32; c < j.left; c += 64) {
+        uint32_t v[32];
+        tc_ld32(taddr + c, v);
+        // the store that last used this piece has finished reading it
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        tc_ld_wait();
+        __syncwarp();
+        stage_columns<EPI>(v, lane, piece);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tma_store_2d(&tmC, col0, j.row0 + c, smem_u32(piece));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (take0) arrive_at_leader(&dempty[0]);
+        if (take1) arrive_at_leader(&dempty[1]);
+      }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
+  } else if (warp >= 4 + WL_EPI_WARPS) {
+    // ---------------- FP8 -> bf16 converters: shared -> registers -> tensor memory ----------------
+    const int quarter = warp & 3;
+    const uint32_t grp = (warp - 4 - WL_EPI_WARPS) >> 2;   // even / odd 64-element K steps
+    const int row = !SWIGLU ? quarter * 32 + lane : quarter * 16 + (lane & 15) + (lane & 16) * 4;
+    const int block = SWIGLU ? lane >> 4 : static_cast<int>(rank);      // scale block row of this lane's weights
+    Ring rw;
+    uint32_t slot = grp, ph = 0u;                          // this group's slots: grp, grp + 2
+    bool ok = true;
+    for (int job = pair; job < total_jobs && ok && !*abort_flag; job += n_pairs) {
+      const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+      const float* srow = g.scales + static_cast<long long>((j.b_row >> 7) + block) * g.scale_cols;
+      // 16 scales of this lane's row at a time, spread over its half of the warp and handed out by shuffle: a load
+      // per stage put an L2 round trip on every stage (decode gate/up product 3.3 instead of 1.5 ms)
+      float s16 = 0.f;
+      for (int kb = 0; kb < g.k_steps / 2; ++kb) {
+        if ((kb & 15) == 0) s16 = kb + (lane & 15) < g.scale_cols ? __ldg(srow + kb + (lane & 15)) : 0.f;
+        const float s = __shfl_sync(0xFFFFFFFFu, s16, (lane & 16) | (kb & 15));
+        ok = mbar_wait(smem_u32(&wfull[rw.i]), rw.ph, abort_flag, g.status, 57);
+        ok = __all_sync(0xFFFFFFFFu, ok);
+        if (!ok) break;
+        const uint8_t* src = smem + rw.i * WL_W_STAGE + row * 128;
+        uint4 q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint4*>(src + (((grp * 4 + i) ^ (row & 7)) << 4));
+        uint32_t o[32];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint4 lo, hi;
+          convert16(q[i], s, lo, hi);
+          o[8 * i] = lo.x; o[8 * i + 1] = lo.y; o[8 * i + 2] = lo.z; o[8 * i + 3] = lo.w;
+          o[8 * i + 4] = hi.x; o[8 * i + 5] = hi.y; o[8 * i + 6] = hi.z; o[8 * i + 7] = hi.w;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&wempty[rw.i]));
+        rw.next(WL_SW);
+        ok = mbar_wait(smem_u32(&afree[slot]), ph ^ 1u, abort_flag, g.status, 58);
+        ok = __all_sync(0xFFFFFFFFu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        tc_st32(tmem_base + WL_A_COL0 + slot * WL_A_COLS + (static_cast<uint32_t>(quarter * 32) << 16), o);
+        tc_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_at_leader(&aready[slot]);
+        slot ^= 2u;
+        if (slot == grp) ph ^= 1u;
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();      // neither CTA leaves while the other may still signal it or use its TMEM
+  if (warp == 3) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  }
+}
+
+template <int EPI>
+int launch_kernel(const Handle* h, const CUtensorMap& tw, const CUtensorMap& t64, const CUtensorMap& t16,
+                  const CUtensorMap& tc, const WlArgs& a, int grid, cudaStream_t st) {
+  static bool done[64];
+  if (!(h->device >= 0 && h->device < 64 && done[h->device])) {
+    MG_CUDA(cudaFuncSetAttribute(grouped_gemm_wl_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(WL_SMEM)));
+    if (h->device >= 0 && h->device < 64) done[h->device] = true;
+  }
+  grouped_gemm_wl_kernel<EPI><<<grid, WL_THREADS, WL_SMEM, st>>>(tw, t64, t16, tc, a);
+  MG_CUDA(cudaGetLastError());
+  return MG_OK;
+}
+
+}  // namespace
+
+int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
+  const bool swiglu = p.epilogue == EPI_SWIGLU_BF16;
+  MG_REQUIRE(p.b_fp8 && p.scales != nullptr && p.pad_offsets != nullptr && (swiglu || p.epilogue == EPI_PLAIN_BF16),
+             MG_ERR_CONFIG, "weight-lane GEMM: grouped FP8 weights and bf16 outputs only");
+  MG_REQUIRE(p.K % 128 == 0 && p.n_per_group % 256 == 0 && p.ldo % 16 == 0, MG_ERR_SHAPE,
+             "weight-lane GEMM: K=%d, N per expert=%d", p.K, p.n_per_group);
+  CUtensorMap tw, t64, t16, tc;
+  int rc = encode_2d(h, &tw, p.b, static_cast<uint64_t>(p.n_groups) * p.n_per_group, static_cast<uint64_t>(p.K), 64,
+                     TM_FP8_SW128);
+  if (rc != MG_OK) return rc;
+  rc = encode_2d(h, &t64, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 64, TM_BF16);
+  if (rc != MG_OK) return rc;
+  rc = encode_2d(h, &t16, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 16, TM_BF16);
+  if (rc != MG_OK) return rc;
+  rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32,
+                 swiglu ? TM_OUT_16 : TM_OUT_PIECE);
+  if (rc != MG_OK) return rc;
+  WlArgs a;
+  a.pad_offsets = p.pad_offsets;
+  a.counts = p.counts;
+  a.n_groups = p.n_groups;
+  a.n_tiles = p.n_per_group / 256;
+  a.n_per_group = p.n_per_group;
+  a.k_steps = p.K / WL_K;
+  a.scales = p.scales;
+  a.scale_cols = p.K / 128;
+  a.status = h->d_status;
+  const int64_t tiles = (p.a_rows + WL_MAX_TOKENS - 1) / WL_MAX_TOKENS + p.n_groups;
+  int64_t pairs = h->sm_count / 2;
+  if (tiles * a.n_tiles < pairs) pairs = tiles * a.n_tiles;
+  const int grid = static_cast<int>(2 * pairs);
+  return swiglu ? launch_kernel<EPI_SWIGLU_BF16>(h, tw, t64, t16, tc, a, grid, st)
+                : launch_kernel<EPI_PLAIN_BF16>(h, tw, t64, t16, tc, a, grid, st);
+}
+
+}  // namespace mg
+

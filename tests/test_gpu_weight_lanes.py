@@ -1,0 +1,82 @@
+"""GPU: the expert GEMMs with the weights on the accumulator's lanes (gemm_wl.cu), at the edges of their jobs: no
+row, one row, multiples of 32 tokens and the rows around them, both accumulator halves, one job and several per
+expert.  Rows between the segments hold NaN, which must not reach a live row."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle import moe_oracle as O
+from tests.util import make_layer
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(got, ref, mag, what):
+    """bf16 rounding of the result (2^-9, doubled for a value at a rounding edge) plus fp32 sums in any order:
+    n additions of terms of total magnitude `mag` err by less than n 2^-24 mag, here with n <= 512."""
+    err = (got.double() - ref).abs()
+    bound = 2.0 ** -8 * ref.abs() + 512 * 2.0 ** -24 * mag
+    assert torch.isfinite(got.float()).all(), what
+    assert bool((err <= bound).all()), (what, float((err / bound.clamp_min(1e-30)).max()))
+
+
+def _reference(x, wg, wu, wd, h_got):
+    """h and its magnitude from x; out and its magnitude from the h the kernel produced."""
+    x, wg, wu, wd = (t.double() for t in (x, wg, wu, wd))
+    g, u = F.linear(x, wg), F.linear(x, wu)
+    gm, um = F.linear(x.abs(), wg.abs()), F.linear(x.abs(), wu.abs())
+    h = F.silu(g) * u
+    # |d silu| <= 1.1: errors of g and u reach h times the other factor; __expf and the fast division add 4 ulp
+    h_mag = 1.1 * gm * u.abs() + F.silu(g).abs() * um
+    hq = h_got.double()
+    return h, h_mag, F.linear(hq, wd), F.linear(hq.abs(), wd.abs())
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("counts", [
+    [0, 1, 0, 31, 32, 33, 0, 2],
+    [63, 64, 65, 127, 128, 129, 0, 0],
+    [191, 192, 193, 255, 256, 257, 1, 0],
+    [383, 384, 385, 0, 767, 769, 32, 16],
+    [3100, 0, 1, 5, 0, 0, 40, 400],
+    [0, 0, 0, 0, 0, 0, 0, 1],
+])
+def test_expert_products_at_job_edges(built_lib, counts, fp8):
+    spec = O.LayerSpec(512, 384, 8, 2, 0, 1, 1, O.GATE_SOFTMAX_GREEDY, False, 1.0,
+                       O.WEIGHT_FP8_BLOCK128 if fp8 else O.WEIGHT_BF16, O.COMBINE_FP32)
+    _, W = O.make_inputs(spec, 4, 11)
+    layer = make_layer(spec, W)
+    cnt = torch.tensor(counts)
+    pad = torch.zeros(9, dtype=torch.int64)
+    pad[1:] = ((cnt + 127) // 128 * 128).cumsum(0)
+    rows = int(pad[-1]) + 256
+    x = torch.full((rows, 512), float("nan"), dtype=torch.bfloat16, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for e, c in enumerate(counts):
+        x[pad[e]:pad[e] + c] = torch.randn(c, 512, generator=g, device="cuda").to(torch.bfloat16)
+    h, out = layer.expert_ffn(x, pad.int().cuda(), cnt.int().cuda())
+    torch.cuda.synchronize()
+    assert layer.device_status()[0] == 0
+    for e, c in enumerate(counts):
+        s = slice(int(pad[e]), int(pad[e]) + c)
+        w = [m[e].cuda() for m in (W.w_gate, W.w_up, W.w_down)]
+        rh, mh, ro, mo = _reference(x[s], *w, h[s])
+        _close(h[s], rh, mh, ("h", e, c))
+        _close(out[s], ro, mo, ("out", e, c))
+
+
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 256, 257, 384, 385, 1000, 3500])
+def test_shared_expert_at_job_edges(built_lib, T):
+    spec = O.LayerSpec(512, 128, 8, 2, 384, 1, 1, O.GATE_SOFTMAX_GREEDY, False, 1.0, O.WEIGHT_BF16, O.COMBINE_FP32)
+    x, W = O.make_inputs(spec, T, 12)
+    layer = make_layer(spec, W)
+    x = x.cuda()
+    out = layer.shared_ffn(x)
+    torch.cuda.synchronize()
+    assert layer.device_status()[0] == 0
+    xd, (wg, wu, wd) = x.double(), (m.cuda().double() for m in W.shared)
+    h = F.silu(F.linear(xd, wg)) * F.linear(xd, wu)
+    # the kernel rounds h to bf16 on the way: 2^-9 of it, carried through the second product
+    hm = F.linear(h.abs(), wd.abs())
+    err = (out.double() - F.linear(h, wd)).abs()
+    assert bool((err <= 2.0 ** -8 * F.linear(h, wd).abs() + 2.0 ** -8 * hm).all())
