@@ -774,7 +774,13 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
 // The whole plan in one block, for batches of up to kPlanSmallTokens tokens: a bitmap per (32 tokens, expert) gives
 // the counts and the stable ranks, one block scan the offsets.  Same results as the four kernels above, which cost a
 // launch each: 20 -> 8 us at 8 tokens, 23 -> 10 us at 512.  The limit is one token per thread of the block.
+// A token that names an expert twice counts twice, as in plan_count_kernel: the bitmap holds it once, so the
+// repeats are counted beside it, per run of kPlanTokens tokens like the block counts there.
 constexpr int kPlanSmallTokens = 1024;
+__host__ __device__ constexpr int plan_small_runs(int T) { return (T + kPlanTokens - 1) / kPlanTokens; }
+constexpr size_t plan_small_smem(int T, int n) {
+  return static_cast<size_t>(2 * ((T + 31) / 32) + plan_small_runs(T)) * n * sizeof(int32_t);
+}
 __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restrict__ idx, int T, int k, int lo, int n,
                                                           int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                                                           int32_t* __restrict__ pad_offsets,
@@ -784,13 +790,17 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
   const int W = (T + 31) >> 5;
   uint32_t* bm = reinterpret_cast<uint32_t*>(sm);  // [W][n] tokens of the run of 32 that picked e
   int32_t* wbase = sm + W * n;                     // [W][n] first row of the run's tokens
+  int32_t* again = wbase + W * n;                  // [plan_small_runs(T)][n] repeated picks of e
+  constexpr int RUN_W = kPlanTokens / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < W * n; i += blockDim.x) bm[i] = 0u;
+  for (int i = tid; i < plan_small_runs(T) * n; i += blockDim.x) again[i] = 0;
   __syncthreads();
   if (tid < T) {
+    const uint32_t bit = 1u << lane;
     for (int j = 0; j < k; ++j) {
       const int e = idx[tid * k + j] - lo;
-      if (e >= 0 && e < n) atomicOr(&bm[warp * n + e], 1u << lane);
+      if (e >= 0 && e < n && (atomicOr(&bm[warp * n + e], bit) & bit)) atomicAdd(&again[warp / RUN_W * n + e], 1);
     }
   }
   __syncthreads();
@@ -799,6 +809,7 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
     for (int w = 0; w < W; ++w) {
       wbase[w * n + tid] = c;
       c += __popc(bm[w * n + tid]);
+      if (w + 1 == W || (w + 1) % RUN_W == 0) c += again[w / RUN_W * n + tid];
     }
   }
   const int32_t cp = (c + kTileM - 1) / kTileM * kTileM;
@@ -832,11 +843,11 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
 
 static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo, int n, int32_t* counts,
                              int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row, cudaStream_t st) {
-  const size_t smem = static_cast<size_t>(2) * ((T + 31) / 32) * n * sizeof(int32_t);
+  const size_t smem = plan_small_smem(T, n);
   static bool done[64];
   if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[h->device])) {
     MG_CUDA(cudaFuncSetAttribute(plan_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 2 * (kPlanSmallTokens / 32) * kMaxExperts * static_cast<int>(sizeof(int32_t))));
+                                 static_cast<int>(plan_small_smem(kPlanSmallTokens, kMaxExperts))));
     if (h->device >= 0 && h->device < 64) done[h->device] = true;
   }
   const int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;

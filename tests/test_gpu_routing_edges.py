@@ -32,6 +32,24 @@ def test_permute_plan_at_the_one_block_limit(built_lib, T, E, k):
     assert torch.equal(dst.cpu().long().view(-1), want)
 
 
+@pytest.mark.parametrize("lo,n", [(0, 24), (5, 13)])
+@pytest.mark.parametrize("T", [1, 40, 256, 257, 700, 1024])
+def test_one_block_plan_of_repeated_and_foreign_picks_equals_the_general_plan(built_lib, T, lo, n):
+    """Picks that name an expert twice count twice and foreign picks not at all, in one block as in the four
+    kernels of larger batches; those run here on the same picks followed by tokens without a pick."""
+    _, layer = _router_only(24, 6)
+    idx = torch.randint(0, 24, (T, 6), generator=torch.Generator().manual_seed(T), dtype=torch.int32)
+    idx[::7, 5] = idx[::7, 0]
+    idx[::5, 2] = -1
+    got = layer.permute_plan(idx.cuda(), lo, n)
+    padded = torch.cat([idx, torch.full((1100, 6), -1, dtype=torch.int32)])
+    want = layer.permute_plan(padded.cuda(), lo, n)
+    assert torch.equal(got[0].cpu().long(), torch.bincount(idx[(idx >= lo) & (idx < lo + n)].long() - lo, minlength=n))
+    for a, b in zip(got[:3], want[:3]):
+        assert torch.equal(a, b)
+    assert torch.equal(got[3], want[3][:T])
+
+
 @pytest.mark.parametrize("gating,E,k,n_group,topk_group", [
     (O.GATE_SOFTMAX_GREEDY, 64, 6, 1, 1), (O.GATE_SOFTMAX_GROUP_MAX, 160, 6, 8, 3),
     (O.GATE_SIGMOID_NOAUX_TC, 256, 8, 8, 4), (O.GATE_SOFTMAX_GROUP_MAX, 96, 4, 3, 2)])
