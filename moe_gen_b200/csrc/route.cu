@@ -3,7 +3,7 @@
 // 128-bit vector accesses on rows.
 #include <mutex>
 
-#include "common.cuh"
+#include "tc.cuh"
 
 namespace mg {
 
@@ -98,11 +98,12 @@ __device__ __forceinline__ float kth_best_value(const float (&c0)[P], uint32_t g
 }
 
 // Near-ties are listed in `fix` when it is given (route_topk_kernel) or, with FIX_INLINE, returned as this lane's
-// experts in play (route_fused_kernel recomputes them in the same warp; groups are runs of lanes there).
+// experts in play (the blocks of route_fused_kernel recompute them; groups are runs of lanes there).
 template <int P, bool FIX_INLINE = false>
 __device__ __forceinline__ uint32_t route_token(const float* logits, const float* __restrict__ bias,
                                                 int64_t t, const RouteParams& rp, int32_t* __restrict__ out_idx,
-                                                float* __restrict__ out_w, int32_t* __restrict__ fix) {
+                                                float* __restrict__ out_w, int32_t* __restrict__ fix,
+                                                bool store = true) {
   const bool detect = FIX_INLINE || fix != nullptr;
   uint32_t found = 0;
   const int lane = threadIdx.x & 31;
@@ -347,7 +348,7 @@ __device__ __forceinline__ uint32_t route_token(const float* logits, const float
     if (rp.k > 1 && rp.norm) my_w = __fdiv_rn(my_w, __fadd_rn(denom, 1e-20f));
     else my_w = __fmul_rn(my_w, rp.scale);
   }
-  if (lane < rp.k) {
+  if (store && lane < rp.k) {
     out_idx[t * rp.k + lane] = my_idx;
     out_w[t * rp.k + lane] = my_w;
   }
@@ -515,42 +516,157 @@ __global__ void __launch_bounds__(256) route_fix_pairs_kernel(const __nv_bfloat1
   }
 }
 
-// Routing and the near-tie fix-up in one pass: a block routes 8 tokens, recomputes the logits in play of its close
-// tokens (a warp per logit) and routes those tokens again.  Same logits, picks and weights as the listing kernels
-// above; no lists in memory.  Bound by launches and latency at decode sizes: V2-Lite at 8 tokens spent 23 us in
-// memset, top-k, two fix-up kernels and the second top-k, 8 us now; V3 at 4096 skewed tokens 0.13 -> 0.05 ms, at
-// 65536 tokens beside the de-quantisation 1.30 -> 0.65 ms.
+// 4 tokens x 4 experts of logits by one warp, lanes across H, so that an operand is widened to fp64 once per four
+// multiply-adds: widening is the slow instruction here (16 a cycle and SM against 64 fp64 multiply-adds).  Eight
+// bytes a lane and step keep the tile within the registers of the routing around it.
+constexpr int kTileTok = 4, kTileExp = 4;
+template <int UNROLL>
+__device__ __forceinline__ void exact_tile(const __nv_bfloat16* const (&xr)[kTileTok], const __nv_bfloat16* w, int H,
+                                           int lane, double (&acc)[kTileTok][kTileExp]) {
+#pragma unroll
+  for (int j = 0; j < kTileTok; ++j)
+#pragma unroll
+    for (int i = 0; i < kTileExp; ++i) acc[j][i] = 0.0;
+#pragma unroll UNROLL
+  for (int v = lane; v < (H >> 2); v += 32) {
+    uint2 xv[kTileTok], wv[kTileExp];
+#pragma unroll
+    for (int j = 0; j < kTileTok; ++j) xv[j] = __ldg(reinterpret_cast<const uint2*>(xr[j]) + v);
+#pragma unroll
+    for (int i = 0; i < kTileExp; ++i) wv[i] = __ldg(reinterpret_cast<const uint2*>(w + static_cast<int64_t>(i) * H) + v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      double xd[kTileTok];
+#pragma unroll
+      for (int j = 0; j < kTileTok; ++j) {
+        const uint32_t pair = q < 2 ? xv[j].x : xv[j].y;
+        xd[j] = (q & 1) ? bf16_hi_f64(pair) : bf16_lo_f64(pair);
+      }
+#pragma unroll
+      for (int i = 0; i < kTileExp; ++i) {
+        const uint32_t pair = q < 2 ? wv[i].x : wv[i].y;
+        const double wd = (q & 1) ? bf16_hi_f64(pair) : bf16_lo_f64(pair);
+#pragma unroll
+        for (int j = 0; j < kTileTok; ++j) acc[j][i] = fma(xd[j], wd, acc[j][i]);
+      }
+    }
+  }
+}
+
+// Routing and the near-tie fix-up in one pass: a cluster of C blocks routes 8 tokens, recomputes the logits in play of
+// its close tokens and routes those tokens again.  Picks and weights as with the listing kernels above, and the same
+// logits while their list of pairs holds (where it overflows they recompute the whole row instead); no lists in memory.
+// Bound by launches and latency at decode sizes: V2-Lite at 8 tokens spent 23 us in memset, top-k, two fix-up kernels
+// and the second top-k, 8 us now; V3 at 4096 skewed tokens 0.13 -> 0.05 ms, at 65536 tokens beside the
+// de-quantisation 1.30 -> 0.65 ms.
+//
+// Rows of zeros (padding), or any rows whose logits lie within the error bound of one another, have every expert in
+// play, and a warp per logit, all of them on the SM that routed the token, took 15 times as long as the listing
+// kernels.  So a cluster's tokens are `groups` apart, which deals out a run of padding evenly; every block of a
+// cluster routes all 8 tokens (the first one stores) and takes the logits of every C-th run of 4 experts; and where
+// an eighth of the logits is in play they go by tiles, a tile with fewer than kTileExp of them still one by one.
+// FEW: the form for clusters, with registers for more loads in flight; two of its blocks fit an SM, three of the other.
+// Measured, us of routing with all rows zero, listing kernels / a warp per logit on one SM / this: V2-Lite 8 tokens
+// 36 / 122 / 17, 4096 tokens 164 / 324 / 116; V2-236B 512 tokens 123 / 644 / 98; V3 without a correction bias 8 tokens
+// 79 / 1202 / 78, 65536 tokens 20.7 / 54.5 / 17.5 ms.  Behind the listing kernels, whose lists level the load over all
+// SMs: V3 without a bias at 128 tokens (82 / 1212 / 116), and rows that leave some six logits of each token in play (1024
+// tokens 62 / 143 / 110).
 constexpr int kRouteWarps = 8;
-template <int P>
-__global__ void __launch_bounds__(kRouteWarps * 32) route_fused_kernel(float* logits, const float* __restrict__ bias,
-                                                                       RouteParams rp,
-                                                                       const __nv_bfloat16* __restrict__ x,
-                                                                       const __nv_bfloat16* __restrict__ gate_w, int H,
-                                                                       int32_t* __restrict__ out_idx,
-                                                                       float* __restrict__ out_w) {
+template <int P, bool FEW>
+__global__ void __launch_bounds__(kRouteWarps * 32, (FEW ? 16 : 24) / kRouteWarps)
+route_fused_kernel(float* logits, const float* __restrict__ bias, RouteParams rp, const __nv_bfloat16* __restrict__ x,
+                   const __nv_bfloat16* __restrict__ gate_w, int H, int32_t* __restrict__ out_idx,
+                   float* __restrict__ out_w, int groups, int cluster) {
   __shared__ uint16_t pairs[kRouteWarps * kMaxExperts];       // token of the block << 9 | expert
+  __shared__ uint32_t play[kRouteWarps][kMaxExperts / 32];    // the same as bits
   __shared__ int n_pairs;
   static_assert(kMaxExperts == 1 << 9, "pairs are packed for 512 experts");
+  const int C = FEW ? cluster : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kRouteWarps, t = t0 + warp;
+  const int rank = FEW ? static_cast<int>(blockIdx.x) % C : 0;
+  const int64_t t0 = blockIdx.x / C, t = t0 + static_cast<int64_t>(warp) * groups;
   if (threadIdx.x == 0) n_pairs = 0;
+  if (lane < kMaxExperts / 32) play[warp][lane] = 0u;
   __syncthreads();
-  uint32_t in_play = 0;
-  if (t < rp.T) in_play = route_token<P, true>(logits, bias, t, rp, out_idx, out_w, nullptr);
+  // Recomputes the logits in play (this lane's experts of its warp's token); false when the group has none.
+  auto fix_up = [&](uint32_t in_play) {
 #pragma unroll
-  for (int i = 0; i < P; ++i)
-    if ((in_play >> i) & 1u) pairs[atomicAdd(&n_pairs, 1)] = static_cast<uint16_t>(warp << 9 | (lane * P + i));
-  __syncthreads();
-  const int n = n_pairs;
-  if (n == 0) return;
-  for (int i = warp; i < n; i += kRouteWarps) {
-    const int64_t tok = t0 + (pairs[i] >> 9);
-    const int e = pairs[i] & (kMaxExperts - 1);
-    const double a = exact_logit(x + tok * H, gate_w + static_cast<int64_t>(e) * H, H >> 3, lane);
-    if (lane == 0) logits[tok * rp.E + e] = static_cast<float>(a);
+    for (int i = 0; i < P; ++i) {
+      const int e = lane * P + i;
+      if (((in_play >> i) & 1u) && (!FEW || e / kTileExp % C == rank)) {
+        pairs[atomicAdd(&n_pairs, 1)] = static_cast<uint16_t>(warp << 9 | e);
+        atomicOr(&play[warp][e >> 5], 1u << (e & 31));
+      }
+    }
+    // the blocks of a cluster saw the same logits, so they agree on whether there is anything to do
+    if (!__syncthreads_or(in_play != 0u)) return false;
+    __syncwarp();
+    if (FEW) cluster_sync_all();                               // every block has read the logits it routed by
+    const int n = n_pairs;
+    auto single = [&](int j, int e) {
+      const int64_t tok = t0 + static_cast<int64_t>(j) * groups;
+      const double a = exact_logit(x + tok * H, gate_w + static_cast<int64_t>(e) * H, H >> 3, lane);
+      if (lane == 0) logits[tok * rp.E + e] = static_cast<float>(a);
+    };
+    if (n * C < rp.E * kRouteWarps / 8) {
+      for (int i = warp; i < n; i += kRouteWarps) single(pairs[i] >> 9, pairs[i] & (kMaxExperts - 1));
+    } else {
+      constexpr int PARTS = kRouteWarps / kTileTok;            // every warp takes tiles of all of them in turn
+      for (int it = warp; ; it += kRouteWarps) {
+        const int e0 = (it / PARTS * C + rank) * kTileExp, j0 = (it + it / kRouteWarps) % PARTS * kTileTok;
+        if (e0 >= rp.E) break;
+        uint32_t bits = 0;                                     // kTileExp bits per token
+#pragma unroll
+        for (int j = 0; j < kTileTok; ++j)
+          bits |= ((play[j0 + j][e0 >> 5] >> (e0 & 31)) & ((1u << kTileExp) - 1u)) << (j * kTileExp);
+        if (__popc(bits) < kTileExp) {
+          for (; bits != 0u; bits &= bits - 1u) {
+            const int b = __ffs(bits) - 1;
+            single(j0 + b / kTileExp, e0 + b % kTileExp);
+          }
+          continue;
+        }
+        const __nv_bfloat16* xr[kTileTok];
+#pragma unroll
+        for (int j = 0; j < kTileTok; ++j) {
+          const int64_t tok = t0 + static_cast<int64_t>(j0 + j) * groups;
+          xr[j] = x + (tok < rp.T ? tok : t0) * H;
+        }
+        double acc[kTileTok][kTileExp];
+        exact_tile<FEW ? 2 : 1>(xr, gate_w + static_cast<int64_t>(e0) * H, H, lane, acc);
+#pragma unroll
+        for (int j = 0; j < kTileTok; ++j) {
+          float* row = logits + (t0 + static_cast<int64_t>(j0 + j) * groups) * rp.E + e0;
+#pragma unroll
+          for (int i = 0; i < kTileExp; ++i) {
+            double a = acc[j][i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xFFFFFFFFu, a, o);
+            if (lane == 0 && ((bits >> (j * kTileExp + i)) & 1u)) row[i] = static_cast<float>(a);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (FEW) cluster_sync_all(); else __syncthreads();         // the recomputed logits are in place
+    return true;
+  };
+  const bool mine = t < rp.T;
+  if constexpr (FEW) {
+    // Both passes run the same code, in a loop: the second finds it in the instruction cache, where at decode sizes a
+    // pass is mostly waiting for instructions (V3, 8 tokens with one close one: 35 us with a second copy, 31 so).
+    bool route = mine;
+#pragma unroll 1
+    for (bool last = false; ; last = true) {
+      const uint32_t in_play = route ? route_token<P, true>(logits, bias, t, rp, out_idx, out_w, nullptr, rank == 0) : 0u;
+      if (last || !fix_up(in_play)) return;
+      route = rank == 0 && __any_sync(0xFFFFFFFFu, in_play != 0u);
+    }
+  } else {
+    const uint32_t in_play = mine ? route_token<P, true>(logits, bias, t, rp, out_idx, out_w, nullptr) : 0u;
+    if (fix_up(in_play) && __any_sync(0xFFFFFFFFu, in_play != 0u))
+      route_token<P>(logits, bias, t, rp, out_idx, out_w, nullptr);
   }
-  __syncthreads();
-  if (__any_sync(0xFFFFFFFFu, in_play != 0u)) route_token<P>(logits, bias, t, rp, out_idx, out_w, nullptr);
 }
 
 static int route_P(int n_experts) {
@@ -625,9 +741,25 @@ int launch_route_fused(const Handle* h, const void* x, const void* gate_w, float
                        d.routed_scale, route_fix_err(d.hidden), 0, T};
   const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
   const __nv_bfloat16* wb = static_cast<const __nv_bfloat16*>(gate_w);
-  const unsigned grid = static_cast<unsigned>((T + kRouteWarps - 1) / kRouteWarps);
+  // clusters as large as two blocks an SM allow: up to 296 tokens 8 blocks on 148 SMs, from 1185 tokens on none
+  const int groups = static_cast<int>((T + kRouteWarps - 1) / kRouteWarps);
+  int C = 8;
+  while (C > 1 && static_cast<int64_t>(groups) * C > 2 * h->sm_count) C >>= 1;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(C);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(groups) * C);
+  cfg.blockDim = dim3(kRouteWarps * 32);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
 #define MG_ROUTE_CASE(PP) \
-  case PP: route_fused_kernel<PP><<<grid, kRouteWarps * 32, 0, st>>>(logits, bias, rp, xb, wb, d.hidden, idx, w); break
+  case PP: \
+    if (C > 1) MG_CUDA(cudaLaunchKernelEx(&cfg, route_fused_kernel<PP, true>, logits, bias, rp, xb, wb, d.hidden, idx, w, groups, C)); \
+    else MG_CUDA(cudaLaunchKernelEx(&cfg, route_fused_kernel<PP, false>, logits, bias, rp, xb, wb, d.hidden, idx, w, groups, 1)); \
+    break
   switch (P) {
     MG_ROUTE_CASE(1); MG_ROUTE_CASE(2); MG_ROUTE_CASE(4); MG_ROUTE_CASE(5); MG_ROUTE_CASE(8); MG_ROUTE_CASE(16);
   }

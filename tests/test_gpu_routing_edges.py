@@ -75,3 +75,61 @@ def test_forward_routes_as_the_staged_call(built_lib, gating, E, k, n_group, top
     assert torch.equal(view(1, (T, k), torch.int32), idx)
     assert torch.equal(view(2, (T, k), torch.float32), w)
     assert torch.equal(view(0, (T, E), torch.float32), logits)
+
+
+def _workspace(layer, which, T, shape, dtype):
+    off = layer.workspace_view(which, T) - layer._ws.data_ptr()
+    n = torch.Size(shape).numel() * 4
+    return layer._ws[off:off + n].view(dtype).view(shape)
+
+
+@pytest.mark.parametrize("gating,E,k,n_group,topk_group,lane_runs", [
+    (O.GATE_SOFTMAX_GREEDY, 64, 6, 1, 1, True), (O.GATE_SOFTMAX_GROUP_MAX, 160, 6, 8, 3, True),
+    (O.GATE_SIGMOID_NOAUX_TC, 256, 8, 8, 4, True), (O.GATE_SOFTMAX_GROUP_MAX, 96, 4, 4, 2, False)])
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 296, 297, 592, 593, 1184, 1185, 2500])
+def test_rows_with_many_logits_in_play_are_routed_by_the_exact_logits(built_lib, gating, E, k, n_group, topk_group,
+                                                                      lane_runs, T):
+    """Rows of zeros, tiny rows and rows with a few close logits among ordinary ones, alone and in runs, at the edges of
+    the cluster sizes: picks as from the correctly rounded logits.  Where the listing kernels' list of pairs holds, the
+    logits and weights are theirs bit for bit; where it overflows they recompute whole rows, and a logit out of play may
+    be off by the bound e of the router product, a weight by 2 e of itself (softmax; the sigmoid moves by e / 4, and its
+    share of the sum by twice that).  Groups of six lanes take the listing kernels either way."""
+    H = 1024
+    spec = O.LayerSpec(H, 128, E, k, 0, n_group, topk_group, gating, True, 1.0, O.WEIGHT_BF16, O.COMBINE_FP32)
+    g = torch.Generator().manual_seed(T)
+    gw = (torch.randn(E, H, generator=g) * 0.02).to(torch.bfloat16)
+    bias = torch.zeros(E) if gating == O.GATE_SIGMOID_NOAUX_TC else None
+    layer = make_layer(spec, O.LayerWeights(gw, bias))
+    base = torch.randn(T, H, generator=g).to(torch.bfloat16)
+    for name in ("ordinary", "zeros", "tail", "tiny", "scattered"):
+        x = base.clone()
+        if name == "zeros":
+            x[:] = 0
+        elif name == "tail":
+            x[T // 2:] = 0
+        elif name == "tiny":
+            x *= torch.tensor(2.0 ** -11, dtype=torch.bfloat16)
+        elif name == "scattered":
+            x[::5] = 0
+            x[1::5] *= torch.tensor(2.0 ** -9, dtype=torch.bfloat16)
+        x = x.cuda()
+        idx, w, logits, fix = layer.gate_route(x)
+        layer.forward(x)
+        torch.cuda.synchronize()
+        assert layer.device_status() == (0, 0)
+        got_idx, got_w = _workspace(layer, 1, T, (T, k), torch.int32), _workspace(layer, 2, T, (T, k), torch.float32)
+        exact = (x.double() @ gw.cuda().double().t()).float()
+        want = layer.route_topk(exact)[0]
+        assert torch.equal(got_idx.sort(1).values, want.sort(1).values), (name, T)
+        assert torch.equal(got_idx.sort(1).values, idx.sort(1).values), (name, T)
+        n_fix, n_rows, n_pairs = (int(v) for v in fix[:3])
+        if name == "zeros":                              # every token ties, with all its logits (or groups) in play
+            assert n_fix == T and (n_pairs > 0 or not lane_runs), (n_fix, n_rows, n_pairs)
+        if n_pairs <= 8 * T + 64 or not lane_runs:
+            assert torch.equal(got_w, w) and torch.equal(_workspace(layer, 0, T, (T, E), torch.float32), logits), name
+        else:
+            assert n_rows > 0
+            bound = 2 * (6.0e-9 * H + 4.0e-6) * max(1.0, float(exact.abs().max())) + 8 * 2.0 ** -24
+            order, ref = got_idx.argsort(1), idx.argsort(1)
+            a, b = got_w.gather(1, order), w.gather(1, ref)
+            assert float(((a - b).abs() / b.abs()).max()) <= bound, name
