@@ -1552,6 +1552,10 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   const bool m256 = p.b_fp8 && !pair && !f32_out && !dense && h->opt_fp8_m256 &&
                     p.a_rows >= static_cast<int64_t>(p.n_groups) * (h->opt_fp8_m256 == 2 ? 0 : 120 + 127);
   if (p.ring != nullptr) return launch_ring_gemm(h, p, st);
+  if (p.b_fp8) {
+    MG_REQUIRE(!f32_out && p.scales != nullptr && p.K % 128 == 0 && p.K <= 128 * 128, MG_ERR_SHAPE,
+               "FP8 weights need scales, K a multiple of 128 up to 16384 and a bf16 epilogue");
+  }
   // FP8 weights converted in the kernel, by default with the weights on the lanes: one conversion per 384 tokens of
   // an expert and MMAs as wide as its rows.  V3 shape, gate/up + down, ms before (128- or 256-row tiles) and now:
   // 64 tokens 3.3 and 2.3, 4096 skewed tokens 6.9 and 4.9, 16384 tokens 14.1 and 11.6.  MG_OPT_FP8_M256 = 0 or 2
@@ -1570,11 +1574,6 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
     rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32, TM_OUT_PIECE);
     if (rc != MG_OK) return rc;
   }
-  if (p.b_fp8) {
-    MG_REQUIRE(!f32_out && p.scales != nullptr && p.K % 128 == 0 && p.K <= 128 * 128, MG_ERR_SHAPE,
-               "FP8 weights need scales, K a multiple of 128 up to 16384 and a bf16 epilogue");
-  }
-
   GemmArgs a;
   a.pad_offsets = p.pad_offsets;
   a.counts = p.counts;

@@ -80,3 +80,18 @@ def test_shared_expert_at_job_edges(built_lib, T):
     hm = F.linear(h.abs(), wd.abs())
     err = (out.double() - F.linear(h, wd)).abs()
     assert bool((err <= 2.0 ** -8 * F.linear(h, wd).abs() + 2.0 ** -8 * hm).all())
+
+
+@pytest.mark.parametrize("form", [0, 1, 2])
+def test_inner_size_beyond_the_scale_row_is_refused_in_every_form(built_lib, form):
+    """FP8 weights converted in the kernel take K up to 16384, whichever form converts them."""
+    from moe_gen_b200 import MoELayer
+    from moe_gen_b200 import lib as L
+    layer = MoELayer(hidden=256, inter=16512, n_experts=4, top_k=2, weight_format=L.WEIGHT_FP8_BLOCK128, device="cuda:0")
+    layer.set_router(torch.zeros(4, 256))
+    layer.set_option(L.OPT_FP8_M256, form)
+    with pytest.raises(L.MoeGenError, match="K a multiple of 128 up to 16384") as e:
+        layer.forward(torch.zeros(3, 256, dtype=torch.bfloat16, device="cuda"))
+    assert e.value.code == -2
+    torch.cuda.synchronize()
+    assert layer.device_status() == (0, 0)
