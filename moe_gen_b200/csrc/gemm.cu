@@ -345,7 +345,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int ct = (cw >> 1) * 32 + lane;                 // 0..127 inside the group
     const int units = g.bn * (BK / 16);                   // 16-byte units of the FP8 tile
     uint32_t it = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
       const Tile t = locate_tile(tile, s_pad, s_cnt, g.n_groups, g.n_tiles, g.n_per_group, g.bn, g.group_m);
       const float* srow = g.scales + static_cast<long long>(t.b_row >> 7) * g.scale_cols;
       // one scale per 128 rows x 128 columns: rows [0,128) and [128,256) of the tile
@@ -388,10 +388,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int row_in_tile = quarter * 32 + lane;
     EpiWarp ew{epi_stage + quarter * 2 * EPI_PIECE_BYTES, 0u, lane, 2};
     uint32_t tcount = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const Tile t = locate_tile(tile, s_pad, s_cnt, g.n_groups, g.n_tiles, g.n_per_group, g.bn, g.group_m);
       const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
-      if (!mbar_wait(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 4)) break;
+      if (!mbar_wait_warp(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 4)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
       const bool live = row_in_tile < t.valid_rows;
@@ -615,7 +615,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     const uint32_t grp = cw & 1;
     const int ct = (cw >> 1) * 32 + lane;
     uint32_t it = 0;
-    for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs) {
+    for (int tile = pair; tile < total_tiles; tile += n_pairs) {
       const Tile2 t = locate_tile2(tile, s_pad, s_cnt, s_pp, g.n_groups, g.n_tiles, g.n_per_group);
       // the half tile is 128 rows = one scale block row
       const float* srow = g.scales + static_cast<long long>((t.b_row >> 7) + static_cast<int>(rank)) * g.scale_cols;
@@ -657,10 +657,10 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     const int row_in_half = quarter * 32 + lane;
     EpiWarp ew{epi_stage + quarter * 2 * EPI_PIECE_BYTES, 0u, lane, 2};
     uint32_t tcount = 0;
-    for (int tile = pair; tile < total_tiles && !*abort_flag; tile += n_pairs, ++tcount) {
+    for (int tile = pair; tile < total_tiles; tile += n_pairs, ++tcount) {
       const Tile2 t = locate_tile2(tile, s_pad, s_cnt, s_pp, g.n_groups, g.n_tiles, g.n_per_group);
       const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
-      if (!mbar_wait(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 14)) break;
+      if (!mbar_wait_warp(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 14)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
       const int my_rows = t.rows_left - static_cast<int>(rank) * BM;      // rows of my half that are real
@@ -913,7 +913,7 @@ grouped_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       fetch(ld, qb);
       fetch(ld, qc);
       fetch(ld, qd);
-      for (uint32_t it = 0; it < n_it && !*abort_flag; it += 4) {
+      for (uint32_t it = 0; it < n_it; it += 4) {
         if (!emit(cv, qa, it)) break;
         fetch(ld, qa);
         if (it + 1 >= n_it || !emit(cv, qb, it + 1)) break;
@@ -929,11 +929,11 @@ grouped_gemm_w8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const int quarter = warp & 3;
     EpiWarp ew{epi_stage + quarter * 2 * EPI_PIECE_BYTES, 0u, lane, 2};
     uint32_t tcount = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const Tile2 t = locate_w8<TM>(tile, s_pad, s_cnt, s_pp, g);
       const uint32_t acc = C::NACC == 2 ? (tcount & 1u) : 0u;
       const uint32_t acc_ph = C::NACC == 2 ? ((tcount >> 1) & 1u) : (tcount & 1u);
-      if (!mbar_wait(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 24)) break;
+      if (!mbar_wait_warp(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 24)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int sub = 0; sub < C::SUBS; ++sub) {
@@ -1293,10 +1293,10 @@ grouped_gemm_ring_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     const int row_in_tile = quarter * 32 + lane;
     EpiWarp ew{epi_stage + quarter * 2 * EPI_PIECE_BYTES, 0u, lane, 2};
     uint32_t tcount = 0;
-    for (int tile = blockIdx.x; tile < total_tiles && !*abort_flag; tile += gridDim.x, ++tcount) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tcount) {
       const RingTile t = locate_ring(tile, s_pad, s_cnt, s_gb, g, r);
       const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
-      if (!mbar_wait(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 46)) break;
+      if (!mbar_wait_warp(smem_u32(&tfull[acc]), acc_ph, abort_flag, g.status, 46)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
       const bool live = row_in_tile < t.valid_rows;
@@ -1320,21 +1320,37 @@ grouped_gemm_ring_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 }
 
 
-// Self-test of the bounded wait: one thread waits on a barrier that nothing will ever complete,
-// with a short limit; the wait must give up, record MG_DEV_WAIT_TIMEOUT and let the kernel end.
+// Self-test of the bounded waits on barriers that nothing will ever complete, with a short limit: the first warp waits
+// with one thread, the others as a warp-wide role does.  Each round of those completes its first barrier and waits on
+// one that stays open; the waits must give up, record MG_DEV_WAIT_TIMEOUT and let every warp reach the closing barrier.
+constexpr int PROBE_WARPS = 9;
 __global__ void wait_probe_kernel(unsigned long long limit_ns, int32_t* status) {
-  __shared__ uint64_t bar;
-  __shared__ int abort_flag;
+  __shared__ uint64_t never, pass[PROBE_WARPS];
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(smem_u32(&bar), 1);
-    abort_flag = 0;
+    mbar_init(smem_u32(&never), 1);
+    for (int i = 0; i < PROBE_WARPS; ++i) mbar_init(smem_u32(&pass[i]), 1);
+    abort_word = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_wait(smem_u32(&bar), 0, &abort_flag, status, 99, limit_ns);
   }
+  __syncthreads();
+  if (warp == 0) {
+    if (lane == 0) mbar_wait(smem_u32(&never), 0, abort_flag, status, 99, limit_ns);
+  } else {
+    for (uint32_t round = 0; round < 2; ++round) {
+      if (lane == 0) mbar_arrive(smem_u32(&pass[warp]));
+      if (!mbar_wait_warp(smem_u32(&pass[warp]), round & 1u, abort_flag, status, 99, limit_ns)) break;
+      if (!mbar_wait_warp(smem_u32(&never), 0, abort_flag, status, 99, limit_ns)) break;
+    }
+    __syncwarp();
+  }
+  __syncthreads();
 }
 
 int launch_wait_probe(const Handle* h, int limit_ms, cudaStream_t st) {
-  wait_probe_kernel<<<1, 32, 0, st>>>(static_cast<unsigned long long>(limit_ms) * 1000000ull, h->d_status);
+  wait_probe_kernel<<<1, 32 * PROBE_WARPS, 0, st>>>(static_cast<unsigned long long>(limit_ms) * 1000000ull, h->d_status);
   MG_CUDA(cudaGetLastError());
   return MG_OK;
 }

@@ -25,7 +25,11 @@
 //   aready/afree   the four 32-column slots of converted weights in TMEM; aready on the leader counts the
 //                  four warps of both CTAs, afree by commit to both
 //   dfull/dempty   accumulator halves; a job of more than HALF tokens takes both
-// Every wait is bounded (mbar_wait); on expiry the roles leave their loops and the kernel ends.
+// Every wait is bounded (mbar_wait); on expiry the roles leave their loops and the kernel ends.  The lanes of a
+// warp-wide role leave by the vote on a wait only, all at once: a lane that read the abort flag on its own would wait
+// at the closing barrier for lanes that wait for it in a warp-wide instruction, without a limit.  A role that gives
+// up has waited for the limit while the others could run ahead by a ring's length at most, so the loads still in
+// flight then were issued about as long ago and have landed.
 #include "tc.cuh"
 
 namespace mg {
@@ -347,7 +351,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     const int quarter = warp & 3;
     uint8_t* piece = pieces + (warp - 4) * WL_PIECE;
     uint32_t used0 = 0u, used1 = 0u, turn = 0u;
-    for (int job = pair; job < total_jobs && !*abort_flag; job += n_pairs) {
+    for (int job = pair; job < total_jobs; job += n_pairs) {
       const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
       const bool wide = j.n_tok > WL_HALF;
       const uint32_t h = wide ? 0u : turn;
@@ -395,7 +399,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     Ring rw;
     uint32_t slot = grp, ph = 0u;                          // this group's slots: grp, grp + 2
     bool ok = true;
-    for (int job = pair; job < total_jobs && ok && !*abort_flag; job += n_pairs) {
+    for (int job = pair; job < total_jobs && ok; job += n_pairs) {
       const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
       const float* srow = g.scales + static_cast<long long>((j.b_row >> 7) + block) * g.scale_cols;
       // 16 scales of this lane's row at a time, spread over its half of the warp and handed out by shuffle: a load

@@ -73,6 +73,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// The same for the roles that a whole warp plays, which leave their loops by this vote only: another role may raise the
+// flag, and the limit run out, between the readings of two lanes, and a lane that left on its own would wait at the
+// kernel's closing barrier for lanes that wait for it in a warp-wide instruction, without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status,
+                                               int where, unsigned long long limit_ns = WAIT_LIMIT_NS) {
+  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag, status, where, limit_ns)) != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1,
                                             uint32_t bar) {
   asm volatile(

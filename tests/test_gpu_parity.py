@@ -623,6 +623,19 @@ def test_bounded_wait_gives_up_and_reports(built_lib):
     assert O.rel_l2(y.cpu().float(), O.layer_forward(spec, x, W, gold_fp32=True)["y"]) <= TOL_LAYER
 
 
+def test_bounded_wait_of_whole_warps_ends_for_every_lane(built_lib):
+    """Warp-wide roles that run into the limit, or are told by another role, leave together: every launch ends, on
+    time, whichever lane or warp gives up first."""
+    import time
+    layer = make_layer(O.LayerSpec(256, 128, 8, 2), O.LayerWeights(torch.zeros(8, 256, dtype=torch.bfloat16), None), DEV)
+    for i in range(40):
+        t0 = time.time()
+        assert layer.lib.mg_selftest_wait_timeout(layer._h, 1 + i % 4, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert time.time() - t0 < 2.0
+        assert layer.device_status() == (1, 99) and layer.device_status() == (0, 0)
+
+
 @pytest.mark.parametrize("push", [False, True, "copy"])
 @pytest.mark.parametrize("dedup", [False, True])
 @pytest.mark.parametrize("n_ranks", [2, 4])
