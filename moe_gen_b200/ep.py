@@ -218,16 +218,12 @@ class EPMoELayer:
             nd = C.c_size_t()
             L.check(self.lib.mg_dequant_ws_bytes(lay._h, C.byref(nd)))
             # FP8: scratch for the library's FP8 mode (the L2-resident ring from 1024 rows per expert on, or
-            # the bf16 copy of pre-dequantise mode); below that the GEMMs convert in shared memory
+            # the bf16 copy of pre-dequantise mode); below that the GEMMs convert in the kernel
             mode = lay.options.get(L.OPT_FP8_MODE, 0)
             Tb = max(T, self._batch_tokens)    # parts of one batch share the de-quantised copy
             use_deq = nd.value > 0 and (mode in (L.FP8_PREDEQUANT, L.FP8_RING) or
                                         (mode == L.FP8_AUTO and Tb * self.world * k >= 1024 * E))
             self.deq = torch.empty(nd.value, dtype=torch.uint8, device=self.dev) if use_deq else None
-            if nd.value > 0 and L.OPT_FP8_M256 not in lay.options:
-                # the library picks the tile height of its convert-in-the-GEMM kernels from the rows of
-                # the buffer it is given; here that is the receive capacity, so decide from the batch
-                L.check(self.lib.mg_set_option(lay._h, L.OPT_FP8_M256, 2 if T * self.world * k >= 120 * E else 0))
             # rows the dispatch, duplicate-fill and combine kernels may address in a rank's buffers (looked at by
             # a -DMG_BOUNDS_CHECK build of the library only)
             L.check(self.lib.mg_set_option(lay._h, L.OPT_ROWS_BOUND, max(mb.cap for mb in self._mbs)))

@@ -191,3 +191,42 @@ def gpu_ep_worker(rank, world, port, spec, T_global, seed, result):
     ep_m.close()
     ep.close()
     dist.destroy_process_group()
+
+
+def gpu_ep_options_worker(rank, world, port, spec, T_global, result):
+    """Which library options the expert-parallel layer sets by itself, over batch sizes, and that a later plain forward
+    of the same layer gives the same bits."""
+    from moe_gen_b200.ep import EPMoELayer
+    from tests.util import make_layer
+    os.environ.setdefault("NCCL_NVLS_ENABLE", "0")
+    torch.cuda.set_device(rank)
+    _init(rank, world, port, "nccl")
+    x_all, W = O.make_inputs(spec, T_global, 4)
+    layer = make_layer(spec, W, f"cuda:{rank}", rank, world)
+
+    class Recorder:
+        def __init__(self, lib):
+            self.lib, self.options = lib, []
+
+        def __getattr__(self, name):
+            fn = getattr(self.lib, name)
+            if name != "mg_set_option":
+                return fn
+
+            def call(h, option, value):
+                self.options.append(option)
+                return fn(h, option, value)
+            return call
+    layer.lib = Recorder(layer.lib)
+    ep = EPMoELayer(layer)
+    same = True
+    for n in (T_global, 7, 1):
+        x = x_all[:n].to(f"cuda:{rank}")
+        y = ep.forward(x)
+        y1 = layer.forward(x)
+        torch.cuda.synchronize()
+        same = same and torch.equal(y.view(torch.int16), y1.view(torch.int16))
+    result["options"], result["same"], result["status"] = layer.lib.options, same, layer.device_status()
+    dist.barrier()
+    ep.close()
+    dist.destroy_process_group()

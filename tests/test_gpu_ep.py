@@ -43,3 +43,18 @@ def test_expert_parallel_on_gpus(built_lib, spec, T, world):
         assert all(r in (None, True) for r in result["overflow_reported"]), result["overflow_reported"]
         assert result["routing_agree"] > 0.995
         assert result["rel_l2"] <= 1e-2
+
+
+def test_expert_parallel_layer_leaves_the_form_of_the_fp8_gemms_alone(built_lib):
+    """The form of the kernels that convert FP8 weights is the library's default or the layer owner's choice; setting it
+    from the expert-parallel wrapper would also change what the layer does afterwards."""
+    from moe_gen_b200 import lib as L
+    spec = O.LayerSpec(256, 128, 16, 4, 128, 4, 2, O.GATE_SIGMOID_NOAUX_TC, True, 2.5, O.WEIGHT_FP8_BLOCK128, O.COMBINE_FP32)
+    ctx = mp.get_context("spawn")
+    with ctx.Manager() as mgr:
+        result = mgr.dict()
+        p = ctx.Process(target=ep_worker.gpu_ep_options_worker, args=(0, 1, _free_port(), spec, 900, result))
+        p.start()
+        assert ep_worker.join_all([p], 300) == [0]
+        assert result["options"] and L.OPT_FP8_M256 not in result["options"]
+        assert result["same"] and result["status"] == (0, 0)
