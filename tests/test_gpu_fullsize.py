@@ -9,6 +9,8 @@ The CPU oracle cannot run these sizes in test time, so each case is checked thro
     fp32-accumulated output),
 and the DeepSeek-V2-Lite configuration, which the reference itself runs on CPU, against the fixture
 recorded from the reference's DeepseekV2MoE at the full size (tests/golden/v2lite_full.npz)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -188,6 +190,12 @@ def test_named_configuration_at_full_shape(layers, name, T, zipf):
     yf = layer.forward(x)
     torch.cuda.synchronize()
     assert layer.device_status() == (0, 0)
+    # ... which the forward does in one pass: the same picks, weights and logits for every token
+    for which, listed in ((0, logits_f), (1, idx_f), (2, w_f)):
+        p = C.c_void_p()
+        assert layer.lib.mg_workspace_ptr(layer._h, layer._ws.data_ptr(), T, 0, which, C.byref(p)) == 0
+        off = p.value - layer._ws.data_ptr()
+        assert torch.equal(layer._ws[off:off + 4 * listed.numel()].view(listed.dtype).view(listed.shape), listed), which
     agree = ~differ[tokens]
     if bool(agree.any()):
         assert O.rel_l2(yf[tokens][agree].float().cpu(), ref[agree].cpu()) <= TOL_LAYER

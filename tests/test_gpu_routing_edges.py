@@ -32,6 +32,25 @@ def test_permute_plan_at_the_one_block_limit(built_lib, T, E, k):
     assert torch.equal(dst.cpu().long().view(-1), want)
 
 
+@pytest.mark.parametrize("gating", [O.GATE_SOFTMAX_GREEDY, O.GATE_SOFTMAX_TOPK_RENORM])
+@pytest.mark.parametrize("E", [36, 40, 100, 160, 252])
+def test_router_product_in_narrow_tiles_equals_the_wide_ones(built_lib, E, gating):
+    """32-column tiles while they fit one wave, at expert counts that are no multiple of 32: the same bits as rows of a
+    batch too large for them, fp32 and bf16-rounded logits, at the edges of the row tiles and of the rule."""
+    _, layer = _router_only(E, 4, gating=gating)
+    tiles = torch.cuda.get_device_properties(0).multi_processor_count // ((E + 31) // 32)       # row tiles of one wave
+    x = torch.randn(128 * tiles + 1, 256, generator=torch.Generator().manual_seed(E)).to(torch.bfloat16).cuda()
+    wide = layer.gate_logits(x)
+    exact = x.double() @ layer.gate_w.double().t()
+    # fp32 sums of 256 products in any order; bf16 logits round once more
+    bound = 256 * 2.0 ** -24 * (x.double().abs() @ layer.gate_w.double().abs().t())
+    if gating == O.GATE_SOFTMAX_TOPK_RENORM:
+        bound = bound + 2.0 ** -8 * exact.abs()
+    assert bool(((wide.double() - exact).abs() <= bound).all())
+    for T in (1, 127, 128, 129, 128 * tiles - 1, 128 * tiles):
+        assert torch.equal(layer.gate_logits(x[:T].contiguous()), wide[:T]), T
+
+
 @pytest.mark.parametrize("lo,n", [(0, 24), (5, 13)])
 @pytest.mark.parametrize("T", [1, 40, 256, 257, 700, 1024])
 def test_one_block_plan_of_repeated_and_foreign_picks_equals_the_general_plan(built_lib, T, lo, n):
@@ -55,14 +74,14 @@ def test_one_block_plan_of_repeated_and_foreign_picks_equals_the_general_plan(bu
     (O.GATE_SIGMOID_NOAUX_TC, 256, 8, 8, 4), (O.GATE_SOFTMAX_GROUP_MAX, 96, 4, 3, 2)])
 @pytest.mark.parametrize("T", [1, 8, 9, 700])
 def test_forward_routes_as_the_staged_call(built_lib, gating, E, k, n_group, topk_group, T):
-    """The forward's picks, weights and recomputed logits are those of the listing kernels, bit for bit; the last
-    configuration's groups are not runs of lanes."""
+    """The forward's picks, weights and logits are those of the staged call, bit for bit; every configuration's groups are
+    runs of lanes (8 in the last one).  Tokens that tie: the next test."""
     spec = O.LayerSpec(512, 128, E, k, 0, n_group, topk_group, gating, True, 1.0, O.WEIGHT_BF16, O.COMBINE_FP32)
     _, W = O.make_inputs(spec, 1, 7)
     layer = make_layer(spec, W)
     g = torch.Generator(device="cuda").manual_seed(T)
     x = torch.randn(T, 512, generator=g, device="cuda").to(torch.bfloat16)
-    x[T // 2:] = x[0]                                   # repeated tokens, and a few rows that nearly tie
+    x[T // 2:] = x[0]                                   # repeated tokens, and rows of a single column
     x[::3, 1:] = 0
     idx, w, logits, _ = layer.gate_route(x)
     layer.forward(x)
@@ -89,7 +108,7 @@ def _workspace(layer, which, T, shape, dtype):
 @pytest.mark.parametrize("T", [1, 7, 8, 9, 296, 297, 592, 593, 1184, 1185, 2500])
 def test_rows_with_many_logits_in_play_are_routed_by_the_exact_logits(built_lib, gating, E, k, n_group, topk_group,
                                                                       lane_runs, T):
-    """Rows of zeros, tiny rows and rows with a few close logits among ordinary ones, alone and in runs, at the edges of
+    """Rows of zeros (all, a few, the last half), tiny rows and rows with a few close logits among ordinary ones, alone and in runs, at the edges of
     the cluster sizes: picks as from the correctly rounded logits.  Where the listing kernels' list of pairs holds, the
     logits and weights are theirs bit for bit; where it overflows they recompute whole rows, and a logit out of play may
     be off by the bound e of the router product, a weight by 2 e of itself (softmax; the sigmoid moves by e / 4, and its
@@ -101,10 +120,12 @@ def test_rows_with_many_logits_in_play_are_routed_by_the_exact_logits(built_lib,
     bias = torch.zeros(E) if gating == O.GATE_SIGMOID_NOAUX_TC else None
     layer = make_layer(spec, O.LayerWeights(gw, bias))
     base = torch.randn(T, H, generator=g).to(torch.bfloat16)
-    for name in ("ordinary", "zeros", "tail", "tiny", "scattered"):
+    for name in ("ordinary", "zeros", "few", "tail", "tiny", "scattered"):
         x = base.clone()
         if name == "zeros":
             x[:] = 0
+        elif name == "few":
+            x[::97] = 0
         elif name == "tail":
             x[T // 2:] = 0
         elif name == "tiny":
@@ -124,7 +145,9 @@ def test_rows_with_many_logits_in_play_are_routed_by_the_exact_logits(built_lib,
         assert torch.equal(got_idx.sort(1).values, idx.sort(1).values), (name, T)
         n_fix, n_rows, n_pairs = (int(v) for v in fix[:3])
         if name == "zeros":                              # every token ties, with all its logits (or groups) in play
-            assert n_fix == T and (n_pairs > 0 or not lane_runs), (n_fix, n_rows, n_pairs)
+            assert n_fix == T and (n_pairs > 0 if lane_runs else n_rows == T), (n_fix, n_rows, n_pairs)
+        if name == "few":                                # the list holds them: compared bit for bit below
+            assert n_fix > 0 and (0 < n_pairs <= 8 * T + 64 or T < 296 or not lane_runs), (n_fix, n_pairs)
         if n_pairs <= 8 * T + 64 or not lane_runs:
             assert torch.equal(got_w, w) and torch.equal(_workspace(layer, 0, T, (T, E), torch.float32), logits), name
         else:

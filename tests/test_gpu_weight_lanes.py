@@ -1,6 +1,7 @@
-"""GPU: the expert GEMMs with the weights on the accumulator's lanes (gemm_wl.cu), at the edges of their jobs: no
-row, one row, multiples of 32 tokens and the rows around them, both accumulator halves, one job and several per
-expert.  Rows between the segments hold NaN, which must not reach a live row."""
+"""GPU: the expert GEMMs with the weights on the accumulator's lanes (gemm_wl.cu, FP8 weights), at the edges of their
+jobs: no row, one row, multiples of 32 tokens and the rows around them, both accumulator halves, one job and several per
+expert and per SM pair.  Rows between the segments hold NaN, which must not reach a live row.  The bf16 cases and the
+shared expert run the kernel with the tokens on the lanes (gemm.cu) at the same edges."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -95,3 +96,66 @@ def test_inner_size_beyond_the_scale_row_is_refused_in_every_form(built_lib, for
     assert e.value.code == -2
     torch.cuda.synchronize()
     assert layer.device_status() == (0, 0)
+
+
+def _random_fp8_layer(hidden, inter, n_experts, seed):
+    """A layer whose expert weights are random e4m3 values of every exponent below 2^5, drawn on the GPU."""
+    from moe_gen_b200 import MoELayer
+    from moe_gen_b200 import lib as L
+    layer = MoELayer(hidden=hidden, inter=inter, n_experts=n_experts, top_k=2, weight_format=L.WEIGHT_FP8_BLOCK128,
+                     device="cuda:0")
+    layer.set_router(torch.zeros(n_experts, hidden))
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    for e in range(n_experts):
+        mats, scales = [], []
+        for m, n in ((inter, hidden), (inter, hidden), (hidden, inter)):
+            byte = torch.randint(0, 0x60, (m, n), generator=g, device="cuda", dtype=torch.uint8)
+            sign = torch.randint(0, 2, (m, n), generator=g, device="cuda", dtype=torch.uint8)
+            mats.append((byte | (sign << 7)).view(torch.float8_e4m3fn))
+            scales.append(torch.rand(m // 128, n // 128, generator=g, device="cuda") * 0.01 + 0.001)
+        layer.load_expert(e, *mats, tuple(scales))
+    return layer
+
+
+# every pattern repeats over the experts: narrow jobs (up to 192 tokens, one accumulator half), jobs of one and of two
+# MMAs (up to 256 tokens, up to 384) and experts of several jobs next to one another
+PATTERNS = {
+    "mixed": [1, 384, 32, 193, 0, 256, 257, 192, 769, 64, 385, 5],
+    "narrow": [1, 33, 192, 0, 96, 31, 160, 8],
+    "wide_after_narrow": [7, 384, 7, 300, 7, 7, 224, 7],
+}
+
+
+@pytest.mark.parametrize("hidden,inter,n_experts", [(2304, 2176, 24), (512, 384, 256)])
+@pytest.mark.parametrize("pattern", sorted(PATTERNS))
+def test_several_jobs_per_sm_pair_equal_the_other_forms(built_lib, pattern, hidden, inter, n_experts):
+    """Rings, accumulator halves and scales carried from job to job: every SM pair gets several jobs of different
+    lengths, K passes the 16 scale columns a converter loads at a time and ends inside a group of them (18 and 17
+    columns).  Every live row has the same bits as with the tokens on the lanes and as with weights converted first."""
+    layer = _random_fp8_layer(hidden, inter, n_experts, 3)
+    counts = (PATTERNS[pattern] * n_experts)[:n_experts]
+    tiles = sum((c + 383) // 384 for c in counts)
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert tiles * (2 * inter // 256) > 3 * pairs or tiles * (hidden // 256) > 3 * pairs
+    cnt = torch.tensor(counts)
+    pad = torch.zeros(n_experts + 1, dtype=torch.int64)
+    pad[1:] = ((cnt + 127) // 128 * 128).cumsum(0)
+    rows = int(pad[-1]) + 128
+    x = torch.full((rows, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
+    live = torch.zeros(rows, dtype=torch.bool, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for e, c in enumerate(counts):
+        live[pad[e]:pad[e] + c] = True
+    x[live] = (torch.randn(int(live.sum()), hidden, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    pad_d, cnt_d = pad.int().cuda(), cnt.int().cuda()
+    got = layer.expert_ffn(x, pad_d, cnt_d)
+    again = layer.expert_ffn(x, pad_d, cnt_d)
+    first = layer.expert_ffn(x, pad_d, cnt_d, predequant=True)
+    layer.set_option(4, 0)
+    tokens_on_lanes = layer.expert_ffn(x, pad_d, cnt_d)
+    torch.cuda.synchronize()
+    assert layer.device_status() == (0, 0)
+    for which, out in enumerate(got):
+        assert bool(torch.isfinite(out[live].float()).all()) and bool((out[live] != 0).any())
+        for other in (again, first, tokens_on_lanes):
+            assert torch.equal(out[live].view(torch.int16), other[which][live].view(torch.int16)), which
