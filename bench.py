@@ -519,7 +519,7 @@ def main():
     ap.add_argument("--route-fixup", type=int, default=-1,
                     help="0 = route every token from the tensor-core router product as it is (no near-tie fix-up)")
     ap.add_argument("--fp8-mode", type=int, default=-1, help="0 auto, 1 pre-dequantise, 2 convert in the GEMM")
-    ap.add_argument("--fp8-tall", type=int, default=-1, help="convert-in-GEMM tile height: 0 128 rows, 1 auto, 2 256 rows")
+    ap.add_argument("--fp8-tall", type=int, default=-1, help="convert-in-GEMM form: 0 128-row tiles, 1 weights on the lanes, 2 256-row tiles")
     args = ap.parse_args()
 
     rank = int(os.environ.get("RANK", "0"))

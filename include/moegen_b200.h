@@ -463,8 +463,8 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
 /* Options (no counterpart in the reference).
  * MG_OPT_FP8_MODE, for MG_WEIGHT_FP8_BLOCK128 layers: where the grouped GEMMs get their bf16 operands
  * (the reference de-quantises every expert's matrices on every expert call, moe_gen/models/Wrapper.py:481-491):
- *   MG_FP8_IN_KERNEL   every CTA converts the FP8 weight tiles of its own row tiles in shared memory; no
- *                      scratch; a weight is converted once per 128 or 256 rows that use it;
+ *   MG_FP8_IN_KERNEL   the GEMM kernels convert the FP8 weight tiles they use; no scratch; a weight is
+ *                      converted once per 384 rows that use it (MG_OPT_FP8_M256: other forms);
  *   MG_FP8_PREDEQUANT  a bf16 copy of all local expert weights in scratch (2 bytes per weight), written by
  *                      a separate pass on a side stream one chunk of experts ahead of the bf16 GEMMs;
  *   MG_FP8_RING        the GEMM kernel's CTAs convert every weight once per expert into a bf16 ring of
@@ -472,7 +472,7 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
  *                      58 MB of scratch; measured 5 % slower than MG_FP8_PREDEQUANT at 65536 tokens of the
  *                      DeepSeek-V3 layer (the ring does not stay in L2), so only on request;
  *   MG_FP8_AUTO        (default) in-kernel while an expert sees fewer than 1024 rows on average
- *                      (measured cross-over on the DeepSeek-V3 shape), else pre-dequantise.
+ *                      (DeepSeek-V3 shape: 27.3 against 31.8 ms there, level at 2048 rows), else pre-dequantise.
  * All give bit-identical results.  Set before asking mg_workspace_bytes / mg_dequant_ws_bytes. */
 #define MG_OPT_FP8_MODE    1
 #define MG_FP8_AUTO        0

@@ -58,19 +58,21 @@ static size_t dequant_ws(const Handle* h) {
 }
 
 // How an FP8 layer's grouped GEMMs get bf16 operands (MG_OPT_FP8_MODE):
-//   in-kernel   every CTA converts the weight tiles of its own row tiles in shared memory: no scratch, but
-//               a weight is converted once per 128 or 256 rows that use it;
+//   in-kernel   the GEMM kernels convert the weight tiles they use: no scratch, but a weight is converted once
+//               per 384 rows that use it (MG_OPT_FP8_M256 = 0 or 2: per 128 or 256);
 //   pre-dequant a bf16 copy of all expert weights in scratch, written by a separate pass on a side stream;
 //   ring        the GEMM kernel's own CTAs convert every weight once per expert and share the bf16 copy
 //               through a ring of a few tens of MB (gemm.cu: grouped_gemm_ring_kernel): 58 MB of scratch
 //               instead of 2 bytes per weight.
-// AUTO: converting in the kernel re-does the work for every row tile of an expert; de-quantising first
-// moves every weight through HBM three more times.  On the DeepSeek-V3 shape converting (weights on the lanes,
-// gemm_wl.cu) wins below 1024 rows per expert (512 rows: 13.7 against 16.9 ms a forward); at 2048 rows the two
-// are equal within a box's drift (53.0 and 52.7 ms).  The ring was built to take the large batches without the HBM round
-// trip of the bf16 copy, but L2 does not hold it (measured at the benchmark size: 21.6 GB written to and
-// 35.2 GB read from DRAM by the gate/up launch, i.e. the ring goes through HBM like the separate pass's
-// copy does), and it ends 5 % behind pre-dequantise there; it is chosen only on request.
+// AUTO: converting in the kernel re-does the work for every 384 rows of an expert; de-quantising first moves every
+// weight through HBM three more times.  V3 layer, ms, de-quantised first and converted in the kernel (weights on the
+// lanes, gemm_wl.cu): 512 rows per expert 20.2 and 14.1, 768 rows 26.1 and 19.7, 1024 rows 31.8 and 27.3, 1536 rows
+// 43.1 and 40.8, 2048 rows 54.8 and 53.5 (skewed 56.0 and 53.0), where runs differ by 3 %.  The line at 1024 rows was
+// drawn for 256-row tiles (30.1 there); above it the two are now level or the kernel ahead, so it costs time and not
+// results.  The ring was built to take the large batches without the HBM round trip of the bf16 copy, but L2 does not
+// hold it (measured at the benchmark size: 21.6 GB written to and 35.2 GB read from DRAM by the gate/up launch, i.e.
+// the ring goes through HBM like the separate pass's copy does), and it ends 5 % behind pre-dequantise there; it is
+// chosen only on request.
 constexpr int64_t kRingMaxRows = 1ll << 24;          // rows the ring's counters are sized for
 static int fp8_mode_for(const Handle* h, int64_t rows) {
   if (h->d.weight_format != MG_WEIGHT_FP8_BLOCK128) return MG_FP8_IN_KERNEL;

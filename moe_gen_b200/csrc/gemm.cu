@@ -1547,7 +1547,10 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   int bn;
   const bool f32_out = p.epilogue == EPI_PLAIN_F32 || p.epilogue == EPI_ROUND_BF16_F32;
   // The router product of few tokens in 32-column tiles while those fit in one wave: at up to 128 tokens one CTA read
-  // all of the router (V3: 3.7 MB) alone.  Same bits; V3 at 64 tokens 53 -> 25 us together with the elected issue.
+  // all of the router (V3: 3.7 MB) alone.  Same bits.  us, wide tiles before the elected issue and this: V3 64 tokens
+  // 49 and 23, at the rule's upper end, where the rows are read by 8 CTAs, 2304 tokens 53 and 27; V2-236B 512 tokens 37
+  // and 20, 3712 tokens 40 and 23; 64 experts of 7168 columns 9472 tokens 55 and 39.  Wide tiles with the elected
+  // issue: V3 2305 tokens 52.
   const bool narrow = f32_out && dense && p.n_per_group > BN_NARROW &&
                       (p.dense_rows + BM - 1) / BM * ((p.n_per_group + BN_NARROW - 1) / BN_NARROW) <= h->sm_count;
   if (f32_out) {
@@ -1561,22 +1564,18 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   }
   // SM pairs (2-CTA tiles of 256 x 256) for the bf16 expert GEMMs when switched on
   const bool pair = h->opt_pair_gemm && !f32_out;
-  // FP8 weights converted in the kernel, tokens on the lanes (on request): 256-row tiles once experts average 120
-  // live rows (a_rows also counts up to 127 rows of padding per expert); below that most tall tiles
-  // would be half empty, the layer is bound by streaming the weights from HBM, and the 128-row
-  // kernel, whose FP8 bytes arrive by TMA, streams them faster than register loads do
-  const bool m256 = p.b_fp8 && !pair && !f32_out && !dense && h->opt_fp8_m256 &&
-                    p.a_rows >= static_cast<int64_t>(p.n_groups) * (h->opt_fp8_m256 == 2 ? 0 : 120 + 127);
   if (p.ring != nullptr) return launch_ring_gemm(h, p, st);
   if (p.b_fp8) {
     MG_REQUIRE(!f32_out && p.scales != nullptr && p.K % 128 == 0 && p.K <= 128 * 128, MG_ERR_SHAPE,
                "FP8 weights need scales, K a multiple of 128 up to 16384 and a bf16 epilogue");
   }
   // FP8 weights converted in the kernel, by default with the weights on the lanes: one conversion per 384 tokens of
-  // an expert and MMAs as wide as its rows.  V3 shape, gate/up + down, ms before (128- or 256-row tiles) and now:
-  // 64 tokens 3.3 and 2.3, 4096 skewed tokens 6.9 and 4.9, 16384 tokens 14.1 and 11.6.  MG_OPT_FP8_M256 = 0 or 2
-  // asks for the tiles with tokens on the lanes.
-  if (p.b_fp8 && !dense && !f32_out && !pair && h->opt_fp8_m256 == 1) return launch_gemm_wl(h, p, st);
+  // an expert and MMAs as wide as its rows.  V3 layer, ms, 128-row tiles / 256-row tiles / weights on the lanes: 64
+  // tokens 3.7 / 4.5 / 2.6, 4096 skewed tokens 8.0 / 7.7 / 5.5, 16384 tokens 20.5 / 16.3 / 14.1, 32768 tokens 37.4 /
+  // 30.1 / 27.3.  MG_OPT_FP8_M256 = 0 or 2 asks for the tiles with tokens on the lanes.
+  const bool convert = p.b_fp8 && !dense && !f32_out && !pair;
+  if (convert && h->opt_fp8_m256 == 1) return launch_gemm_wl(h, p, st);
+  const bool m256 = convert && h->opt_fp8_m256 == 2;
   CUtensorMap ta, tb;
   int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), m256 ? 2 * BM : BM, TM_BF16);
   if (rc != MG_OK) return rc;

@@ -303,7 +303,7 @@ def test_fp8_weights_converted_in_the_gemm_equal_dequantise_first(built_lib, H, 
             assert torch.equal(o1.cpu()[live].view(torch.int16), o2.cpu()[live].view(torch.int16)), (mode, ring_mib)
     layer.set_option(7, 56)
     layer.set_option(1, 0)
-    for tall in (0, 2, 1):                             # 128-row tiles, 256-row tiles, by expert size
+    for tall in (0, 2, 1):                             # 128-row tiles, 256-row tiles, weights on the lanes
         layer.set_option(4, tall)
         h4, o4 = layer.expert_ffn(perm, pad, counts, predequant=False)
         _status_ok(layer)
