@@ -9,22 +9,35 @@
 //     carries the FP8 bytes and the tokens only: per 64-element K step and SM 8 KiB + 8 KiB FP8 in and out and
 //     N/2 * 128 B of tokens in and out, where a bf16 tile built in shared memory adds 16-32 KiB each way.
 //
-// Measured on the DeepSeek-V3 shape, gate/up + down products, tokens on the lanes before and now: 64 tokens 3.3 and
-// 2.3 ms, 333 skewed 3.0 and 2.1, 4096 skewed 6.9 and 4.9, 16384 tokens 14.2 and 11.6; the same bits.  Decode reads
-// 10.0 GB in 2.3 ms, 4.3 TB/s of the measured 6.5: the bound there is the hand-over between converters and MMA
-// issuer, not HBM.  Jobs of 192, 256 and 320 tokens were up to 25 % slower at 2048 rows per expert (more
-// conversions), sixteen converter warps no faster than eight.
+// What bounds it.  Decode: the weights' bytes and the conversion, which share the step.  DeepSeek-V3 shape, 64 tokens,
+// gate/up + down products: 2.30 ms before and 1.80 ms with the five changes below, 5.6 TB/s of the measured 6.5 (without
+// the conversion 1.49 ms, the HBM rate).  From a few thousand tokens on: the 1000 W cap (SM clock 1.1-1.3 GHz), where
+// every weight byte moved and converted once more costs time: 16384 tokens 11.4 and 10.5 ms.  Jobs of at most 320, 256
+// and 192 tokens were 1, 9 and 14 % slower there; prefetching tokens or weights into L2 ahead of the rings 2 to 15 %.
+//   * two products by one packed multiplication (convert16): the converters are bound by issue slots, 2.8 instructions
+//     per element of which 2.5 are conversions and the product: 64 tokens 2.30 and 2.10 ms;
+//   * 128 K elements per hand-over: half as many waits, votes and commits per element, on both sides;
+//   * the list of jobs is made by one warp, ahead: a look-up by every role between two jobs stopped the pipeline for
+//     two thousand cycles, 13 % of a job of the down product (these two: 2.10 and 1.80 ms);
+//   * the epilogue reads the accumulator in the layout of 8x8 fragments, so that SwiGLU's two halves meet in one thread
+//     and stmatrix transposes: half the instructions and no shuffles (16384 tokens, down product 4.05 and 3.85 ms);
+//   * jobs alternate between the two ends of the accumulator columns and the next one starts as soon as the columns that
+//     both need have been read (3.85 and 3.80 ms; the clock falls as the tensor cores idle less).
+// Direct stores of the output from registers were slower than pieces staged for TMA (down product, 16384 tokens 4.5
+// against 4.0 ms).
 //
-// Roles per CTA: warp 0 = weight TMA, warp 1 = token TMA, warp 2 = MMA issuer (leader CTA), warp 3 = job table and
+// Roles per CTA: warp 0 = weight TMA, warp 1 = token TMA, warp 2 = MMA issuer (leader CTA), warp 3 = job list and
 // TMEM owner, warps 4-11 = epilogue (two per lane quarter, alternate 32-token chunks), warps 12-19 = converters: a
-// thread owns one lane = one weight row; warps 12-15 take the even 64-element K steps, 16-19 the odd ones.
+// thread owns one lane = one weight row; warps 12-15 take the even stages of 128 K elements, 16-19 the odd ones.
 //
 // Barriers (per CTA unless said otherwise):
-//   wfull/wempty   weight ring, stages of 128 rows x 128 K bytes, released by the converter warps
+//   wfull/wempty   weight ring, stages of 128 rows x 128 K bytes, released by the four converter warps that read it
 //   tfull/tempty   token ring; leader's tfull counts both CTAs' bytes, tempty by commit to both
-//   aready/afree   the four 32-column slots of converted weights in TMEM; aready on the leader counts the
-//                  four warps of both CTAs, afree by commit to both
-//   dfull/dempty   accumulator halves; a job of more than HALF tokens takes both
+//   aready/afree   the two 64-column slots of converted weights in TMEM, one per converter group; aready on the leader
+//                  counts the four warps of both CTAs, afree by commit to both
+//   dfull/dempty   accumulators of even and odd jobs, dempty once an epilogue has read all of one
+//   dpart          an epilogue has read the columns that the next job's accumulator shares with its own
+//   jfull/jempty   job list
 // Every wait is bounded (mbar_wait); on expiry the roles leave their loops and the kernel ends.  The lanes of a
 // warp-wide role leave by the vote on a wait only, all at once: a lane that read the abort flag on its own would wait
 // at the closing barrier for lanes that wait for it in a warp-wide instruction, without a limit.  A role that gives
@@ -41,18 +54,19 @@ constexpr int WL_GROUP_T = 8;                  // token tiles per L2 reuse group
 constexpr int WL_K = 64;                       // K elements per MMA step (one 128-byte swizzle row of bf16)
 constexpr int WL_T_STAGE = WL_MAX_TOKENS / 2 * WL_K * 2;      // 24 KiB: this CTA's half of the tokens
 constexpr int WL_W_STAGE = 128 * 128;          // 16 KiB: 128 rows of 64 bf16 or of 128 FP8
-constexpr int WL_A_SLOTS = 4;
-constexpr int WL_A_COLS = 32;                  // 64 bf16 per lane
+constexpr int WL_A_SLOTS = 2;                  // one per converter group
+constexpr int WL_A_COLS = 64;                  // 128 bf16 per lane
 
 constexpr int WL_SW = 6, WL_ST = 4;            // weight and token stages
 constexpr int WL_EPI_WARPS = 8, WL_CONV_WARPS = 8;
 constexpr int WL_THREADS = (4 + WL_EPI_WARPS + WL_CONV_WARPS) * 32;
-constexpr int WL_HALF = WL_MAX_TOKENS / 2;     // columns of an accumulator half
-constexpr int WL_A_COL0 = WL_MAX_TOKENS;       // converted weights above the accumulator
+constexpr int WL_A_COL0 = WL_MAX_TOKENS;       // converted weights above the accumulators
+static_assert(WL_SW % 2 == 0, "the two converter groups take alternate stages of the weight ring");
 constexpr int WL_RING_BYTES = WL_SW * WL_W_STAGE + WL_ST * WL_T_STAGE;
-constexpr int WL_PIECE = 2048;                 // epilogue staging per warp: 32 tokens x 32 outputs
-constexpr int WL_BARS = 2 * WL_SW + 2 * WL_ST + 2 * WL_A_SLOTS + 4;
-constexpr size_t WL_SMEM = 1024 + WL_RING_BYTES + WL_EPI_WARPS * WL_PIECE + 8 * WL_BARS + 16 + 4 * (3 * kMaxExperts + 3);
+constexpr int WL_PIECE = 1024;                 // epilogue staging: 32 tokens x 16 outputs or 16 tokens x 32 outputs
+constexpr int WL_JOBS = 4;                     // jobs announced ahead
+constexpr int WL_BARS = 2 * WL_SW + 2 * WL_ST + 2 * WL_A_SLOTS + 5 + 2 * WL_JOBS;
+constexpr size_t WL_SMEM = 1024 + WL_RING_BYTES + WL_EPI_WARPS * 2 * WL_PIECE + 8 * WL_BARS + 32 + 32 * WL_JOBS + 4 * (3 * kMaxExperts + 3);
 static_assert(WL_SMEM <= 232448, "shared memory exceeds the 227 KiB a CTA may have");
 
 struct WlArgs {
@@ -74,12 +88,14 @@ struct Ring {
   }
 };
 
-struct Job {
+struct alignas(16) Job {
   int row0;      // first token row
   int left;      // live tokens
-  int n_tok;     // left rounded up to 32: the MMA's N
+  int n_tok;     // left rounded up to 32: the MMA's N; 0: no further job
   int b_row;     // first of the 256 weight rows
   int n_idx;
+  int next_tok;  // n_tok of the job after this one
+  int pad[2];
 };
 
 // K steps that share one token stage: a job of few tokens packs several, so that the ring holds as many bytes in
@@ -88,7 +104,6 @@ __device__ __forceinline__ int steps_per_stage(int n_tok) {
   const int h = n_tok >> 1;
   return h <= 24 ? 8 : h <= 48 ? 4 : h <= 96 ? 2 : 1;
 }
-__device__ __forceinline__ int round32(int v) { return (v + 31) & ~31; }
 
 // s_jp[e] = token tiles of the experts before e
 __device__ __forceinline__ Job locate_job(int job, const int* s_pad, const int* s_cnt, const int* s_jp, const WlArgs& g) {
@@ -106,11 +121,13 @@ __device__ __forceinline__ Job locate_job(int job, const int* s_pad, const int* 
   const int gt = min(WL_GROUP_T, nt - grp * WL_GROUP_T);
   const int n = rem / gt;
   const int m = grp * WL_GROUP_T + (rem - n * gt);
-  const int size = round32((s_cnt[e] + nt - 1) / nt);      // tiles of one expert are equally long
+  const int units = (s_cnt[e] + 31) >> 5;                  // 32 tokens each, dealt out evenly over the expert's tiles
+  const int base = units / nt, more = units - base * nt;
+  const int first = (m * base + min(m, more)) * 32;
   Job j;
-  j.row0 = s_pad[e] + m * size;
-  j.left = min(size, s_cnt[e] - m * size);
-  j.n_tok = round32(j.left);
+  j.row0 = s_pad[e] + first;
+  j.n_tok = (base + (m < more ? 1 : 0)) * 32;
+  j.left = min(j.n_tok, s_cnt[e] - first);
   j.b_row = e * g.n_per_group + n * 256;
   j.n_idx = n;
   return j;
@@ -139,6 +156,19 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
 }
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// 32 FP8 values -> 16 words of bf16 pairs, kept where they stand: without the empty statement the compiler moves the
+// conversion below the next wait
+__device__ __forceinline__ void convert32(const uint4& q0, const uint4& q1, float s, uint32_t* o) {
+  uint4 w[4];
+  convert16(q0, s, w[0], w[1]);
+  convert16(q1, s, w[2], w[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    asm volatile("" : "+r"(w[i].x), "+r"(w[i].y), "+r"(w[i].z), "+r"(w[i].w));
+    o[4 * i] = w[i].x; o[4 * i + 1] = w[i].y; o[4 * i + 2] = w[i].z; o[4 * i + 3] = w[i].w;
+  }
+}
+
 // Arrival on the leader CTA's barrier with the default semantics (release at CTA scope).  What it announces is tensor
 // memory, ordered by tcgen05 fences; at cluster scope the release would first wait until every global store of
 // the warp has reached L2, microseconds per tile in the epilogue.
@@ -146,30 +176,24 @@ __device__ __forceinline__ void arrive_at_leader(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(smem_u32(bar), 0)) : "memory");
 }
 
-// 32 accumulator columns (tokens) of this thread's lane -> rows of the warp's staging piece, [token][output].
-// SwiGLU: lanes 0-15 of a warp hold gate rows, lanes 16-31 the up rows of the same 16 outputs; two tokens at a
-// time the halves trade values, lanes 0-15 finish token t and lanes 16-31 token t + 1.  The pieces are what the
-// TMA store's box wants: 32 rows of 16 outputs, or of 32 outputs with 64-byte swizzle; either way a warp's
-// 2-byte stores of one instruction fall into one run of 64 bytes.
-template <int EPI>
-__device__ __forceinline__ void stage_columns(const uint32_t (&v)[32], int lane, uint8_t* piece) {
-  if (EPI == EPI_SWIGLU_BF16) {
-    const bool up = lane >= 16;
-    uint8_t* dst = piece + (lane >> 4) * 32 + (lane & 15) * 2;
-#pragma unroll
-    for (int t = 0; t < 32; t += 2) {
-      const float a = __uint_as_float(v[t]), b = __uint_as_float(v[t + 1]);
-      const float got = __shfl_xor_sync(0xFFFFFFFFu, up ? a : b, 16);
-      const float h = up ? silu_f(got) * b : silu_f(a) * got;
-      *reinterpret_cast<__nv_bfloat16*>(dst + t * 32) = __float2bfloat16_rn(h);
-    }
-  } else {
-    const uint32_t chunk = lane >> 3, in_chunk = (lane & 7) * 2;
-#pragma unroll
-    for (int t = 0; t < 32; ++t)
-      *reinterpret_cast<__nv_bfloat16*>(piece + t * 64 + ((chunk ^ ((t >> 1) & 3)) << 4) + in_chunk) =
-          __float2bfloat16_rn(__uint_as_float(v[t]));
-  }
+// 16 lanes (weight rows) x 32 columns (tokens) of the accumulator in the layout of 8x8 fragments: registers 4x, 4x + 1
+// hold row lane / 4, tokens 8x + 2 (lane mod 4) and the next; 4x + 2, 4x + 3 the same of row lane / 4 + 8.
+__device__ __forceinline__ void tc_ld_16x32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+// four 8x8 fragments, transposed: fragment m's column i goes to the 16 bytes that lane 8m + i points at
+__device__ __forceinline__ void store_fragments(uint32_t addr, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(m0), "r"(m1),
+               "r"(m2), "r"(m3)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 template <int EPI>
@@ -180,7 +204,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* pieces = smem + WL_RING_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(pieces + WL_EPI_WARPS * WL_PIECE);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(pieces + WL_EPI_WARPS * 2 * WL_PIECE);
   uint64_t* wfull = bars;
   uint64_t* wempty = wfull + WL_SW;
   uint64_t* tfull = wempty + WL_SW;
@@ -189,9 +213,13 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   uint64_t* afree = aready + WL_A_SLOTS;
   uint64_t* dfull = afree + WL_A_SLOTS;
   uint64_t* dempty = dfull + 2;
+  uint64_t* dpart = dempty + 2;
+  uint64_t* jfull = dpart + 1;
+  uint64_t* jempty = jfull + WL_JOBS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + WL_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_pad = reinterpret_cast<int*>(tmem_slot + 4);
+  Job* s_job = reinterpret_cast<Job*>((reinterpret_cast<uintptr_t>(tmem_slot + 2) + 15) & ~uintptr_t(15));
+  int* s_pad = reinterpret_cast<int*>(s_job + WL_JOBS);
   int* s_cnt = s_pad + kMaxExperts + 1;
   int* s_jp = s_cnt + kMaxExperts + 1;
 
@@ -200,10 +228,15 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < WL_SW; ++s) { mbar_init(smem_u32(&wfull[s]), 1); mbar_init(smem_u32(&wempty[s]), WL_CONV_WARPS); }
+    for (int s = 0; s < WL_SW; ++s) { mbar_init(smem_u32(&wfull[s]), 1); mbar_init(smem_u32(&wempty[s]), WL_CONV_WARPS / 2); }
     for (int s = 0; s < WL_ST; ++s) { mbar_init(smem_u32(&tfull[s]), 1); mbar_init(smem_u32(&tempty[s]), 1); }
     for (int s = 0; s < WL_A_SLOTS; ++s) { mbar_init(smem_u32(&aready[s]), 8); mbar_init(smem_u32(&afree[s]), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&dfull[s]), 1); mbar_init(smem_u32(&dempty[s]), 2 * WL_EPI_WARPS); }
+    mbar_init(smem_u32(dpart), 2 * WL_EPI_WARPS);
+    for (int s = 0; s < WL_JOBS; ++s) {
+      mbar_init(smem_u32(&jfull[s]), 1);
+      mbar_init(smem_u32(&jempty[s]), 2 + (rank == 0 ? 1 : 0) + WL_EPI_WARPS + WL_CONV_WARPS);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -246,12 +279,29 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   const uint32_t w_base = smem_u32(smem);
   const uint32_t t_base = w_base + WL_SW * WL_W_STAGE;
 
+  // the next job, for a role of one thread and for a role of a warp; false: none left, or the kernel is being left
+  auto take_job = [&](Job& j, Ring& r) {
+    if (*abort_flag || !mbar_wait(smem_u32(&jfull[r.i]), r.ph, abort_flag, g.status, 60)) return false;
+    j = s_job[r.i];
+    mbar_arrive(smem_u32(&jempty[r.i]));
+    r.next(WL_JOBS);
+    return j.n_tok != 0;
+  };
+  auto take_job_warp = [&](Job& j, Ring& r) {
+    if (!wait_warp(smem_u32(&jfull[r.i]), r.ph, abort_flag, g.status, 61)) return false;
+    j = s_job[r.i];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&jempty[r.i]));
+    r.next(WL_JOBS);
+    return j.n_tok != 0;
+  };
+
   if (warp == 0) {
     // ---------------- weight TMA (both CTAs, own 128 rows) ----------------
     if (elect_one()) {
-      Ring r;
-      for (int job = pair; job < total_jobs && !*abort_flag; job += n_pairs) {
-        const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+      Ring r, rj;
+      Job j;
+      while (take_job(j, rj)) {
         // SwiGLU rows come in blocks of 128 gate then 128 up; this CTA takes 64 of each
         const int row_a = SWIGLU ? j.b_row + static_cast<int>(rank) * 64 : j.b_row + static_cast<int>(rank) * 128;
         const int row_b = row_a + (SWIGLU ? 128 : 64);
@@ -268,9 +318,9 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   } else if (warp == 1) {
     // ---------------- token TMA (both CTAs, own half of each MMA's N) ----------------
     if (elect_one()) {
-      Ring r;
-      for (int job = pair; job < total_jobs && !*abort_flag; job += n_pairs) {
-        const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+      Ring r, rj;
+      Job j;
+      while (take_job(j, rj)) {
         const int h1 = min(j.n_tok, 256) >> 1, h2 = (j.n_tok >> 1) - h1;
         const int row1 = j.row0 + static_cast<int>(rank) * h1, row2 = j.row0 + 256 + static_cast<int>(rank) * h2;
         const int kpt = steps_per_stage(j.n_tok);
@@ -295,97 +345,159 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   } else if (warp == 2) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     if (rank == 0 && elect_one()) {
-      Ring rt, ra;
-      uint32_t used0 = 0u, used1 = 0u, turn = 0u;      // uses of the accumulator halves
+      Ring rt, ra, rj;
+      uint32_t seq = 0u, parts = 0u;       // jobs, and waits for a part of the accumulator
+      int n_before = 0;
       // kind::f16: D fp32 (bit 4), A bf16 (bit 7), B bf16 (bit 10), both K-major, N>>3 at 17, M>>4 at 24
       const uint32_t id0 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(256 >> 4) << 24);
       bool ok = true;
-      for (int job = pair; job < total_jobs && ok && !*abort_flag; job += n_pairs) {
-        const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
-        const bool wide = j.n_tok > WL_HALF;
-        const uint32_t h = wide ? 0u : turn;
-        if (!wide) turn ^= 1u;
-        const bool take0 = wide || h == 0u, take1 = wide || h == 1u;
-        ok = (!take0 || mbar_wait(smem_u32(&dempty[0]), (used0 & 1u) ^ 1u, abort_flag, g.status, 53)) &&
-             (!take1 || mbar_wait(smem_u32(&dempty[1]), (used1 & 1u) ^ 1u, abort_flag, g.status, 53));
+      Job j;
+      while (take_job(j, rj)) {
+        const uint32_t h = seq & 1u;
+        ok = mbar_wait(smem_u32(&dempty[h]), ((seq >> 1) & 1u) ^ 1u, abort_flag, g.status, 53);
+        if (ok && n_before + j.n_tok > WL_MAX_TOKENS) ok = mbar_wait(smem_u32(dpart), parts++ & 1u, abort_flag, g.status, 62);
         if (!ok) break;
-        used0 += take0;
-        used1 += take1;
+        ++seq;
+        n_before = j.n_tok;
         tc_fence_after();
         const int n1 = min(j.n_tok, 256), n2 = j.n_tok - n1;
         const uint32_t id1 = id0 | (static_cast<uint32_t>(n1 >> 3) << 17), id2 = id0 | (static_cast<uint32_t>(n2 >> 3) << 17);
-        const uint32_t d = tmem_base + h * WL_HALF;
+        const uint32_t d = tmem_base + (h ? WL_MAX_TOKENS - j.n_tok : 0);
         const int kpt = steps_per_stage(j.n_tok), step_bytes = j.n_tok * 64;
         int in_stage = 0;
-        for (int kb = 0; kb < g.k_steps; ++kb) {
-          ok = (in_stage != 0 || mbar_wait(smem_u32(&tfull[rt.i]), rt.ph, abort_flag, g.status, 54)) &&
-               mbar_wait(smem_u32(&aready[ra.i]), ra.ph, abort_flag, g.status, 55);
+        for (int kb = 0; kb < g.k_steps; kb += 2) {
+          ok = mbar_wait(smem_u32(&aready[ra.i]), ra.ph, abort_flag, g.status, 55);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t tb = t_base + rt.i * WL_T_STAGE + in_stage * step_bytes;
-          const uint64_t db = make_smem_desc(tb);
-          const uint64_t db2 = make_smem_desc(tb + n1 * 64);
-          const uint32_t a = tmem_base + WL_A_COL0 + ra.i * WL_A_COLS;
 #pragma unroll
-          for (int k = 0; k < WL_K / 16; ++k) {
-            // 16 bf16 = 32 bytes = 2 sixteen-byte units inside the swizzle row, or 8 columns of tensor memory
-            const uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
-            tc_mma_pair_ts(d, a + 8 * k, db + 2 * k, id1, accumulate);
-            if (n2 > 0) tc_mma_pair_ts(d + 256, a + 8 * k, db2 + 2 * k, id2, accumulate);
+          for (int half = 0; half < 2; ++half) {
+            if (in_stage == 0) {
+              ok = mbar_wait(smem_u32(&tfull[rt.i]), rt.ph, abort_flag, g.status, 54);
+              if (!ok) break;
+              tc_fence_after();
+            }
+            const uint32_t tb = t_base + rt.i * WL_T_STAGE + in_stage * step_bytes;
+            const uint64_t db = make_smem_desc(tb);
+            const uint64_t db2 = make_smem_desc(tb + n1 * 64);
+            const uint32_t a = tmem_base + WL_A_COL0 + ra.i * WL_A_COLS + half * (WL_A_COLS / 2);
+#pragma unroll
+            for (int k = 0; k < WL_K / 16; ++k) {
+              // 16 bf16 = 32 bytes = 2 sixteen-byte units inside the swizzle row, or 8 columns of tensor memory
+              const uint32_t accumulate = (kb | half | k) != 0 ? 1u : 0u;
+              tc_mma_pair_ts(d, a + 8 * k, db + 2 * k, id1, accumulate);
+              if (n2 > 0) tc_mma_pair_ts(d + 256, a + 8 * k, db2 + 2 * k, id2, accumulate);
+            }
+            if (++in_stage == kpt || kb + half + 1 == g.k_steps) {
+              tc_commit_pair(smem_u32(&tempty[rt.i]));
+              rt.next(WL_ST);
+              in_stage = 0;
+            }
           }
+          if (!ok) break;
           tc_commit_pair(smem_u32(&afree[ra.i]));
-          if (++in_stage == kpt || kb + 1 == g.k_steps) {
-            tc_commit_pair(smem_u32(&tempty[rt.i]));
-            rt.next(WL_ST);
-            in_stage = 0;
-          }
           ra.next(WL_A_SLOTS);
         }
         if (!ok) break;
-        if (take0) tc_commit_pair(smem_u32(&dfull[0]));
-        if (take1) tc_commit_pair(smem_u32(&dfull[1]));
+        tc_commit_pair(smem_u32(&dfull[h]));
+      }
+    }
+  } else if (warp == 3) {
+    // ---------------- job list of this pair ----------------
+    // a look-up costs a binary search over the experts and two divisions, a thousand cycles and more where the issue
+    // slots are busy: done once here and ahead, not by every role between two jobs
+    if (elect_one()) {
+      Ring rj;
+      Job j, next;
+      j.n_tok = 0;
+      if (pair < total_jobs) j = locate_job(pair, s_pad, s_cnt, s_jp, g);
+      for (int job = pair + n_pairs;; job += n_pairs, rj.next(WL_JOBS)) {
+        next.n_tok = 0;
+        if (job < total_jobs) next = locate_job(job, s_pad, s_cnt, s_jp, g);
+        j.next_tok = next.n_tok;
+        if (!mbar_wait(smem_u32(&jempty[rj.i]), rj.ph ^ 1u, abort_flag, g.status, 59)) break;
+        s_job[rj.i] = j;
+        mbar_arrive(smem_u32(&jfull[rj.i]));
+        if (j.n_tok == 0) break;
+        j = next;
       }
     }
   } else if (warp >= 4 && warp < 4 + WL_EPI_WARPS) {
     // ---------------- epilogue (both CTAs, own 128 lanes) ----------------
     const int quarter = warp & 3;
-    uint8_t* piece = pieces + (warp - 4) * WL_PIECE;
-    uint32_t used0 = 0u, used1 = 0u, turn = 0u;
-    for (int job = pair; job < total_jobs; job += n_pairs) {
-      const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
-      const bool wide = j.n_tok > WL_HALF;
-      const uint32_t h = wide ? 0u : turn;
-      if (!wide) turn ^= 1u;
-      const bool take0 = wide || h == 0u, take1 = wide || h == 1u;
-      bool ok;
-      ok = (!take0 || mbar_wait(smem_u32(&dfull[0]), used0 & 1u, abort_flag, g.status, 56)) &&
-           (!take1 || mbar_wait(smem_u32(&dfull[1]), used1 & 1u, abort_flag, g.status, 56));
-      ok = __all_sync(0xFFFFFFFFu, ok);
-      if (!ok) break;
-      used0 += take0;
-      used1 += take1;
+    // two pieces of output rows per warp: one is filled while the other leaves
+    const uint32_t piece0 = smem_u32(pieces + (warp - 4) * 2 * WL_PIECE);
+    uint32_t piece = 0u;
+    auto next_piece = [&]() {
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
       __syncwarp();
+      return piece0 + piece * WL_PIECE;
+    };
+    auto send_piece = [&](int col, int row) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tma_store_2d(&tmC, col, row, piece0 + piece * WL_PIECE);
+      piece ^= 1u;
+    };
+    uint32_t seq = 0u;
+    Ring rj;
+    Job j;
+    while (take_job_warp(j, rj)) {
+      const uint32_t h = seq & 1u;
+      if (!wait_warp(smem_u32(&dfull[h]), (seq >> 1) & 1u, abort_flag, g.status, 56)) break;
+      ++seq;
       tc_fence_after();
       const int col0 = SWIGLU ? j.n_idx * 128 + static_cast<int>(rank) * 64 + quarter * 16
                               : j.n_idx * 256 + static_cast<int>(rank) * 128 + quarter * 32;
-      const uint32_t taddr = tmem_base + h * WL_HALF + (static_cast<uint32_t>(quarter * 32) << 16);
-      for (int c = (warp - 4) / 4 * 32; c < j.left; c += 64) {
-        uint32_t v[32];
-        tc_ld32(taddr + c, v);
-        // the store that last used this piece has finished reading it
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      const uint32_t taddr = tmem_base + (h ? WL_MAX_TOKENS - j.n_tok : 0) + (static_cast<uint32_t>(quarter * 32) << 16);
+      auto release = [&](uint64_t* bar) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_at_leader(bar);
+      };
+      // chunks of 32 tokens, those first that lie in the next job's columns: once all warps have read them, the next
+      // job's MMAs may start
+      const int chunks = j.n_tok >> 5, shared = j.next_tok == 0 ? 0 : max(0, j.n_tok + j.next_tok - WL_MAX_TOKENS) >> 5;
+      const int i0 = (warp - 4) >> 2;
+      if (shared > 0 && i0 >= shared) release(dpart);
+      if (i0 >= chunks) release(&dempty[h]);
+      for (int i = i0; i < chunks; i += 2) {
+        const int c = 32 * (h ? i : chunks - 1 - i);
+        uint32_t va[16], vb[16];                // lanes 0-15 and 16-31 of the quarter
+        tc_ld_16x32(taddr + c, va);
+        tc_ld_16x32(taddr + (16u << 16) + c, vb);
         tc_ld_wait();
-        __syncwarp();
-        stage_columns<EPI>(v, lane, piece);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) tma_store_2d(&tmC, col0, j.row0 + c, smem_u32(piece));
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (take0) arrive_at_leader(&dempty[0]);
-        if (take1) arrive_at_leader(&dempty[1]);
+        // this warp's share is in registers
+        if (i < shared && i + 2 >= shared) release(dpart);
+        if (i + 2 >= chunks) release(&dempty[h]);
+        if (SWIGLU) {
+          // va: gate rows, vb: the up rows of the same 16 outputs; a piece is 32 tokens x 16 outputs
+          uint32_t p[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            p[i] = pack_bf16(silu_f(__uint_as_float(va[2 * i])) * __uint_as_float(vb[2 * i]),
+                             silu_f(__uint_as_float(va[2 * i + 1])) * __uint_as_float(vb[2 * i + 1]));
+          const uint32_t dst = next_piece() + (8 * (lane >> 4) + (lane & 7)) * 32 + ((lane >> 3) & 1) * 16;
+          store_fragments(dst, p[0], p[1], p[2], p[3]);
+          store_fragments(dst + 512, p[4], p[5], p[6], p[7]);
+          send_piece(col0, j.row0 + c);
+        } else {
+          // two pieces of 16 tokens x 32 outputs, in the 64-byte swizzle of the store's tensor map
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (c + 16 * t >= j.left) break;
+            const uint32_t tok = lane & 7, m = lane >> 3;
+            const uint32_t dst = next_piece() + tok * 64 + ((m ^ ((tok >> 1) & 3)) << 4);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              const int i = 8 * t + 4 * x;
+              store_fragments(dst + x * 512, pack_bf16(__uint_as_float(va[i]), __uint_as_float(va[i + 1])),
+                              pack_bf16(__uint_as_float(va[i + 2]), __uint_as_float(va[i + 3])),
+                              pack_bf16(__uint_as_float(vb[i]), __uint_as_float(vb[i + 1])),
+                              pack_bf16(__uint_as_float(vb[i + 2]), __uint_as_float(vb[i + 3])));
+            }
+            send_piece(col0, j.row0 + c + 16 * t);
+          }
+        }
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -393,51 +505,53 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   } else if (warp >= 4 + WL_EPI_WARPS) {
     // ---------------- FP8 -> bf16 converters: shared -> registers -> tensor memory ----------------
     const int quarter = warp & 3;
-    const uint32_t grp = (warp - 4 - WL_EPI_WARPS) >> 2;   // even / odd 64-element K steps
+    const uint32_t grp = (warp - 4 - WL_EPI_WARPS) >> 2;   // even / odd stages, counted over all jobs
     const int row = !SWIGLU ? quarter * 32 + lane : quarter * 16 + (lane & 15) + (lane & 16) * 4;
     const int block = SWIGLU ? lane >> 4 : static_cast<int>(rank);      // scale block row of this lane's weights
-    Ring rw;
-    uint32_t slot = grp, ph = 0u;                          // this group's slots: grp, grp + 2
+    const uint32_t a_slot = tmem_base + WL_A_COL0 + grp * WL_A_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
+    const int stages = g.k_steps / 2;
+    Ring rw, rj;
+    rw.i = grp;
+    uint32_t ph = 0u;
+    int first = static_cast<int>(grp);
+    Job j;
     bool ok = true;
-    for (int job = pair; job < total_jobs && ok; job += n_pairs) {
-      const Job j = locate_job(job, s_pad, s_cnt, s_jp, g);
+    while (ok && take_job_warp(j, rj)) {
       const float* srow = g.scales + static_cast<long long>((j.b_row >> 7) + block) * g.scale_cols;
-      // 16 scales of this lane's row at a time, spread over its half of the warp and handed out by shuffle: a load
-      // per stage put an L2 round trip on every stage (decode gate/up product 3.3 instead of 1.5 ms)
       float s16 = 0.f;
-      for (int kb = 0; kb < g.k_steps / 2; ++kb) {
-        if ((kb & 15) == 0) s16 = kb + (lane & 15) < g.scale_cols ? __ldg(srow + kb + (lane & 15)) : 0.f;
-        const float s = __shfl_sync(0xFFFFFFFFu, s16, (lane & 16) | (kb & 15));
-        ok = mbar_wait(smem_u32(&wfull[rw.i]), rw.ph, abort_flag, g.status, 57);
-        ok = __all_sync(0xFFFFFFFFu, ok);
+      for (int kb = first; kb < stages; kb += 2) {
+        // the scales of this group's next 16 stages, spread over a lane's half of the warp and handed out by shuffle
+        const int in16 = ((kb - first) >> 1) & 15;
+        if (in16 == 0) s16 = kb + 2 * (lane & 15) < stages ? __ldg(srow + kb + 2 * (lane & 15)) : 0.f;
+        const float s = __shfl_sync(0xFFFFFFFFu, s16, (lane & 16) | in16);
+        ok = wait_warp(smem_u32(&wfull[rw.i]), rw.ph, abort_flag, g.status, 57);
         if (!ok) break;
         const uint8_t* src = smem + rw.i * WL_W_STAGE + row * 128;
-        uint4 q[4];
+        uint4 q[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint4*>(src + (((grp * 4 + i) ^ (row & 7)) << 4));
+        for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const uint4*>(src + ((i ^ (row & 7)) << 4));
         uint32_t o[32];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 lo, hi;
-          convert16(q[i], s, lo, hi);
-          o[8 * i] = lo.x; o[8 * i + 1] = lo.y; o[8 * i + 2] = lo.z; o[8 * i + 3] = lo.w;
-          o[8 * i + 4] = hi.x; o[8 * i + 5] = hi.y; o[8 * i + 6] = hi.z; o[8 * i + 7] = hi.w;
-        }
+        convert32(q[0], q[1], s, o);
+        convert32(q[2], q[3], s, o + 16);
+        ok = wait_warp(smem_u32(&afree[grp]), ph ^ 1u, abort_flag, g.status, 58);
+        if (!ok) break;
+        ph ^= 1u;
+        tc_fence_after();
+        tc_st32(a_slot, o);
+        uint32_t o2[32];
+        convert32(q[4], q[5], s, o2);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&wempty[rw.i]));
-        rw.next(WL_SW);
-        ok = mbar_wait(smem_u32(&afree[slot]), ph ^ 1u, abort_flag, g.status, 58);
-        ok = __all_sync(0xFFFFFFFFu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        tc_st32(tmem_base + WL_A_COL0 + slot * WL_A_COLS + (static_cast<uint32_t>(quarter * 32) << 16), o);
+        convert32(q[6], q[7], s, o2 + 16);
+        tc_st32(a_slot + WL_A_COLS / 2, o2);
+        rw.i += 2;
+        if (rw.i >= WL_SW) { rw.i -= WL_SW; rw.ph ^= 1u; }
         tc_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_at_leader(&aready[slot]);
-        slot ^= 2u;
-        if (slot == grp) ph ^= 1u;
+        if (lane == 0) arrive_at_leader(&aready[grp]);
       }
+      first = (first + stages) & 1;
     }
   }
 
@@ -481,8 +595,8 @@ int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
   if (rc != MG_OK) return rc;
   rc = encode_2d(h, &t16, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 16, TM_BF16);
   if (rc != MG_OK) return rc;
-  rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo), 32,
-                 swiglu ? TM_OUT_16 : TM_OUT_PIECE);
+  rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo),
+                 swiglu ? 32 : 16, swiglu ? TM_OUT_16 : TM_OUT_PIECE);
   if (rc != MG_OK) return rc;
   WlArgs a;
   a.pad_offsets = p.pad_offsets;

@@ -80,6 +80,10 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
                                                int where, unsigned long long limit_ns = WAIT_LIMIT_NS) {
   return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag, status, where, limit_ns)) != 0;
 }
+// The same with the common case, a barrier that all lanes find complete, kept to one vote.
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int where) {
+  return __all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)) || mbar_wait_warp(bar, parity, abort_flag, status, where);
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1,
                                             uint32_t bar) {
   asm volatile(
@@ -176,7 +180,8 @@ __device__ __forceinline__ void convert16(const uint4& q, float s, uint4& lo, ui
   for (int i = 0; i < 8; ++i) {
     __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2(p[i], __NV_E4M3);
     float2 f = __half22float2(*reinterpret_cast<__half2*>(&hr));
-    __nv_bfloat162 b = __floats2bfloat162_rn(__fmul_rn(f.x, s), __fmul_rn(f.y, s));
+    const float2 r = __fmul2_rn(f, make_float2(s, s));      // one instruction for the two products
+    __nv_bfloat162 b = __floats2bfloat162_rn(r.x, r.y);
     o[i] = *reinterpret_cast<uint32_t*>(&b);
   }
   lo = make_uint4(o[0], o[1], o[2], o[3]);
