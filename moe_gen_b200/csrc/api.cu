@@ -49,7 +49,7 @@ static int64_t padded_rows(const Handle* h, int64_t rows) {
 
 // workspace carving ---------------------------------------------------------------------
 enum { WS_LOGITS, WS_IDX, WS_W, WS_COUNTS, WS_OFFSETS, WS_PAD, WS_DST, WS_PERM, WS_H, WS_OUT, WS_PLAN,
-       WS_HS, WS_SHARED, WS_DEQ, WS_FIX, WS_N };
+       WS_HS, WS_SHARED, WS_DEQ, WS_FIX, WS_JOBS, WS_N };
 struct WsLayout { size_t off[WS_N]; size_t total; };
 
 static size_t dequant_ws(const Handle* h) {
@@ -131,6 +131,7 @@ static WsLayout ws_layout(const Handle* h, int64_t T, int64_t R) {
   take(WS_HS, static_cast<size_t>(T) * d.inter_shared * 2);
   take(WS_SHARED, d.inter_shared ? static_cast<size_t>(T) * d.hidden * 2 : 0);
   take(WS_FIX, route_fix_bytes(T));
+  take(WS_JOBS, kJobCounters * sizeof(int32_t));
   L.total = off;
   return L;
 }
@@ -551,7 +552,7 @@ static int join_return(Handle* h, cudaStream_t st) {
 
 static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const int32_t* counts, int64_t rows_padded,
                       const void* packed, void* h_buf, void* out_rows, void* deq, cudaStream_t st, int* launches,
-                      bool timed = false, const ReturnHook* hook = nullptr) {
+                      bool timed = false, const ReturnHook* hook = nullptr, int32_t* job_counters = nullptr) {
   if (hook != nullptr) {
     int rc0 = ensure_return_stream(h);
     if (rc0 != MG_OK) return rc0;
@@ -581,6 +582,7 @@ static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const i
     if (timed) mark(h, MG_STAGE_DEQUANT, st);
     p.a = perm_x; p.b = base + L.w13; p.n_groups = E; p.n_per_group = 2 * d.inter; p.K = d.hidden;
     p.pad_offsets = pad; p.counts = counts; p.out = h_buf; p.ldo = d.inter; p.epilogue = EPI_SWIGLU_BF16;
+    p.next_job = job_counters;
     p.b_fp8 = fp8;
     p.scales = fp8 ? reinterpret_cast<const float*>(base + L.s13) : nullptr;
     int rc = launch_grouped_gemm(h, p, st);
@@ -588,6 +590,7 @@ static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const i
     if (timed) mark(h, MG_STAGE_EXPERT_GEMM1, st);
     p.a = h_buf; p.b = base + L.w2; p.n_per_group = d.hidden; p.K = d.inter; p.out = out_rows; p.ldo = d.hidden;
     p.epilogue = EPI_PLAIN_BF16;
+    p.next_job = job_counters != nullptr ? job_counters + 1 : nullptr;
     p.scales = fp8 ? reinterpret_cast<const float*>(base + L.s2) : nullptr;
     if (hook != nullptr && mode != MG_FP8_RING) {
       // the down projection in parts of experts, each part's rows sent home while the next part computes
@@ -645,6 +648,7 @@ static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const i
       if (n <= 0) continue;
       if (!reuse) MG_CUDA(cudaStreamWaitEvent(st, which == 0 ? h->ev_w13[c] : h->ev_w2[c], 0));
       p.n_groups = n; p.pad_offsets = pad + lo; p.counts = counts + lo; p.b_fp8 = false; p.scales = nullptr;
+      p.next_job = job_counters != nullptr ? job_counters + which * kDequantChunks + c : nullptr;
       if (which == 0) {
         p.a = perm_x; p.b = w13 + static_cast<size_t>(lo) * 2 * d.inter * d.hidden; p.n_per_group = 2 * d.inter;
         p.K = d.hidden; p.out = h_buf; p.ldo = d.inter; p.epilogue = EPI_SWIGLU_BF16;
@@ -839,14 +843,16 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   }
   if (rc != MG_OK) return rc;
   mark(h, MG_STAGE_ROUTE_TOPK, st);
-  rc = launch_permute_plan(h, idx, T, 0, d.n_experts, counts, offsets, pad, dst, plan, st, &launches);
+  rc = launch_permute_plan(h, idx, T, 0, d.n_experts, counts, offsets, pad, dst, plan, st, &launches,
+                           reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]));
   if (rc != MG_OK) return rc;
   mark(h, MG_STAGE_PERMUTE_PLAN, st);
   rc = launch_permute_rows(h, d_x, dst, T, perm, st);
   if (rc != MG_OK) return rc;
   mark(h, MG_STAGE_PERMUTE_ROWS, st);
   launches += 1;
-  rc = expert_ffn(h, perm, pad, counts, padded_rows(h, T * d.top_k), d_packed, hbuf, orow, deq, st, &launches, true);
+  rc = expert_ffn(h, perm, pad, counts, padded_rows(h, T * d.top_k), d_packed, hbuf, orow, deq, st, &launches, true,
+                  nullptr, reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]));
   if (rc != MG_OK) return rc;
   if (shared_early) {
     MG_CUDA(cudaStreamWaitEvent(st, h->ev_shared_out, 0));

@@ -18,6 +18,7 @@ constexpr int kPeerShift = 24;       // expert-parallel destinations: rank << 24
 constexpr int kPeerRowMask = (1 << kPeerShift) - 1;
 constexpr int kSkipRow = -(1 << 30); // stays negative after the in-segment rank is added
 constexpr int kDequantChunks = 8;    // expert chunks of the overlapped FP8 de-quantisation
+constexpr int kJobCounters = 2 * kDequantChunks;   // one per expert GEMM launch of a forward
 constexpr int kStageSlots = 32;      // forwards whose per-stage times are kept for averaging
 
 // thread-local error text -------------------------------------------------------------
@@ -44,6 +45,32 @@ struct TensorMapCache {
     uint32_t box_rows, kind;
     CUtensorMap map;
   };
+  Entry e[kEntries];
+  int used = 0, next = 0;
+};
+
+// Tensor maps of a weight-lane GEMM launch (gemm_wl.cu).  Token rows are seen as [K / 64][rows][64], so that one copy
+// fetches all steps of a stage: with a copy per step and per 64 or 16 tokens the kernel's token role was late at 32 to 128
+// tokens per expert (V3, 4096 skewed tokens 4.89 against 4.77 ms).
+struct WlMaps {
+  CUtensorMap w;                // FP8: weights [blocks of 128 rows][128][K]; bf16: [8][blocks][16][K]
+  CUtensorMap t[8];             // 16 .. 128 tokens
+  CUtensorMap t2[4];            // 16 .. 64 tokens beyond the first 128, one step
+  CUtensorMap c;                // output pieces
+};
+struct WlMapCache {
+  static constexpr int kEntries = 24;      // a forward launches 2, with weights de-quantised first 16
+  struct Key {
+    const void *a, *b, *out;
+    int64_t a_rows, w_rows, ldo;
+    int K;
+    bool fp8, swiglu;
+    bool operator==(const Key& o) const {
+      return a == o.a && b == o.b && out == o.out && a_rows == o.a_rows && w_rows == o.w_rows && ldo == o.ldo && K == o.K &&
+             fp8 == o.fp8 && swiglu == o.swiglu;
+    }
+  };
+  struct Entry { Key key; WlMaps maps; };
   Entry e[kEntries];
   int used = 0, next = 0;
 };
@@ -97,6 +124,7 @@ struct Handle {
   int stage_calls;        // forwards recorded since timing was enabled
   cudaEvent_t stage_ev[kStageSlots][MG_STAGE_COUNT + 1];   // ring of event sets, one per forward
   mutable TensorMapCache tmaps;
+  mutable WlMapCache wl_maps;
 };
 constexpr uint32_t kMagic = 0x4d474232u;  // "MGB2"
 
@@ -120,7 +148,7 @@ int launch_route_fused(const Handle* h, const void* x, const void* gate_w, float
 size_t plan_ws_bytes(const Handle* h, int64_t T);
 int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expert_lo, int n_exp,
                         int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,
-                        void* ws, cudaStream_t st, int* launches);
+                        void* ws, cudaStream_t st, int* launches, int32_t* job_counters = nullptr);
 int launch_permute_plan_static(const Handle* h, const int32_t* idx, int64_t T, int expert_lo, int n_exp,
                                int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,
                                cudaStream_t st);
@@ -209,6 +237,7 @@ struct GemmProblem {
   void* out;              // bf16 or fp32
   int64_t ldo;            // elements between output rows
   int epilogue;
+  int32_t* next_job;           // weight-lane GEMM: zeroed counter its jobs are handed out by, or nullptr
   // W8A16 through the L2-resident ring (grouped FP8 weights only): scratch for the bf16 ring and its
   // 2 x max_granules counters, sized with ring_plan(); nullptr = not this path
   void* ring;

@@ -1409,6 +1409,22 @@ int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64_t rows
   return MG_OK;
 }
 
+int encode_map(CUtensorMap* map, const void* base, bool bytes, int rank, const uint64_t (&dims)[4],
+               const uint64_t (&strides)[3], const uint32_t (&box)[4]) {
+  EncodeTiledFn fn = get_encode_fn();
+  MG_REQUIRE(fn != nullptr, MG_ERR_DRIVER, "cuTensorMapEncodeTiled not available from the driver");
+  cuuint64_t d[4], s[3];
+  cuuint32_t b[4], estr[4];
+  for (int i = 0; i < 4; ++i) { d[i] = dims[i]; b[i] = box[i]; estr[i] = 1; if (i < 3) s[i] = strides[i]; }
+  CUresult r = fn(map, bytes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank,
+                  const_cast<void*>(base), d, s, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  MG_REQUIRE(r == CUDA_SUCCESS, MG_ERR_DRIVER, "cuTensorMapEncodeTiled failed (%d): %llu x %llu x %llu, box %u x %u x %u",
+             static_cast<int>(r), static_cast<unsigned long long>(dims[0]), static_cast<unsigned long long>(dims[1]),
+             static_cast<unsigned long long>(dims[2]), box[0], box[1], box[2]);
+  return MG_OK;
+}
+
 // the opt-in to more than 48 KiB of dynamic shared memory is a per-device attribute of the kernel:
 // set once per (kernel, device)
 template <typename K>

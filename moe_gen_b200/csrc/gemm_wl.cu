@@ -10,7 +10,7 @@
 //     N/2 * 128 B of tokens in and out, where a bf16 tile built in shared memory adds 16-32 KiB each way.
 //
 // What bounds it.  Decode: the weights' bytes and the conversion, which share the step.  DeepSeek-V3 shape, 64 tokens,
-// gate/up + down products: 2.30 ms before and 1.80 ms with the five changes below, 5.6 TB/s of the measured 6.5 (without
+// gate/up + down products: 2.30 ms before and 1.80 ms with the changes below, 5.6 TB/s of the measured 6.5 (without
 // the conversion 1.49 ms, the HBM rate).  From a few thousand tokens on: the 1000 W cap (SM clock 1.1-1.3 GHz), where
 // every weight byte moved and converted once more costs time: 16384 tokens 11.4 and 10.5 ms.  Jobs of at most 320, 256
 // and 192 tokens were 1, 9 and 14 % slower there; prefetching tokens or weights into L2 ahead of the rings 2 to 15 %.
@@ -21,8 +21,13 @@
 //     two thousand cycles, 13 % of a job of the down product (these two: 2.10 and 1.80 ms);
 //   * the epilogue reads the accumulator in the layout of 8x8 fragments, so that SwiGLU's two halves meet in one thread
 //     and stmatrix transposes: half the instructions and no shuffles (16384 tokens, down product 4.05 and 3.85 ms);
+//   * one copy per token stage, through a map that sees the rows as [K / 64][rows][64], instead of one per step and per 64
+//     or 16 tokens (4096 skewed tokens 4.89 and 4.77 ms);
 //   * jobs alternate between the two ends of the accumulator columns and the next one starts as soon as the columns that
 //     both need have been read (3.85 and 3.80 ms; the clock falls as the tensor cores idle less).
+//   * jobs are handed out by a counter (next_job), not in fixed turns: pairs that start late or get long jobs take fewer,
+//     and the jobs under way stay neighbours in the list, whose weights and tokens L2 then holds: V3 layer 16384 tokens
+//     13.1 and 11.9 ms, 65536 tokens 51 and 44, 4096 skewed 4.94 and 4.79.
 // Direct stores of the output from registers were slower than pieces staged for TMA (down product, 16384 tokens 4.5
 // against 4.0 ms).
 //
@@ -37,7 +42,7 @@
 //                  counts the four warps of both CTAs, afree by commit to both
 //   dfull/dempty   accumulators of even and odd jobs, dempty once an epilogue has read all of one
 //   dpart          an epilogue has read the columns that the next job's accumulator shares with its own
-//   jfull/jempty   job list
+//   jfull/jempty   the next job, for the roles of a CTA; mfull: its number, from the leader's list to the other CTA's
 // Every wait is bounded (mbar_wait); on expiry the roles leave their loops and the kernel ends.  The lanes of a
 // warp-wide role leave by the vote on a wait only, all at once: a lane that read the abort flag on its own would wait
 // at the closing barrier for lanes that wait for it in a warp-wide instruction, without a limit.  A role that gives
@@ -49,28 +54,36 @@ namespace mg {
 
 namespace {
 
-constexpr int WL_MAX_TOKENS = 384;             // tokens per job: 384 accumulator columns
 constexpr int WL_GROUP_T = 8;                  // token tiles per L2 reuse group (weight tiles vary slower inside)
 constexpr int WL_K = 64;                       // K elements per MMA step (one 128-byte swizzle row of bf16)
-constexpr int WL_T_STAGE = WL_MAX_TOKENS / 2 * WL_K * 2;      // 24 KiB: this CTA's half of the tokens
 constexpr int WL_W_STAGE = 128 * 128;          // 16 KiB: 128 rows of 64 bf16 or of 128 FP8
-constexpr int WL_A_SLOTS = 2;                  // one per converter group
+constexpr int WL_A_SLOTS = 2;                  // FP8: converted weights, one slot per converter group
 constexpr int WL_A_COLS = 64;                  // 128 bf16 per lane
-
-constexpr int WL_SW = 6, WL_ST = 4;            // weight and token stages
 constexpr int WL_EPI_WARPS = 8, WL_CONV_WARPS = 8;
-constexpr int WL_THREADS = (4 + WL_EPI_WARPS + WL_CONV_WARPS) * 32;
-constexpr int WL_A_COL0 = WL_MAX_TOKENS;       // converted weights above the accumulators
-static_assert(WL_SW % 2 == 0, "the two converter groups take alternate stages of the weight ring");
-constexpr int WL_RING_BYTES = WL_SW * WL_W_STAGE + WL_ST * WL_T_STAGE;
 constexpr int WL_PIECE = 1024;                 // epilogue staging: 32 tokens x 16 outputs or 16 tokens x 32 outputs
-constexpr int WL_JOBS = 4;                     // jobs announced ahead
-constexpr int WL_BARS = 2 * WL_SW + 2 * WL_ST + 2 * WL_A_SLOTS + 5 + 2 * WL_JOBS;
-constexpr size_t WL_SMEM = 1024 + WL_RING_BYTES + WL_EPI_WARPS * 2 * WL_PIECE + 8 * WL_BARS + 32 + 32 * WL_JOBS + 4 * (3 * kMaxExperts + 3);
-static_assert(WL_SMEM <= 232448, "shared memory exceeds the 227 KiB a CTA may have");
+constexpr int WL_JOBS = 1;                     // announced ahead: few, so that the last jobs go to whoever is free
+constexpr int WL_MAIL = 4;                     // job numbers on their way from the leader to the other CTA
+template <bool FP8>
+struct WlCfg {
+  static constexpr int MAX_TOKENS = 384;                       // per job
+  // Weight and token stages.  bf16, ms at 8 and 3, 6 and 4, 5 and 5 stages: V2-236B 512 tokens 1.265, 1.302, 1.31, 2048
+  // tokens 1.55, 1.59, 1.63, 32768 tokens 11.3, -, 11.9; Mixtral 2048 tokens 1.54, 1.52, 1.53.  With jobs of at most 256
+  // tokens (8 and 4) V2-236B 8192 tokens 4.2 against 3.3.
+  static constexpr int SW = FP8 ? 6 : 8, ST = FP8 ? 4 : 3;
+  static constexpr int T_STAGE = MAX_TOKENS / 2 * WL_K * 2;    // this CTA's half of the tokens
+  static constexpr int THREADS = (4 + WL_EPI_WARPS + (FP8 ? WL_CONV_WARPS : 0)) * 32;
+  static constexpr int ACC_COLS = FP8 ? MAX_TOKENS : 512;      // accumulator columns; FP8: converted weights above them
+  static constexpr int RING_BYTES = SW * WL_W_STAGE + ST * T_STAGE;
+  static constexpr int BARS = 5 + 2 * WL_JOBS + 2 * (SW + ST + WL_A_SLOTS) + WL_MAIL;
+  static constexpr size_t SMEM = 1024 + RING_BYTES + WL_EPI_WARPS * 2 * WL_PIECE + 8 * BARS + 32 + 32 * WL_JOBS + 4 * WL_MAIL +
+                                 4 * (3 * kMaxExperts + 3);
+  static_assert(SMEM <= 232448, "shared memory exceeds the 227 KiB a CTA may have");
+};
+static_assert(WlCfg<true>::SW % 2 == 0, "the two converter groups take alternate stages of the weight ring");
 
 struct WlArgs {
-  const int32_t* pad_offsets;
+  const int32_t* pad_offsets;   // nullptr: dense, one group
+  int dense_rows;
   const int32_t* counts;
   int n_groups;
   int n_tiles;                  // 256-row weight tiles per group
@@ -78,6 +91,7 @@ struct WlArgs {
   int k_steps;                  // K / 64
   const float* scales;          // [rows / 128][K / 128]
   int scale_cols;
+  int32_t* next_job;            // counts the jobs handed out beyond each pair's first; nullptr: every n_pairs-th job
   int32_t* status;
 };
 
@@ -94,15 +108,15 @@ struct alignas(16) Job {
   int n_tok;     // left rounded up to 32: the MMA's N; 0: no further job
   int b_row;     // first of the 256 weight rows
   int n_idx;
-  int next_tok;  // n_tok of the job after this one
-  int pad[2];
+  int pad[3];
 };
 
-// K steps that share one token stage: a job of few tokens packs several, so that the ring holds as many bytes in
-// flight as a job of many
-__device__ __forceinline__ int steps_per_stage(int n_tok) {
-  const int h = n_tok >> 1;
-  return h <= 24 ? 8 : h <= 48 ? 4 : h <= 96 ? 2 : 1;
+// K steps that share a token stage, for h tokens per CTA: a job of few tokens packs several, so that the ring holds as
+// many bytes in flight as a job of many
+template <bool FP8>
+__host__ __device__ constexpr int steps_per_stage(int h) {
+  const int fit = WlCfg<FP8>::T_STAGE / (h * WL_K * 2);
+  return fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
 }
 
 // s_jp[e] = token tiles of the experts before e
@@ -196,30 +210,32 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WL_THREADS, 1)
-grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmT64,
-                       const __grid_constant__ CUtensorMap tmT16, const __grid_constant__ CUtensorMap tmC, const WlArgs g) {
+template <int EPI, bool FP8>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WlCfg<FP8>::THREADS, 1)
+grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
+  using C = WlCfg<FP8>;
   constexpr bool SWIGLU = EPI == EPI_SWIGLU_BF16;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* pieces = smem + WL_RING_BYTES;
+  uint8_t* pieces = smem + C::RING_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(pieces + WL_EPI_WARPS * 2 * WL_PIECE);
-  uint64_t* wfull = bars;
-  uint64_t* wempty = wfull + WL_SW;
-  uint64_t* tfull = wempty + WL_SW;
-  uint64_t* tempty = tfull + WL_ST;
-  uint64_t* aready = tempty + WL_ST;
-  uint64_t* afree = aready + WL_A_SLOTS;
-  uint64_t* dfull = afree + WL_A_SLOTS;
+  uint64_t* dfull = bars;
   uint64_t* dempty = dfull + 2;
   uint64_t* dpart = dempty + 2;
   uint64_t* jfull = dpart + 1;
   uint64_t* jempty = jfull + WL_JOBS;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + WL_BARS);
+  uint64_t* wfull = jempty + WL_JOBS;
+  uint64_t* wempty = wfull + C::SW;
+  uint64_t* tfull = wempty + C::SW;
+  uint64_t* tempty = tfull + C::ST;
+  uint64_t* aready = tempty + C::ST;                 // FP8
+  uint64_t* afree = aready + WL_A_SLOTS;
+  uint64_t* mfull = afree + WL_A_SLOTS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   Job* s_job = reinterpret_cast<Job*>((reinterpret_cast<uintptr_t>(tmem_slot + 2) + 15) & ~uintptr_t(15));
-  int* s_pad = reinterpret_cast<int*>(s_job + WL_JOBS);
+  int* s_mail = reinterpret_cast<int*>(s_job + WL_JOBS);
+  int* s_pad = s_mail + WL_MAIL;
   int* s_cnt = s_pad + kMaxExperts + 1;
   int* s_jp = s_cnt + kMaxExperts + 1;
 
@@ -228,19 +244,26 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < WL_SW; ++s) { mbar_init(smem_u32(&wfull[s]), 1); mbar_init(smem_u32(&wempty[s]), WL_CONV_WARPS / 2); }
-    for (int s = 0; s < WL_ST; ++s) { mbar_init(smem_u32(&tfull[s]), 1); mbar_init(smem_u32(&tempty[s]), 1); }
-    for (int s = 0; s < WL_A_SLOTS; ++s) { mbar_init(smem_u32(&aready[s]), 8); mbar_init(smem_u32(&afree[s]), 1); }
+    for (int s = 0; s < C::SW; ++s) { mbar_init(smem_u32(&wfull[s]), 1); mbar_init(smem_u32(&wempty[s]), FP8 ? WL_CONV_WARPS / 2 : 1); }
+    for (int s = 0; s < C::ST; ++s) { mbar_init(smem_u32(&tfull[s]), 1); mbar_init(smem_u32(&tempty[s]), 1); }
+    if (FP8)
+      for (int s = 0; s < WL_A_SLOTS; ++s) { mbar_init(smem_u32(&aready[s]), 8); mbar_init(smem_u32(&afree[s]), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&dfull[s]), 1); mbar_init(smem_u32(&dempty[s]), 2 * WL_EPI_WARPS); }
     mbar_init(smem_u32(dpart), 2 * WL_EPI_WARPS);
     for (int s = 0; s < WL_JOBS; ++s) {
       mbar_init(smem_u32(&jfull[s]), 1);
-      mbar_init(smem_u32(&jempty[s]), 2 + (rank == 0 ? 1 : 0) + WL_EPI_WARPS + WL_CONV_WARPS);
+      mbar_init(smem_u32(&jempty[s]), 2 + (rank == 0 ? 1 : 0) + WL_EPI_WARPS + (FP8 ? WL_CONV_WARPS : 0));
     }
+    for (int s = 0; s < WL_MAIL; ++s) mbar_init(smem_u32(&mfull[s]), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) { s_pad[i] = g.pad_offsets[i]; s_cnt[i] = g.counts[i]; }
+  if (g.pad_offsets != nullptr) {
+    for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) { s_pad[i] = g.pad_offsets[i]; s_cnt[i] = g.counts[i]; }
+  } else if (threadIdx.x == 0) {
+    s_pad[0] = 0;
+    s_cnt[0] = g.dense_rows;
+  }
   __syncthreads();
   if (warp == 3) {
     // token tiles before each expert: lane sums of runs of 16 experts, warp scan, runs written out
@@ -248,7 +271,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     int sum = 0;
     for (int i = 0; i < RUN; ++i) {
       const int e = lane * RUN + i;
-      if (e < g.n_groups) sum += (s_cnt[e] + WL_MAX_TOKENS - 1) / WL_MAX_TOKENS;
+      if (e < g.n_groups) sum += (s_cnt[e] + C::MAX_TOKENS - 1) / C::MAX_TOKENS;
     }
     int inc = sum;
 #pragma unroll
@@ -261,7 +284,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       const int e = lane * RUN + i;
       if (e < g.n_groups) {
         s_jp[e] = run;
-        run += (s_cnt[e] + WL_MAX_TOKENS - 1) / WL_MAX_TOKENS;
+        run += (s_cnt[e] + C::MAX_TOKENS - 1) / C::MAX_TOKENS;
         if (e == g.n_groups - 1) s_jp[g.n_groups] = run;
       }
     }
@@ -277,7 +300,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   const uint32_t tmem_base = *tmem_slot;
   const int total_jobs = s_jp[g.n_groups] * g.n_tiles;
   const uint32_t w_base = smem_u32(smem);
-  const uint32_t t_base = w_base + WL_SW * WL_W_STAGE;
+  const uint32_t t_base = w_base + C::SW * WL_W_STAGE;
 
   // the next job, for a role of one thread and for a role of a warp; false: none left, or the kernel is being left
   auto take_job = [&](Job& j, Ring& r) {
@@ -302,16 +325,25 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       Ring r, rj;
       Job j;
       while (take_job(j, rj)) {
-        // SwiGLU rows come in blocks of 128 gate then 128 up; this CTA takes 64 of each
-        const int row_a = SWIGLU ? j.b_row + static_cast<int>(rank) * 64 : j.b_row + static_cast<int>(rank) * 128;
-        const int row_b = row_a + (SWIGLU ? 128 : 64);
-        for (int kb = 0; kb < g.k_steps / 2; ++kb, r.next(WL_SW)) {
-          if (!mbar_wait(smem_u32(&wempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 51)) break;
-          const uint32_t fb = smem_u32(&wfull[r.i]);
-          const uint32_t dst = w_base + r.i * WL_W_STAGE;
-          mbar_expect_tx(fb, WL_W_STAGE);
-          tma_load_2d(dst, &tmW, kb * 128, row_a, fb);
-          tma_load_2d(dst + 64 * 128, &tmW, kb * 128, row_b, fb);
+        const int blk = j.b_row >> 7, r0 = static_cast<int>(rank);
+        if (FP8) {
+          // SwiGLU rows come in blocks of 128 gate then 128 up; this CTA takes 64 of each
+          for (int kb = 0; kb < g.k_steps / 2; ++kb, r.next(C::SW)) {
+            if (!mbar_wait(smem_u32(&wempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 51)) break;
+            const uint32_t fb = smem_u32(&wfull[r.i]), dst = w_base + r.i * WL_W_STAGE;
+            mbar_expect_tx(fb, WL_W_STAGE);
+            if (SWIGLU) tma_load_3d(dst, &maps.w, kb * 128, r0 * 64, blk, fb);
+            else tma_load_3d(dst, &maps.w, kb * 128, 0, blk + r0, fb);
+          }
+        } else {
+          for (int kb = 0; kb < g.k_steps; ++kb, r.next(C::SW)) {
+            if (!mbar_wait(smem_u32(&wempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 51)) break;
+            const uint32_t fb = smem_u32(&wfull[r.i]), dst = w_base + r.i * WL_W_STAGE;
+            if (rank == 0) mbar_expect_tx(fb, 2 * WL_W_STAGE);           // of both CTAs
+            // SwiGLU: 16 gate rows, the 16 up rows of the same outputs, the next 16 gate rows ...
+            if (SWIGLU) tma_load_4d_pair(dst, &maps.w, kb * WL_K, 0, blk, r0 * 4, fb);
+            else tma_load_4d_pair(dst, &maps.w, kb * WL_K, 0, blk + r0, 0, fb);
+          }
         }
       }
     }
@@ -323,22 +355,16 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       while (take_job(j, rj)) {
         const int h1 = min(j.n_tok, 256) >> 1, h2 = (j.n_tok >> 1) - h1;
         const int row1 = j.row0 + static_cast<int>(rank) * h1, row2 = j.row0 + 256 + static_cast<int>(rank) * h2;
-        const int kpt = steps_per_stage(j.n_tok);
-        for (int kb0 = 0; kb0 < g.k_steps; kb0 += kpt, r.next(WL_ST)) {
+        const int kpt = steps_per_stage<FP8>(j.n_tok >> 1);
+        const CUtensorMap* m1 = &maps.t[(h1 >> 4) - 1];
+        const CUtensorMap* m2 = &maps.t2[(max(h2, 16) >> 4) - 1];
+        for (int kb = 0; kb < g.k_steps; kb += kpt, r.next(C::ST)) {
           if (!mbar_wait(smem_u32(&tempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 52)) break;
-          const int kbs = min(kpt, g.k_steps - kb0);
           const uint32_t fb = smem_u32(&tfull[r.i]);
-          if (rank == 0) mbar_expect_tx(fb, kbs * j.n_tok * 128);
-          for (int i = 0; i < kbs; ++i) {
-            const uint32_t dst = t_base + r.i * WL_T_STAGE + i * (h1 + h2) * 128;
-            const int kx = (kb0 + i) * WL_K;
-            int o = 0;
-            for (; o + 64 <= h1; o += 64) tma_load_2d_pair(dst + o * 128, &tmT64, kx, row1 + o, fb);
-            for (; o < h1; o += 16) tma_load_2d_pair(dst + o * 128, &tmT16, kx, row1 + o, fb);
-            o = 0;
-            for (; o + 64 <= h2; o += 64) tma_load_2d_pair(dst + (h1 + o) * 128, &tmT64, kx, row2 + o, fb);
-            for (; o < h2; o += 16) tma_load_2d_pair(dst + (h1 + o) * 128, &tmT16, kx, row2 + o, fb);
-          }
+          const uint32_t dst = t_base + r.i * C::T_STAGE;
+          if (rank == 0) mbar_expect_tx(fb, kpt * j.n_tok * 128);      // steps beyond K arrive as zeros
+          tma_load_3d_pair(dst, m1, 0, row1, kb, fb);
+          if (h2 > 0) tma_load_3d_pair(dst + h1 * 128, m2, 0, row2, kb, fb);
         }
       }
     }
@@ -355,47 +381,71 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       while (take_job(j, rj)) {
         const uint32_t h = seq & 1u;
         ok = mbar_wait(smem_u32(&dempty[h]), ((seq >> 1) & 1u) ^ 1u, abort_flag, g.status, 53);
-        if (ok && n_before + j.n_tok > WL_MAX_TOKENS) ok = mbar_wait(smem_u32(dpart), parts++ & 1u, abort_flag, g.status, 62);
+        if (ok && n_before + j.n_tok > C::ACC_COLS) ok = mbar_wait(smem_u32(dpart), parts++ & 1u, abort_flag, g.status, 62);
         if (!ok) break;
         ++seq;
         n_before = j.n_tok;
         tc_fence_after();
         const int n1 = min(j.n_tok, 256), n2 = j.n_tok - n1;
         const uint32_t id1 = id0 | (static_cast<uint32_t>(n1 >> 3) << 17), id2 = id0 | (static_cast<uint32_t>(n2 >> 3) << 17);
-        const uint32_t d = tmem_base + (h ? WL_MAX_TOKENS - j.n_tok : 0);
-        const int kpt = steps_per_stage(j.n_tok), step_bytes = j.n_tok * 64;
+        const uint32_t d = tmem_base + (h ? C::ACC_COLS - j.n_tok : 0);
+        const int kpt = steps_per_stage<FP8>(j.n_tok >> 1), step_bytes = j.n_tok * 64;
         int in_stage = 0;
-        for (int kb = 0; kb < g.k_steps; kb += 2) {
-          ok = mbar_wait(smem_u32(&aready[ra.i]), ra.ph, abort_flag, g.status, 55);
-          if (!ok) break;
-          tc_fence_after();
+        if (FP8) {
+          for (int kb = 0; kb < g.k_steps; kb += 2) {
+            ok = mbar_wait(smem_u32(&aready[ra.i]), ra.ph, abort_flag, g.status, 55);
+            if (!ok) break;
+            tc_fence_after();
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            if (in_stage == 0) {
-              ok = mbar_wait(smem_u32(&tfull[rt.i]), rt.ph, abort_flag, g.status, 54);
-              if (!ok) break;
-              tc_fence_after();
+            for (int half = 0; half < 2; ++half) {
+              if (in_stage == 0) {
+                ok = mbar_wait(smem_u32(&tfull[rt.i]), rt.ph, abort_flag, g.status, 54);
+                if (!ok) break;
+                tc_fence_after();
+              }
+              const uint32_t tb = t_base + rt.i * C::T_STAGE + in_stage * step_bytes;
+              const uint64_t db = make_smem_desc(tb);
+              const uint64_t db2 = make_smem_desc(tb + n1 * 64);
+              const uint32_t a = tmem_base + C::ACC_COLS + ra.i * WL_A_COLS + half * (WL_A_COLS / 2);
+#pragma unroll
+              for (int k = 0; k < WL_K / 16; ++k) {
+                // 16 bf16 = 32 bytes = 2 sixteen-byte units inside the swizzle row, or 8 columns of tensor memory
+                const uint32_t accumulate = (kb | half | k) != 0 ? 1u : 0u;
+                tc_mma_pair_ts(d, a + 8 * k, db + 2 * k, id1, accumulate);
+                if (n2 > 0) tc_mma_pair_ts(d + 256, a + 8 * k, db2 + 2 * k, id2, accumulate);
+              }
+              if (++in_stage == kpt || kb + half + 1 == g.k_steps) {
+                tc_commit_pair(smem_u32(&tempty[rt.i]));
+                rt.next(C::ST);
+                in_stage = 0;
+              }
             }
-            const uint32_t tb = t_base + rt.i * WL_T_STAGE + in_stage * step_bytes;
-            const uint64_t db = make_smem_desc(tb);
-            const uint64_t db2 = make_smem_desc(tb + n1 * 64);
-            const uint32_t a = tmem_base + WL_A_COL0 + ra.i * WL_A_COLS + half * (WL_A_COLS / 2);
+            if (!ok) break;
+            tc_commit_pair(smem_u32(&afree[ra.i]));
+            ra.next(WL_A_SLOTS);
+          }
+        } else {
+          for (int kb = 0; kb < g.k_steps; ++kb, ra.next(C::SW)) {
+            ok = (in_stage != 0 || mbar_wait(smem_u32(&tfull[rt.i]), rt.ph, abort_flag, g.status, 54)) &&
+                 mbar_wait(smem_u32(&wfull[ra.i]), ra.ph, abort_flag, g.status, 57);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t tb = t_base + rt.i * C::T_STAGE + in_stage * step_bytes;
+            const uint64_t da = make_smem_desc(w_base + ra.i * WL_W_STAGE);
+            const uint64_t db = make_smem_desc(tb), db2 = make_smem_desc(tb + n1 * 64);
 #pragma unroll
             for (int k = 0; k < WL_K / 16; ++k) {
-              // 16 bf16 = 32 bytes = 2 sixteen-byte units inside the swizzle row, or 8 columns of tensor memory
-              const uint32_t accumulate = (kb | half | k) != 0 ? 1u : 0u;
-              tc_mma_pair_ts(d, a + 8 * k, db + 2 * k, id1, accumulate);
-              if (n2 > 0) tc_mma_pair_ts(d + 256, a + 8 * k, db2 + 2 * k, id2, accumulate);
+              const uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
+              tc_mma_bf16_pair(d, da + 2 * k, db + 2 * k, id1, accumulate);
+              if (n2 > 0) tc_mma_bf16_pair(d + 256, da + 2 * k, db2 + 2 * k, id2, accumulate);
             }
-            if (++in_stage == kpt || kb + half + 1 == g.k_steps) {
+            tc_commit_pair(smem_u32(&wempty[ra.i]));
+            if (++in_stage == kpt || kb + 1 == g.k_steps) {
               tc_commit_pair(smem_u32(&tempty[rt.i]));
-              rt.next(WL_ST);
+              rt.next(C::ST);
               in_stage = 0;
             }
           }
-          if (!ok) break;
-          tc_commit_pair(smem_u32(&afree[ra.i]));
-          ra.next(WL_A_SLOTS);
         }
         if (!ok) break;
         tc_commit_pair(smem_u32(&dfull[h]));
@@ -403,22 +453,35 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     }
   } else if (warp == 3) {
     // ---------------- job list of this pair ----------------
-    // a look-up costs a binary search over the experts and two divisions, a thousand cycles and more where the issue
-    // slots are busy: done once here and ahead, not by every role between two jobs
+    // A look-up costs a binary search over the experts and two divisions, a thousand cycles and more where the issue
+    // slots are busy: done once here and ahead, not by every role between two jobs.  The leader draws the number once all
+    // roles have begun the job before, and passes it to the other CTA; the latter cannot be WL_MAIL jobs behind, since
+    // the leader's MMAs of a job need that CTA's weights and tokens.
     if (elect_one()) {
-      Ring rj;
-      Job j, next;
-      j.n_tok = 0;
-      if (pair < total_jobs) j = locate_job(pair, s_pad, s_cnt, s_jp, g);
-      for (int job = pair + n_pairs;; job += n_pairs, rj.next(WL_JOBS)) {
-        next.n_tok = 0;
-        if (job < total_jobs) next = locate_job(job, s_pad, s_cnt, s_jp, g);
-        j.next_tok = next.n_tok;
+      Ring rj, rm;
+      int job = pair;
+      for (;; rj.next(WL_JOBS)) {
         if (!mbar_wait(smem_u32(&jempty[rj.i]), rj.ph ^ 1u, abort_flag, g.status, 59)) break;
+        if (job < 0) {
+          if (g.next_job == nullptr) {
+            job = ~job + n_pairs;
+          } else if (rank == 0) {
+            job = n_pairs + atomicAdd(g.next_job, 1);
+            st_cluster(map_to_cta(smem_u32(&s_mail[rm.i]), 1), job);
+            mbar_arrive_cluster(map_to_cta(smem_u32(&mfull[rm.i]), 1));
+          } else {
+            if (!mbar_wait_cluster(smem_u32(&mfull[rm.i]), rm.ph, abort_flag, g.status, 63)) break;
+            job = *reinterpret_cast<volatile int*>(&s_mail[rm.i]);
+          }
+          rm.next(WL_MAIL);
+        }
+        Job j;
+        j.n_tok = 0;
+        if (job < total_jobs) j = locate_job(job, s_pad, s_cnt, s_jp, g);
         s_job[rj.i] = j;
         mbar_arrive(smem_u32(&jfull[rj.i]));
         if (j.n_tok == 0) break;
-        j = next;
+        job = ~job;
       }
     }
   } else if (warp >= 4 && warp < 4 + WL_EPI_WARPS) {
@@ -435,20 +498,23 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     auto send_piece = [&](int col, int row) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) tma_store_2d(&tmC, col, row, piece0 + piece * WL_PIECE);
+      if (lane == 0) tma_store_2d(&maps.c, col, row, piece0 + piece * WL_PIECE);
       piece ^= 1u;
     };
     uint32_t seq = 0u;
     Ring rj;
-    Job j;
-    while (take_job_warp(j, rj)) {
+    Job next;
+    bool more = take_job_warp(next, rj);
+    while (more) {
+      const Job j = next;
+      more = take_job_warp(next, rj);
       const uint32_t h = seq & 1u;
       if (!wait_warp(smem_u32(&dfull[h]), (seq >> 1) & 1u, abort_flag, g.status, 56)) break;
       ++seq;
       tc_fence_after();
       const int col0 = SWIGLU ? j.n_idx * 128 + static_cast<int>(rank) * 64 + quarter * 16
                               : j.n_idx * 256 + static_cast<int>(rank) * 128 + quarter * 32;
-      const uint32_t taddr = tmem_base + (h ? WL_MAX_TOKENS - j.n_tok : 0) + (static_cast<uint32_t>(quarter * 32) << 16);
+      const uint32_t taddr = tmem_base + (h ? C::ACC_COLS - j.n_tok : 0) + (static_cast<uint32_t>(quarter * 32) << 16);
       auto release = [&](uint64_t* bar) {
         tc_fence_before();
         __syncwarp();
@@ -456,7 +522,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
       };
       // chunks of 32 tokens, those first that lie in the next job's columns: once all warps have read them, the next
       // job's MMAs may start
-      const int chunks = j.n_tok >> 5, shared = j.next_tok == 0 ? 0 : max(0, j.n_tok + j.next_tok - WL_MAX_TOKENS) >> 5;
+      const int chunks = j.n_tok >> 5, shared = more ? max(0, j.n_tok + next.n_tok - C::ACC_COLS) >> 5 : 0;
       const int i0 = (warp - 4) >> 2;
       if (shared > 0 && i0 >= shared) release(dpart);
       if (i0 >= chunks) release(&dempty[h]);
@@ -502,13 +568,13 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     __syncwarp();
-  } else if (warp >= 4 + WL_EPI_WARPS) {
+  } else if (FP8 && warp >= 4 + WL_EPI_WARPS) {
     // ---------------- FP8 -> bf16 converters: shared -> registers -> tensor memory ----------------
     const int quarter = warp & 3;
     const uint32_t grp = (warp - 4 - WL_EPI_WARPS) >> 2;   // even / odd stages, counted over all jobs
     const int row = !SWIGLU ? quarter * 32 + lane : quarter * 16 + (lane & 15) + (lane & 16) * 4;
     const int block = SWIGLU ? lane >> 4 : static_cast<int>(rank);      // scale block row of this lane's weights
-    const uint32_t a_slot = tmem_base + WL_A_COL0 + grp * WL_A_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t a_slot = tmem_base + C::ACC_COLS + grp * WL_A_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
     const int stages = g.k_steps / 2;
     Ring rw, rj;
     rw.i = grp;
@@ -545,7 +611,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
         convert32(q[6], q[7], s, o2 + 16);
         tc_st32(a_slot + WL_A_COLS / 2, o2);
         rw.i += 2;
-        if (rw.i >= WL_SW) { rw.i -= WL_SW; rw.ph ^= 1u; }
+        if (rw.i >= C::SW) { rw.i -= C::SW; rw.ph ^= 1u; }
         tc_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -565,17 +631,48 @@ grouped_gemm_wl_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   }
 }
 
-template <int EPI>
-int launch_kernel(const Handle* h, const CUtensorMap& tw, const CUtensorMap& t64, const CUtensorMap& t16,
-                  const CUtensorMap& tc, const WlArgs& a, int grid, cudaStream_t st) {
+template <int EPI, bool FP8>
+int launch_kernel(const Handle* h, const WlMaps& maps, const WlArgs& a, int grid, cudaStream_t st) {
+  using C = WlCfg<FP8>;
   static bool done[64];
   if (!(h->device >= 0 && h->device < 64 && done[h->device])) {
-    MG_CUDA(cudaFuncSetAttribute(grouped_gemm_wl_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(WL_SMEM)));
+    MG_CUDA(cudaFuncSetAttribute(grouped_gemm_wl_kernel<EPI, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(C::SMEM)));
     if (h->device >= 0 && h->device < 64) done[h->device] = true;
   }
-  grouped_gemm_wl_kernel<EPI><<<grid, WL_THREADS, WL_SMEM, st>>>(tw, t64, t16, tc, a);
+  grouped_gemm_wl_kernel<EPI, FP8><<<grid, C::THREADS, C::SMEM, st>>>(maps, a);
   MG_CUDA(cudaGetLastError());
+  return MG_OK;
+}
+
+// From the handle's cache, by what the maps are made of: a forward's launches are few and the same ones again, and fourteen
+// driver calls a launch are 10 us that a decode step would see.
+template <bool FP8>
+int wl_maps(const Handle* h, const GemmProblem& p, bool swiglu, const WlMaps** out) {
+  WlMapCache& cache = h->wl_maps;
+  const WlMapCache::Key key{p.a, p.b, p.out, p.a_rows, static_cast<int64_t>(p.n_groups) * p.n_per_group, p.ldo, p.K, FP8, swiglu};
+  for (int i = 0; i < cache.used; ++i)
+    if (cache.e[i].key == key) { *out = &cache.e[i].maps; return MG_OK; }
+  WlMaps m;
+  const uint64_t K = static_cast<uint64_t>(p.K), blocks = static_cast<uint64_t>(key.w_rows) / 128;
+  const uint32_t both = swiglu ? 2 : 1;
+  int rc = FP8 ? encode_map(&m.w, p.b, true, 3, {K, 128, blocks}, {K, 128 * K}, {128, 128 / both, both})
+               : encode_map(&m.w, p.b, false, 4, {K, 16, blocks, 8}, {2 * K, 256 * K, 32 * K}, {WL_K, 16, both, 8 / both});
+  const uint64_t rows = static_cast<uint64_t>(p.a_rows), steps = K / WL_K;
+  for (int i = 0; i < 12 && rc == MG_OK; ++i) {
+    const uint32_t n = 16 * (i < 8 ? i + 1 : i - 7);
+    rc = encode_map(i < 8 ? &m.t[i] : &m.t2[i - 8], p.a, false, 3, {WL_K, rows, steps}, {2 * K, 2 * WL_K},
+                    {WL_K, n, i < 8 ? static_cast<uint32_t>(steps_per_stage<FP8>(n)) : 1u});
+  }
+  if (rc == MG_OK)
+    rc = encode_2d(h, &m.c, p.out, rows, static_cast<uint64_t>(p.ldo), swiglu ? 32 : 16, swiglu ? TM_OUT_16 : TM_OUT_PIECE);
+  if (rc != MG_OK) return rc;
+  WlMapCache::Entry& e = cache.e[cache.next];
+  e.key = key;
+  e.maps = m;
+  cache.next = (cache.next + 1) % WlMapCache::kEntries;
+  if (cache.used < WlMapCache::kEntries) ++cache.used;
+  *out = &e.maps;
   return MG_OK;
 }
 
@@ -583,23 +680,17 @@ int launch_kernel(const Handle* h, const CUtensorMap& tw, const CUtensorMap& t64
 
 int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
   const bool swiglu = p.epilogue == EPI_SWIGLU_BF16;
-  MG_REQUIRE(p.b_fp8 && p.scales != nullptr && p.pad_offsets != nullptr && (swiglu || p.epilogue == EPI_PLAIN_BF16),
-             MG_ERR_CONFIG, "weight-lane GEMM: grouped FP8 weights and bf16 outputs only");
-  MG_REQUIRE(p.K % 128 == 0 && p.n_per_group % 256 == 0 && p.ldo % 16 == 0, MG_ERR_SHAPE,
+  MG_REQUIRE(swiglu || p.epilogue == EPI_PLAIN_BF16, MG_ERR_CONFIG, "weight-lane GEMM: bf16 outputs only");
+  MG_REQUIRE(!p.b_fp8 || (p.scales != nullptr && p.pad_offsets != nullptr), MG_ERR_CONFIG,
+             "weight-lane GEMM: FP8 weights come with scales and in groups");
+  MG_REQUIRE(p.K % (p.b_fp8 ? 128 : WL_K) == 0 && p.n_per_group % 256 == 0 && p.ldo % 16 == 0, MG_ERR_SHAPE,
              "weight-lane GEMM: K=%d, N per expert=%d", p.K, p.n_per_group);
-  CUtensorMap tw, t64, t16, tc;
-  int rc = encode_2d(h, &tw, p.b, static_cast<uint64_t>(p.n_groups) * p.n_per_group, static_cast<uint64_t>(p.K), 64,
-                     TM_FP8_SW128);
-  if (rc != MG_OK) return rc;
-  rc = encode_2d(h, &t64, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 64, TM_BF16);
-  if (rc != MG_OK) return rc;
-  rc = encode_2d(h, &t16, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 16, TM_BF16);
-  if (rc != MG_OK) return rc;
-  rc = encode_2d(h, &tc, p.out, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.ldo),
-                 swiglu ? 32 : 16, swiglu ? TM_OUT_16 : TM_OUT_PIECE);
+  const WlMaps* maps = nullptr;
+  const int rc = p.b_fp8 ? wl_maps<true>(h, p, swiglu, &maps) : wl_maps<false>(h, p, swiglu, &maps);
   if (rc != MG_OK) return rc;
   WlArgs a;
   a.pad_offsets = p.pad_offsets;
+  a.dense_rows = static_cast<int>(p.dense_rows);
   a.counts = p.counts;
   a.n_groups = p.n_groups;
   a.n_tiles = p.n_per_group / 256;
@@ -607,14 +698,18 @@ int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
   a.k_steps = p.K / WL_K;
   a.scales = p.scales;
   a.scale_cols = p.K / 128;
+  a.next_job = p.next_job;
   a.status = h->d_status;
-  const int64_t tiles = (p.a_rows + WL_MAX_TOKENS - 1) / WL_MAX_TOKENS + p.n_groups;
+  const int max_tokens = p.b_fp8 ? WlCfg<true>::MAX_TOKENS : WlCfg<false>::MAX_TOKENS;
+  const int64_t tiles = (p.a_rows + max_tokens - 1) / max_tokens + p.n_groups;
   int64_t pairs = h->sm_count / 2;
   if (tiles * a.n_tiles < pairs) pairs = tiles * a.n_tiles;
   const int grid = static_cast<int>(2 * pairs);
-  return swiglu ? launch_kernel<EPI_SWIGLU_BF16>(h, tw, t64, t16, tc, a, grid, st)
-                : launch_kernel<EPI_PLAIN_BF16>(h, tw, t64, t16, tc, a, grid, st);
+  if (p.b_fp8)
+    return swiglu ? launch_kernel<EPI_SWIGLU_BF16, true>(h, *maps, a, grid, st)
+                  : launch_kernel<EPI_PLAIN_BF16, true>(h, *maps, a, grid, st);
+  return swiglu ? launch_kernel<EPI_SWIGLU_BF16, false>(h, *maps, a, grid, st)
+                : launch_kernel<EPI_PLAIN_BF16, false>(h, *maps, a, grid, st);
 }
 
 }  // namespace mg
-

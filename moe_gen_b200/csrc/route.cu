@@ -840,9 +840,11 @@ __global__ void __launch_bounds__(256) plan_scan_kernel(int32_t* __restrict__ bl
 
 // one block: offsets = exclusive scan of counts, pad_offsets = the same over counts rounded up to
 // whole 128-row tiles (n <= kMaxExperts = 512 = one value per thread)
-__global__ void __launch_bounds__(kMaxExperts) plan_offsets_kernel(const int32_t* __restrict__ counts, int n,
+__global__ void __launch_bounds__(kMaxExperts) plan_offsets_kernel(int32_t* __restrict__ job_counters,
+                                                                   const int32_t* __restrict__ counts, int n,
                                                                    int32_t* __restrict__ offsets,
                                                                    int32_t* __restrict__ pad_offsets) {
+  if (job_counters != nullptr && threadIdx.x < kJobCounters) job_counters[threadIdx.x] = 0;
   __shared__ int32_t warp_o[kMaxExperts / 32], warp_p[kMaxExperts / 32];
   const int e = threadIdx.x, lane = e & 31, w = e >> 5;
   const int32_t c = e < n ? counts[e] : 0;
@@ -916,7 +918,8 @@ constexpr size_t plan_small_smem(int T, int n) {
 __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restrict__ idx, int T, int k, int lo, int n,
                                                           int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                                                           int32_t* __restrict__ pad_offsets,
-                                                          int32_t* __restrict__ dst_row) {
+                                                          int32_t* __restrict__ dst_row,
+                                                          int32_t* __restrict__ job_counters) {
   extern __shared__ int32_t sm[];
   __shared__ int32_t warp_o[32], warp_p[32];
   const int W = (T + 31) >> 5;
@@ -925,6 +928,7 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
   int32_t* again = wbase + W * n;                  // [plan_small_runs(T)][n] repeated picks of e
   constexpr int RUN_W = kPlanTokens / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (job_counters != nullptr && tid < kJobCounters) job_counters[tid] = 0;
   for (int i = tid; i < W * n; i += blockDim.x) bm[i] = 0u;
   for (int i = tid; i < plan_small_runs(T) * n; i += blockDim.x) again[i] = 0;
   __syncthreads();
@@ -974,7 +978,8 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
 }
 
 static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo, int n, int32_t* counts,
-                             int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row, cudaStream_t st) {
+                             int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row, int32_t* job_counters,
+                             cudaStream_t st) {
   const size_t smem = plan_small_smem(T, n);
   static bool done[64];
   if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[h->device])) {
@@ -983,7 +988,8 @@ static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo,
     if (h->device >= 0 && h->device < 64) done[h->device] = true;
   }
   const int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;
-  plan_small_kernel<<<1, threads, smem, st>>>(idx, T, h->d.top_k, lo, n, counts, offsets, pad_offsets, dst_row);
+  plan_small_kernel<<<1, threads, smem, st>>>(idx, T, h->d.top_k, lo, n, counts, offsets, pad_offsets, dst_row,
+                                              job_counters);
   MG_CUDA(cudaGetLastError());
   return MG_OK;
 }
@@ -997,11 +1003,12 @@ size_t plan_ws_bytes(const Handle* h, int64_t T) {
 
 int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expert_lo, int n_exp,
                         int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,
-                        void* ws, cudaStream_t st, int* launches) {
+                        void* ws, cudaStream_t st, int* launches, int32_t* job_counters) {
   const int k = h->d.top_k;
   if (T > 0 && T <= kPlanSmallTokens) {
     if (launches) *launches += 1;
-    return launch_plan_small(h, idx, static_cast<int>(T), expert_lo, n_exp, counts, offsets, pad_offsets, dst_row, st);
+    return launch_plan_small(h, idx, static_cast<int>(T), expert_lo, n_exp, counts, offsets, pad_offsets, dst_row,
+                             job_counters, st);
   }
   int nblk = static_cast<int>((T + kPlanTokens - 1) / kPlanTokens);
   int32_t* bc = static_cast<int32_t*>(ws);
@@ -1012,7 +1019,7 @@ int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expe
   }
   plan_scan_kernel<<<(n_exp + 7) / 8, 256, 0, st>>>(bc, nblk, n_exp, counts);
   MG_CUDA(cudaGetLastError());
-  plan_offsets_kernel<<<1, kMaxExperts, 0, st>>>(counts, n_exp, offsets, pad_offsets);
+  plan_offsets_kernel<<<1, kMaxExperts, 0, st>>>(job_counters, counts, n_exp, offsets, pad_offsets);
   MG_CUDA(cudaGetLastError());
   if (nblk > 0) {
     size_t smem = static_cast<size_t>(2) * (kPlanTokens / 32) * n_exp * sizeof(int32_t);

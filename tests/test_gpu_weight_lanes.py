@@ -1,7 +1,8 @@
-"""GPU: the expert GEMMs with the weights on the accumulator's lanes (gemm_wl.cu, FP8 weights), at the edges of their
-jobs: no row, one row, multiples of 32 tokens and the rows around them, both accumulator halves, one job and several per
-expert and per SM pair.  Rows between the segments hold NaN, which must not reach a live row.  The bf16 cases and the
-shared expert run the kernel with the tokens on the lanes (gemm.cu) at the same edges."""
+"""GPU: the expert GEMMs with the weights on the accumulator's lanes (gemm_wl.cu), at the edges of their jobs: no row, one
+row, multiples of 32 tokens and the rows around them, accumulators that share columns with the next job's and that do not,
+one job and several per expert and per SM pair, jobs handed out by the counter and in fixed turns.  Rows between the
+segments hold NaN, which must not reach a live row.  The shared expert runs the kernel with the tokens on the lanes
+(gemm.cu) at the same edges."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -159,3 +160,70 @@ def test_several_jobs_per_sm_pair_equal_the_other_forms(built_lib, pattern, hidd
         assert bool(torch.isfinite(out[live].float()).all()) and bool((out[live] != 0).any())
         for other in (again, first, tokens_on_lanes):
             assert torch.equal(out[live].view(torch.int16), other[which][live].view(torch.int16)), which
+
+
+@pytest.mark.parametrize("hidden,inter,n_experts", [(2304, 2176, 24), (512, 384, 256)])
+@pytest.mark.parametrize("pattern", sorted(PATTERNS))
+def test_bf16_jobs_equal_the_form_with_tokens_on_the_lanes(built_lib, pattern, hidden, inter, n_experts):
+    """bf16 weights: the same job patterns; every live row has the same bits as from 256 x 256 tiles with the tokens on the
+    lanes.  K ends inside a stage that packs several steps for few tokens (34 and 6 steps)."""
+    from moe_gen_b200 import MoELayer
+    from moe_gen_b200 import lib as L
+    layer = MoELayer(hidden=hidden, inter=inter, n_experts=n_experts, top_k=2, device="cuda:0")
+    layer.set_router(torch.zeros(n_experts, hidden))
+    g = torch.Generator(device="cuda").manual_seed(4)
+    for e in range(n_experts):
+        layer.load_expert(e, *((torch.randn(*shape, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+                               for shape in ((inter, hidden), (inter, hidden), (hidden, inter))))
+    counts = (PATTERNS[pattern] * n_experts)[:n_experts]
+    cnt = torch.tensor(counts)
+    pad = torch.zeros(n_experts + 1, dtype=torch.int64)
+    pad[1:] = ((cnt + 127) // 128 * 128).cumsum(0)
+    x = torch.full((int(pad[-1]) + 128, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
+    live = torch.zeros(x.shape[0], dtype=torch.bool, device="cuda")
+    for e, c in enumerate(counts):
+        live[pad[e]:pad[e] + c] = True
+    x[live] = torch.randn(int(live.sum()), hidden, generator=g, device="cuda").to(torch.bfloat16)
+    pad_d, cnt_d = pad.int().cuda(), cnt.int().cuda()
+    got = layer.expert_ffn(x, pad_d, cnt_d)
+    again = layer.expert_ffn(x, pad_d, cnt_d)
+    layer.set_option(L.OPT_PAIR_GEMM, 1)
+    tokens_on_lanes = layer.expert_ffn(x, pad_d, cnt_d)
+    torch.cuda.synchronize()
+    assert layer.device_status() == (0, 0)
+    for which, out in enumerate(got):
+        assert bool(torch.isfinite(out[live].float()).all()) and bool((out[live] != 0).any())
+        for other in (again, tokens_on_lanes):
+            assert torch.equal(out[live].view(torch.int16), other[which][live].view(torch.int16)), which
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("T", [1, 40, 1024, 1025, 6000])
+def test_jobs_handed_out_by_the_counter_equal_fixed_turns(built_lib, T, fp8):
+    """The whole layer hands the jobs out by a counter that the plan kernels reset (one kernel up to 1024 tokens, another
+    above); the stages by themselves give every pair its turns.  Same bits, forward after forward and on graph replay."""
+    spec = O.LayerSpec(1024, 768, 32, 4, 256, 1, 1, O.GATE_SOFTMAX_GREEDY, False, 1.0,
+                       O.WEIGHT_FP8_BLOCK128 if fp8 else O.WEIGHT_BF16, O.COMBINE_FP32)
+    x, W = O.make_inputs(spec, T, 90 + T)
+    x[:, 0] = 3.0                                # a skewed load: the router's column 0 decides
+    layer = make_layer(spec, W)
+    x = x.cuda()
+    idx, w = layer.gate_route(x)[:2]
+    counts, offsets, pad, dst = layer.permute_plan(idx)
+    perm = layer.permute_rows(x, dst, layer.padded_rows(T * spec.top_k))
+    want = layer.combine(layer.expert_ffn(perm, pad, counts)[1], dst, idx, w, layer.shared_ffn(x))
+    for _ in range(3):
+        assert torch.equal(layer.forward(x).view(torch.int16), want.view(torch.int16))
+    out, s = torch.empty_like(x), torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        layer.forward(x, out=out)
+        s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            layer.forward(x, out=out)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    assert layer.device_status() == (0, 0)
