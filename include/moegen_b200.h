@@ -471,8 +471,9 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
  *                      MG_OPT_RING_BYTES and fetch their B tiles from it by TMA: no bf16 copy of the weights,
  *                      58 MB of scratch; measured 5 % slower than MG_FP8_PREDEQUANT at 65536 tokens of the
  *                      DeepSeek-V3 layer (the ring does not stay in L2), so only on request;
- *   MG_FP8_AUTO        (default) in-kernel while an expert sees fewer than 1024 rows on average
- *                      (DeepSeek-V3 shape: 27.3 against 31.8 ms there, level at 2048 rows), else pre-dequantise.
+ *   MG_FP8_AUTO        (default) in-kernel (DeepSeek-V3 shape, in-kernel against pre-dequantise: 22.5 and 29.2 ms
+ *                      at 1024 rows per expert, 43.9 and 50.9 ms at 2048); inner sizes beyond 16384, which the kernels
+ *                      that convert refuse, pre-dequantise from 1024 rows per expert on.
  * All give bit-identical results.  Set before asking mg_workspace_bytes / mg_dequant_ws_bytes. */
 #define MG_OPT_FP8_MODE    1
 #define MG_FP8_AUTO        0
@@ -503,8 +504,8 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
  * lanes, 256-row tiles.  Same results. */
 #define MG_OPT_FP8_M256    4
 /* MG_OPT_BATCH_TOKENS: a caller that feeds one batch through mg_moe_forward in chunks sets the
- * batch's total token count here (0 = off, the default); MG_FP8_AUTO then decides on the larger
- * of this and the call's T, because the de-quantised copy can serve every chunk
+ * batch's total token count here (0 = off, the default).  MG_FP8_AUTO looks at it for layers with K beyond 16384 only,
+ * which it de-quantises first from 1024 rows per expert on: the copy can serve every chunk
  * (MG_OPT_KEEP_DEQUANT).  Set before asking mg_workspace_bytes. */
 #define MG_OPT_BATCH_TOKENS 5
 /* MG_OPT_SHARED_EARLY: 1 = mg_moe_forward runs the shared expert's two GEMMs on a library

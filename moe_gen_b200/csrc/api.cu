@@ -64,19 +64,19 @@ static size_t dequant_ws(const Handle* h) {
 //   ring        the GEMM kernel's own CTAs convert every weight once per expert and share the bf16 copy
 //               through a ring of a few tens of MB (gemm.cu: grouped_gemm_ring_kernel): 58 MB of scratch
 //               instead of 2 bytes per weight.
-// AUTO: converting in the kernel re-does the work for every 384 rows of an expert; de-quantising first moves every
-// weight through HBM three more times.  V3 layer, ms, de-quantised first and converted in the kernel (weights on the
-// lanes, gemm_wl.cu): 512 rows per expert 20.2 and 14.1, 768 rows 26.1 and 19.7, 1024 rows 31.8 and 27.3, 1536 rows
-// 43.1 and 40.8, 2048 rows 54.8 and 53.5 (skewed 56.0 and 53.0), where runs differ by 3 %.  The line at 1024 rows was
-// drawn for 256-row tiles (30.1 there); above it the two are now level or the kernel ahead, so it costs time and not
-// results.  The ring was built to take the large batches without the HBM round trip of the bf16 copy, but L2 does not
-// hold it (measured at the benchmark size: 21.6 GB written to and 35.2 GB read from DRAM by the gate/up launch, i.e.
-// the ring goes through HBM like the separate pass's copy does), and it ends 5 % behind pre-dequantise there; it is
-// chosen only on request.
+// AUTO converts in the kernel at every size: it re-does the work for every 384 rows of an expert, where de-quantising
+// first moves every weight through HBM three more times.  V3 layer, ms, de-quantised first and converted in the kernel:
+// 512 rows per expert 18.9 and 12.0, 1024 rows 29.2 and 22.5, 1536 rows 40.0 and 33.3, 2048 rows 50.9 and 43.9 (skewed
+// 51.9 and 44.4), and 0.66 against 0.65 ms for every 1000 tokens more.  Without a scratch copy of the weights either
+// (22.5 GB there).  The ring was built to take the large batches without the HBM round trip of the bf16 copy, but L2
+// does not hold it (measured at the benchmark size: 21.6 GB written to and 35.2 GB read from DRAM by the gate/up launch,
+// i.e. the ring goes through HBM like the separate pass's copy does); it is chosen only on request.
 constexpr int64_t kRingMaxRows = 1ll << 24;          // rows the ring's counters are sized for
 static int fp8_mode_for(const Handle* h, int64_t rows) {
   if (h->d.weight_format != MG_WEIGHT_FP8_BLOCK128) return MG_FP8_IN_KERNEL;
   if (h->opt_fp8_mode != MG_FP8_AUTO) return h->opt_fp8_mode;
+  if (h->d.hidden <= 16384 && h->d.inter <= 16384) return MG_FP8_IN_KERNEL;
+  // K the in-kernel forms refuse: de-quantised first from 1024 rows per expert on
   if (h->opt_batch_tokens * h->d.top_k > rows) rows = h->opt_batch_tokens * h->d.top_k;
   return rows >= static_cast<int64_t>(1024) * h->d.n_experts ? MG_FP8_PREDEQUANT : MG_FP8_IN_KERNEL;
 }
