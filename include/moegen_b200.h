@@ -496,8 +496,10 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
 /* MG_OPT_ROUTE_FIXUP: 1 (default) = mg_moe_forward re-routes near-tie tokens from exactly recomputed logits
  * (see mg_gate_route_topk); 0 = it routes every token from the tensor-core product as it is. */
 #define MG_OPT_ROUTE_FIXUP 10
-/* MG_OPT_PAIR_GEMM: 1 = the bf16 expert GEMMs run on SM pairs (clusters of two CTAs,
- * tcgen05 cta_group::2, 256x256 tiles); 0 = one CTA per SM, 128x256 tiles. */
+/* MG_OPT_PAIR_GEMM: 1 = the expert and shared-expert GEMMs run on SM pairs in tiles of 256 tokens x 256 outputs with
+ * the tokens on the accumulator's lanes (clusters of two CTAs, tcgen05 cta_group::2); 0 (default) = the expert GEMMs
+ * run on SM pairs with the weights on the lanes, up to 384 tokens by 256 outputs, the shared expert's on one CTA per
+ * SM in 128x256 tiles.  Same results. */
 #define MG_OPT_PAIR_GEMM   2
 /* MG_OPT_FP8_M256: form of the convert-in-the-GEMM kernels: 1 (default) = weights on the accumulator's
  * lanes, up to 384 tokens per converted weight; 0 = tokens on the lanes, 128-row tiles; 2 = tokens on the

@@ -1578,7 +1578,7 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
     MG_REQUIRE(p.n_per_group % BN_MAX == 0, MG_ERR_SHAPE, "GEMM N per expert (%d) must be a multiple of %d",
                p.n_per_group, BN_MAX);
   }
-  // SM pairs (2-CTA tiles of 256 x 256) for the bf16 expert GEMMs when switched on
+  // SM pairs with the tokens on the lanes (2-CTA tiles of 256 x 256) when switched on
   const bool pair = h->opt_pair_gemm && !f32_out;
   if (p.ring != nullptr) return launch_ring_gemm(h, p, st);
   if (p.b_fp8) {
@@ -1591,6 +1591,14 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   // 30.1 / 27.3.  MG_OPT_FP8_M256 = 0 or 2 asks for the tiles with tokens on the lanes.
   const bool convert = p.b_fp8 && !dense && !f32_out && !pair;
   if (convert && h->opt_fp8_m256 == 1) return launch_gemm_wl(h, p, st);
+  // bf16 weights of experts as well: MMAs as wide as an expert's rows and not 128 or 256 of them, and fewer operand bytes
+  // per SM (40 KiB per 128 x 384 x 64 instead of 48 per 128 x 256 x 64).  Layer, ms, 128x256 tiles on one CTA per SM and
+  // weights on the lanes: Mixtral 61 tokens 0.545 and 0.491, 16384 9.32 and 8.91; V2-236B 512 tokens 1.36 and 1.25, 32768
+  // 11.58 and 11.58 (power cap); V2-Lite 8 tokens 0.170 and 0.160, 512 0.255 and 0.248, 2048 0.402 and 0.384.
+  // Shared experts (dense) stay with the tokens on the lanes: beside the routing kernels on another stream a pair's CTAs,
+  // with all of the SM's shared memory, keep those waiting (V2-Lite, 4096 tokens 0.63 and 0.68 ms), and later they are
+  // level.
+  if (!p.b_fp8 && !dense && !f32_out && !pair) return launch_gemm_wl(h, p, st);
   const bool m256 = convert && h->opt_fp8_m256 == 2;
   CUtensorMap ta, tb;
   int rc = encode_2d(h, &ta, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), m256 ? 2 * BM : BM, TM_BF16);

@@ -1,4 +1,6 @@
-// W8A16 grouped GEMM with the weights on the accumulator's lanes: D[weight row, token] = W_e[N, K] . X_e[rows, K]^T.
+// Grouped GEMM with the weights on the accumulator's lanes: D[weight row, token] = W_e[N, K] . X_e[rows, K]^T, with FP8
+// weights (W8A16) and with bf16 weights.  What follows is about the FP8 form; the bf16 form has no converters, takes both
+// operands from shared memory and uses all 512 columns of tensor memory for accumulators.
 //
 // A cluster of two CTAs (one SM pair, tcgen05 cta_group::2, M = 256) computes 256 weight rows against up to
 // 384 tokens of one expert.  Compared with tokens on the lanes (gemm.cu):
