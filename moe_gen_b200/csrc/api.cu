@@ -795,7 +795,10 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   int launches = 0;
   const long long guard_keep = h->guard_rows;
   h->guard_rows = padded_rows(h, T * d.top_k);     // what this call's dst_row entries may address
-  struct RestoreGuard { Handle* h; long long v; ~RestoreGuard() { h->guard_rows = v; } } restore_guard{h, guard_keep};
+  struct RestoreGuard { Handle* h; long long v; ~RestoreGuard() { h->guard_rows = v; h->chain = false; } } restore_guard{h, guard_keep};
+  // the launches behind the first one follow by programmatic dependence, unless events of the de-quantisation lie between
+  // them or their times are asked for one by one
+  const bool chain = deq == nullptr && !h->stage_timing;
   if (h->stage_timing) MG_CUDA(cudaEventRecord(h->stage_ev[h->stage_calls % kStageSlots][0], st));
   int rc;
   const bool deq_same = h->deq_scratch == deq && h->deq_packed == d_packed && h->deq_stream == st;
@@ -812,6 +815,7 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
     rc = mg_gate_logits(hh, d_x, d_gate_w, T, logits, stream);
     if (rc != MG_OK) return rc;
     launches += 1;
+    h->chain = chain;
   }
   mark(h, MG_STAGE_GATE_LOGITS, st);
   // The shared expert needs only x: its GEMMs (tensor-bound) run on a second stream beside the
@@ -827,7 +831,10 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
     }
     MG_CUDA(cudaEventRecord(h->ev_shared_in, st));
     MG_CUDA(cudaStreamWaitEvent(h->side2, h->ev_shared_in, 0));
+    const bool keep = h->chain;
+    h->chain = false;
     rc = shared_ffn(h, d_x, T, d_packed, hs, sh, h->side2, false);
+    h->chain = keep;
     if (rc != MG_OK) return rc;
     MG_CUDA(cudaEventRecord(h->ev_shared_out, h->side2));
     launches += 2;
@@ -842,6 +849,7 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
     launches += 1;
   }
   if (rc != MG_OK) return rc;
+  h->chain = chain;
   mark(h, MG_STAGE_ROUTE_TOPK, st);
   rc = launch_permute_plan(h, idx, T, 0, d.n_experts, counts, offsets, pad, dst, plan, st, &launches,
                            reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]));
@@ -856,6 +864,7 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   if (rc != MG_OK) return rc;
   if (shared_early) {
     MG_CUDA(cudaStreamWaitEvent(st, h->ev_shared_out, 0));
+    h->chain = false;
     mark(h, MG_STAGE_SHARED_GEMM1, st);
   } else if (d.inter_shared) {
     rc = shared_ffn(h, d_x, T, d_packed, hs, sh, st, true);

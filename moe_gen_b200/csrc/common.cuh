@@ -123,10 +123,36 @@ struct Handle {
   bool stage_timing;      // record an event after every stage of mg_moe_forward
   int stage_calls;        // forwards recorded since timing was enabled
   cudaEvent_t stage_ev[kStageSlots][MG_STAGE_COUNT + 1];   // ring of event sets, one per forward
+  bool chain = false;     // launches follow one another inside one forward (launch_chained)
   mutable TensorMapCache tmaps;
   mutable WlMapCache wl_maps;
 };
 constexpr uint32_t kMagic = 0x4d474232u;  // "MGB2"
+
+// Kernels of one forward follow one another by programmatic dependent launch: a kernel's blocks are placed as soon as
+// all blocks of the kernel before have begun and find room, set themselves up, and wait (chain_wait) until that kernel
+// has ended and its writes are visible.  Every kernel launched this way waits in every block, and lets the next one go
+// (chain_go) only after its own wait: what a kernel does before its wait may then rely on everything up to the kernel
+// before the last.  Only inside a forward and behind a kernel of it: what precedes the first one is the caller's.
+// Layer, ms, without and with: V2-Lite 8 tokens 0.160 and 0.142, 512 0.248 and 0.231, 2048 0.384 and 0.375, Mixtral 61
+// tokens 0.491 and 0.471, V2-236B 512 tokens 1.247 and 1.227; level from a few milliseconds on.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(const Handle* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = h->chain ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 

@@ -264,6 +264,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  chain_wait();
+  chain_go();
   if (g.pad_offsets != nullptr) {
     for (int i = threadIdx.x; i <= g.n_groups; i += blockDim.x) s_pad[i] = g.pad_offsets[i];
     for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) s_cnt[i] = g.counts[i];
@@ -1442,8 +1444,7 @@ static int launch_epi(const Handle* h, const CUtensorMap& ta, const CUtensorMap&
   static bool done[64];
   int rc = allow_smem(grouped_gemm_kernel<EPI, F8B, NARROW>, smem, h->device, done);
   if (rc != MG_OK) return rc;
-  grouped_gemm_kernel<EPI, F8B, NARROW><<<grid, Cfg<F8B, NARROW>::THREADS, smem, st>>>(ta, tb, tc, args);
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_chained(h, grouped_gemm_kernel<EPI, F8B, NARROW>, grid, Cfg<F8B, NARROW>::THREADS, smem, st, ta, tb, tc, args));
   return MG_OK;
 }
 

@@ -351,6 +351,10 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
     }
   } else if (warp == 1) {
     // ---------------- token TMA (both CTAs, own half of each MMA's N) ----------------
+    // The tokens are the last kernel's output; counts, offsets, job counters and weights are older, so the other roles
+    // begin without waiting.
+    chain_wait();
+    chain_go();
     if (elect_one()) {
       Ring r, rj;
       Job j;
@@ -642,8 +646,7 @@ int launch_kernel(const Handle* h, const WlMaps& maps, const WlArgs& a, int grid
                                  static_cast<int>(C::SMEM)));
     if (h->device >= 0 && h->device < 64) done[h->device] = true;
   }
-  grouped_gemm_wl_kernel<EPI, FP8><<<grid, C::THREADS, C::SMEM, st>>>(maps, a);
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_chained(h, grouped_gemm_wl_kernel<EPI, FP8>, grid, C::THREADS, C::SMEM, st, maps, a));
   return MG_OK;
 }
 

@@ -361,6 +361,8 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const float* __restrict
                                                          int64_t T, RouteParams rp,
                                                          int32_t* __restrict__ out_idx,
                                                          float* __restrict__ out_w, int32_t* __restrict__ fix) {
+  chain_wait();
+  chain_go();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
   route_token<P>(logits, bias, t, rp, out_idx, out_w, fix);
@@ -577,6 +579,8 @@ __global__ void __launch_bounds__(kRouteWarps * 32, (FEW ? 16 : 24) / kRouteWarp
 route_fused_kernel(float* logits, const float* __restrict__ bias, RouteParams rp, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ gate_w, int H, int32_t* __restrict__ out_idx,
                    float* __restrict__ out_w, int groups, int cluster) {
+  chain_wait();
+  chain_go();
   __shared__ uint16_t pairs[kRouteWarps * kMaxExperts];       // token of the block << 9 | expert
   __shared__ uint32_t play[kRouteWarps][kMaxExperts / 32];    // the same as bits
   __shared__ int n_pairs;
@@ -745,16 +749,25 @@ int launch_route_fused(const Handle* h, const void* x, const void* gate_w, float
   const int groups = static_cast<int>((T + kRouteWarps - 1) / kRouteWarps);
   int C = 8;
   while (C > 1 && static_cast<int64_t>(groups) * C > 2 * h->sm_count) C >>= 1;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(C);
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2]{};
+  unsigned n_attr = 0;
+  if (C > 1) {
+    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+    attr[n_attr].val.clusterDim.x = static_cast<unsigned>(C);
+    attr[n_attr].val.clusterDim.y = attr[n_attr].val.clusterDim.z = 1;
+    ++n_attr;
+  }
+  if (h->chain) {
+    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+    ++n_attr;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(groups) * C);
   cfg.blockDim = dim3(kRouteWarps * 32);
   cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = C > 1 ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = n_attr;
 #define MG_ROUTE_CASE(PP) \
   case PP: \
     if (C > 1) MG_CUDA(cudaLaunchKernelEx(&cfg, route_fused_kernel<PP, true>, logits, bias, rp, xb, wb, d.hidden, idx, w, groups, C)); \
@@ -779,7 +792,7 @@ int launch_route_topk(const Handle* h, const float* logits, const float* bias, i
   dim3 grid(static_cast<unsigned>((T + warps - 1) / warps)), block(warps * 32);
   const int P = (d.n_experts + 31) / 32;
 #define MG_ROUTE_CASE(PP)                                                             \
-  route_topk_kernel<PP><<<grid, block, 0, st>>>(logits, bias, T, rp, idx, w, nullptr)
+  MG_CUDA(launch_chained(h, route_topk_kernel<PP>, grid, block, 0, st, logits, bias, T, rp, idx, w, nullptr))
   if (P <= 1) MG_ROUTE_CASE(1);
   else if (P <= 2) MG_ROUTE_CASE(2);
   else if (P <= 4) MG_ROUTE_CASE(4);
@@ -800,6 +813,8 @@ constexpr int kPlanTokens = 256;  // tokens per block (one per thread)
 __global__ void __launch_bounds__(kPlanTokens) plan_count_kernel(const int32_t* __restrict__ idx,
                                                                  int64_t T, int k, int lo, int n,
                                                                  int32_t* __restrict__ block_counts) {
+  chain_wait();
+  chain_go();
   extern __shared__ int32_t hist[];
   for (int e = threadIdx.x; e < n; e += blockDim.x) hist[e] = 0;
   __syncthreads();
@@ -819,6 +834,8 @@ __global__ void __launch_bounds__(kPlanTokens) plan_count_kernel(const int32_t* 
 // per step, warp scan) and writes the expert's total
 __global__ void __launch_bounds__(256) plan_scan_kernel(int32_t* __restrict__ block_counts, int nblk, int n,
                                                         int32_t* __restrict__ counts) {
+  chain_wait();
+  chain_go();
   const int lane = threadIdx.x & 31;
   const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (e >= n) return;
@@ -844,6 +861,8 @@ __global__ void __launch_bounds__(kMaxExperts) plan_offsets_kernel(int32_t* __re
                                                                    const int32_t* __restrict__ counts, int n,
                                                                    int32_t* __restrict__ offsets,
                                                                    int32_t* __restrict__ pad_offsets) {
+  chain_wait();
+  chain_go();
   if (job_counters != nullptr && threadIdx.x < kJobCounters) job_counters[threadIdx.x] = 0;
   __shared__ int32_t warp_o[kMaxExperts / 32], warp_p[kMaxExperts / 32];
   const int e = threadIdx.x, lane = e & 31, w = e >> 5;
@@ -871,6 +890,8 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
                                                                  const int32_t* __restrict__ block_base,
                                                                  const int32_t* __restrict__ pad_offsets,
                                                                  int32_t* __restrict__ dst_row) {
+  chain_wait();
+  chain_go();
   extern __shared__ int32_t sm[];
   constexpr int W = kPlanTokens / 32;
   uint32_t* bm = reinterpret_cast<uint32_t*>(sm);  // [W][n] lanes of warp w that picked e
@@ -920,6 +941,8 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
                                                           int32_t* __restrict__ pad_offsets,
                                                           int32_t* __restrict__ dst_row,
                                                           int32_t* __restrict__ job_counters) {
+  chain_wait();
+  chain_go();
   extern __shared__ int32_t sm[];
   __shared__ int32_t warp_o[32], warp_p[32];
   const int W = (T + 31) >> 5;
@@ -988,9 +1011,8 @@ static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo,
     if (h->device >= 0 && h->device < 64) done[h->device] = true;
   }
   const int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;
-  plan_small_kernel<<<1, threads, smem, st>>>(idx, T, h->d.top_k, lo, n, counts, offsets, pad_offsets, dst_row,
-                                              job_counters);
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_chained(h, plan_small_kernel, 1, threads, smem, st, idx, T, h->d.top_k, lo, n, counts, offsets, pad_offsets,
+                         dst_row, job_counters));
   return MG_OK;
 }
 
@@ -1013,19 +1035,13 @@ int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expe
   int nblk = static_cast<int>((T + kPlanTokens - 1) / kPlanTokens);
   int32_t* bc = static_cast<int32_t*>(ws);
   if (nblk > 0) {
-    plan_count_kernel<<<nblk, kPlanTokens, n_exp * sizeof(int32_t), st>>>(idx, T, k, expert_lo,
-                                                                          n_exp, bc);
-    MG_CUDA(cudaGetLastError());
+    MG_CUDA(launch_chained(h, plan_count_kernel, nblk, kPlanTokens, n_exp * sizeof(int32_t), st, idx, T, k, expert_lo, n_exp, bc));
   }
-  plan_scan_kernel<<<(n_exp + 7) / 8, 256, 0, st>>>(bc, nblk, n_exp, counts);
-  MG_CUDA(cudaGetLastError());
-  plan_offsets_kernel<<<1, kMaxExperts, 0, st>>>(job_counters, counts, n_exp, offsets, pad_offsets);
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_chained(h, plan_scan_kernel, (n_exp + 7) / 8, 256, 0, st, bc, nblk, n_exp, counts));
+  MG_CUDA(launch_chained(h, plan_offsets_kernel, 1, kMaxExperts, 0, st, job_counters, counts, n_exp, offsets, pad_offsets));
   if (nblk > 0) {
     size_t smem = static_cast<size_t>(2) * (kPlanTokens / 32) * n_exp * sizeof(int32_t);
-    plan_place_kernel<<<nblk, kPlanTokens, smem, st>>>(idx, T, k, expert_lo, n_exp, bc,
-                                                       pad_offsets, dst_row);
-    MG_CUDA(cudaGetLastError());
+    MG_CUDA(launch_chained(h, plan_place_kernel, nblk, kPlanTokens, smem, st, idx, T, k, expert_lo, n_exp, bc, pad_offsets, dst_row));
   }
   if (launches) *launches += nblk > 0 ? 4 : 2;
   return MG_OK;
@@ -1096,6 +1112,8 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restri
                                                            int64_t T, int k, int vec_per_row,
                                                            PeerPtrs bufs, PeerPtrs dups, PeerPtrs backs, int my_rank,
                                                            Guard guard) {
+  chain_wait();
+  chain_go();
   const int lane = threadIdx.x & 31;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -1177,10 +1195,8 @@ int launch_permute_rows(const Handle* h, const void* x, const int32_t* dst_row, 
   dim3 grid(static_cast<unsigned>((T + warps - 1) / warps)), block(warps * 32);
   PeerPtrs bufs{};
   bufs.p[0] = perm_x;
-  permute_rows_kernel<false, false, false><<<grid, block, 0, st>>>(static_cast<const uint4*>(x), dst_row, T,
-                                                                   h->d.top_k, h->d.hidden / 8, bufs, bufs, bufs, 0,
-                                                                   Guard{h->d_status, h->guard_rows, 1});
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_chained(h, permute_rows_kernel<false, false, false>, grid, block, 0, st, static_cast<const uint4*>(x), dst_row,
+                         T, h->d.top_k, h->d.hidden / 8, bufs, bufs, bufs, 0, Guard{h->d_status, h->guard_rows, 1}));
   return MG_OK;
 }
 
@@ -1295,6 +1311,8 @@ __global__ void __launch_bounds__(256) combine_kernel(PeerPtrs bufs,
                                                       int64_t T, int k, int vec_per_row, int v_chunk,
                                                       uint4* y, int by_slot, const int32_t* __restrict__ delta,
                                                       Guard guard) {
+  chain_wait();
+  chain_go();
   const int lane = threadIdx.x & 31;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -1411,11 +1429,10 @@ static int launch_combine_impl(const Handle* h, const PeerPtrs& bufs, const int3
   dim3 grid(static_cast<unsigned>((T + warps - 1) / warps), static_cast<unsigned>((vpr + v_chunk - 1) / v_chunk));
   dim3 block(warps * 32);
 #define MG_COMBINE_CASE(M)                                                                       \
-  combine_kernel<M, PEER><<<grid, block, 0, st>>>(bufs, dst_row, idx, w,                          \
-                                                  static_cast<const uint4*>(shared),              \
-                                                  static_cast<const uint4*>(residual), T, k, vpr, \
-                                                  v_chunk, static_cast<uint4*>(y), by_slot, delta,              \
-                                                  Guard{h->d_status, h->guard_rows, PEER ? h->d.ep_size : 1})
+  MG_CUDA(launch_chained(h, combine_kernel<M, PEER>, grid, block, 0, st, bufs, dst_row, idx, w,   \
+                         static_cast<const uint4*>(shared), static_cast<const uint4*>(residual), T, k, vpr, v_chunk, \
+                         static_cast<uint4*>(y), by_slot, delta,                                 \
+                         Guard{h->d_status, h->guard_rows, PEER ? h->d.ep_size : 1}))
   switch (h->d.combine_mode) {
     case MG_COMBINE_FP32: MG_COMBINE_CASE(MG_COMBINE_FP32); break;
     case MG_COMBINE_BF16_PROD: MG_COMBINE_CASE(MG_COMBINE_BF16_PROD); break;
