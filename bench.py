@@ -793,20 +793,11 @@ def main():
         t_g1 = stage_ms["expert_gemm1"] * 1e-3
         tf = alg["gemm1_flops"] / world / t_g1 / 1e12 if t_g1 > 0 else 0.0
     peak_tf = peaks.get("bf16_tflops_sustained", FALLBACK_PEAKS["bf16_tflops_sustained"])
-    roofline = {"kernel": "grouped_gemm_kernel<SWIGLU> (routed gate/up projections + SiLU*mul)" if world == 1 else
-                "grouped_gemm_kernel, both expert GEMMs of rank 0 (expert phase of the expert-parallel forward)",
+    roofline = {"kernel": "grouped_gemm_wl_kernel<SWIGLU> (routed gate/up projections + SiLU*mul)" if world == 1 else
+                "grouped_gemm_wl_kernel, both expert GEMMs of rank 0 (expert phase of the expert-parallel forward)",
                 "bound": "tensor", "achieved": tf, "peak": peak_tf, "unit": "TFLOP/s", "frac": tf / peak_tf,
                 "peak_kind": f"of {peak_kind} sustained bf16 GEMM", "frac_of_burst": tf / peaks.get("bf16_tflops", 1590.0),
                 "traffic": None}
-    if world == 1 and name == "v3" and args.fp8_mode in (-1, 0, 1) and T == WORKLOADS["v3"][12]:
-        # not measured by this run: DRAM bytes of one launch of this kernel (one chunk of 32 experts) as ncu
-        # counted them on this workload (dram__bytes_read.sum + dram__bytes_write.sum, 1-pass counters, mean
-        # of the 8 launches of a forward), recorded once; the same launch moves 3.09 GB algorithmically
-        roofline["traffic"] = 4.88e9
-        roofline["traffic_recorded"] = {"captured": "2026-11-25, commit eea7afe", "algorithmic_bytes": 3.09e9,
-                                        "ratio": round(4.88 / 3.09, 2),
-                                        "note": "bytes per launch from a recorded ncu capture of this workload, not "
-                                                "from this run; the kernel's tile order is unchanged since"}
     hbm = peaks.get("hbm_gbs", FALLBACK_PEAKS["hbm_gbs"])
     Tl = T_total // world
     algl = algorithmic(name, Tl)
