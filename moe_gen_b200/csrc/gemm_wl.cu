@@ -84,8 +84,7 @@ struct WlCfg {
 static_assert(WlCfg<true>::SW % 2 == 0, "the two converter groups take alternate stages of the weight ring");
 
 struct WlArgs {
-  const int32_t* pad_offsets;   // nullptr: dense, one group
-  int dense_rows;
+  const int32_t* pad_offsets;
   const int32_t* counts;
   int n_groups;
   int n_tiles;                  // 256-row weight tiles per group
@@ -260,12 +259,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (g.pad_offsets != nullptr) {
-    for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) { s_pad[i] = g.pad_offsets[i]; s_cnt[i] = g.counts[i]; }
-  } else if (threadIdx.x == 0) {
-    s_pad[0] = 0;
-    s_cnt[0] = g.dense_rows;
-  }
+  for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) { s_pad[i] = g.pad_offsets[i]; s_cnt[i] = g.counts[i]; }
   __syncthreads();
   if (warp == 3) {
     // token tiles before each expert: lane sums of runs of 16 experts, warp scan, runs written out
@@ -685,9 +679,8 @@ int wl_maps(const Handle* h, const GemmProblem& p, bool swiglu, const WlMaps** o
 
 int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
   const bool swiglu = p.epilogue == EPI_SWIGLU_BF16;
-  MG_REQUIRE(swiglu || p.epilogue == EPI_PLAIN_BF16, MG_ERR_CONFIG, "weight-lane GEMM: bf16 outputs only");
-  MG_REQUIRE(!p.b_fp8 || (p.scales != nullptr && p.pad_offsets != nullptr), MG_ERR_CONFIG,
-             "weight-lane GEMM: FP8 weights come with scales and in groups");
+  MG_REQUIRE(p.pad_offsets != nullptr && (!p.b_fp8 || p.scales != nullptr) && (swiglu || p.epilogue == EPI_PLAIN_BF16),
+             MG_ERR_CONFIG, "weight-lane GEMM: grouped weights, FP8 with scales, and bf16 outputs only");
   MG_REQUIRE(p.K % (p.b_fp8 ? 128 : WL_K) == 0 && p.n_per_group % 256 == 0 && p.ldo % 16 == 0, MG_ERR_SHAPE,
              "weight-lane GEMM: K=%d, N per expert=%d", p.K, p.n_per_group);
   const WlMaps* maps = nullptr;
@@ -695,7 +688,6 @@ int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
   if (rc != MG_OK) return rc;
   WlArgs a;
   a.pad_offsets = p.pad_offsets;
-  a.dense_rows = static_cast<int>(p.dense_rows);
   a.counts = p.counts;
   a.n_groups = p.n_groups;
   a.n_tiles = p.n_per_group / 256;
