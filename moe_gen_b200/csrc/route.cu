@@ -101,9 +101,8 @@ __device__ __forceinline__ float kth_best_value(const float (&c0)[P], uint32_t g
 // experts in play (the blocks of route_fused_kernel recompute them; groups are runs of lanes there).
 template <int P, bool FIX_INLINE = false>
 __device__ __forceinline__ uint32_t route_token(const float* logits, const float* __restrict__ bias,
-                                                int64_t t, const RouteParams& rp, int32_t* __restrict__ out_idx,
-                                                float* __restrict__ out_w, int32_t* __restrict__ fix,
-                                                bool store = true) {
+                                                int64_t t, const RouteParams& rp, int32_t* out_idx, float* out_w,
+                                                int32_t* fix, bool store = true) {
   const bool detect = FIX_INLINE || fix != nullptr;
   uint32_t found = 0;
   const int lane = threadIdx.x & 31;
@@ -356,11 +355,9 @@ __device__ __forceinline__ uint32_t route_token(const float* logits, const float
 }
 
 template <int P>
-__global__ void __launch_bounds__(256) route_topk_kernel(const float* __restrict__ logits,
-                                                         const float* __restrict__ bias,
-                                                         int64_t T, RouteParams rp,
-                                                         int32_t* __restrict__ out_idx,
-                                                         float* __restrict__ out_w, int32_t* __restrict__ fix) {
+__global__ void __launch_bounds__(256) route_topk_kernel(const float* logits, const float* __restrict__ bias,
+                                                         int64_t T, RouteParams rp, int32_t* out_idx, float* out_w,
+                                                         int32_t* fix) {
   chain_wait();
   chain_go();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -577,8 +574,8 @@ constexpr int kRouteWarps = 8;
 template <int P, bool FEW>
 __global__ void __launch_bounds__(kRouteWarps * 32, (FEW ? 16 : 24) / kRouteWarps)
 route_fused_kernel(float* logits, const float* __restrict__ bias, RouteParams rp, const __nv_bfloat16* __restrict__ x,
-                   const __nv_bfloat16* __restrict__ gate_w, int H, int32_t* __restrict__ out_idx,
-                   float* __restrict__ out_w, int groups, int cluster) {
+                   const __nv_bfloat16* __restrict__ gate_w, int H, int32_t* out_idx, float* out_w, int groups,
+                   int cluster) {
   chain_wait();
   chain_go();
   __shared__ uint16_t pairs[kRouteWarps * kMaxExperts];       // token of the block << 9 | expert
@@ -810,9 +807,22 @@ int launch_route_topk(const Handle* h, const float* logits, const float* bias, i
 // ---------------------------------------------------------------------------------------
 constexpr int kPlanTokens = 256;  // tokens per block (one per thread)
 
-__global__ void __launch_bounds__(kPlanTokens) plan_count_kernel(const int32_t* __restrict__ idx,
-                                                                 int64_t T, int k, int lo, int n,
-                                                                 int32_t* __restrict__ block_counts) {
+// f(j, pick j) for a token's picks.  They are read eight at a time before the first is used: behind the stores and
+// atomics of f, which may alias them as far as the compiler knows, every read would wait for the one before.
+template <typename F>
+__device__ __forceinline__ void for_each_pick(const int32_t* picks, int k, F f) {
+  for (int j0 = 0; j0 < k; j0 += 8) {
+    int32_t e[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) e[u] = j0 + u < k ? picks[j0 + u] : 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (j0 + u < k) f(j0 + u, e[u]);
+  }
+}
+
+__global__ void __launch_bounds__(kPlanTokens) plan_count_kernel(const int32_t* idx, int64_t T, int k, int lo, int n,
+                                                                 int32_t* block_counts) {
   chain_wait();
   chain_go();
   extern __shared__ int32_t hist[];
@@ -820,10 +830,10 @@ __global__ void __launch_bounds__(kPlanTokens) plan_count_kernel(const int32_t* 
   __syncthreads();
   int64_t t = static_cast<int64_t>(blockIdx.x) * kPlanTokens + threadIdx.x;
   if (t < T) {
-    for (int j = 0; j < k; ++j) {
-      int e = idx[t * k + j] - lo;
+    for_each_pick(idx + t * k, k, [&](int, int32_t pick) {
+      const int e = pick - lo;
       if (e >= 0 && e < n) atomicAdd(&hist[e], 1);
-    }
+    });
   }
   __syncthreads();
   for (int e = threadIdx.x; e < n; e += blockDim.x)
@@ -832,8 +842,7 @@ __global__ void __launch_bounds__(kPlanTokens) plan_count_kernel(const int32_t* 
 
 // one warp per expert: turns block_counts[:, e] into an exclusive prefix over the blocks (32 blocks
 // per step, warp scan) and writes the expert's total
-__global__ void __launch_bounds__(256) plan_scan_kernel(int32_t* __restrict__ block_counts, int nblk, int n,
-                                                        int32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(256) plan_scan_kernel(int32_t* block_counts, int nblk, int n, int32_t* counts) {
   chain_wait();
   chain_go();
   const int lane = threadIdx.x & 31;
@@ -857,10 +866,8 @@ __global__ void __launch_bounds__(256) plan_scan_kernel(int32_t* __restrict__ bl
 
 // one block: offsets = exclusive scan of counts, pad_offsets = the same over counts rounded up to
 // whole 128-row tiles (n <= kMaxExperts = 512 = one value per thread)
-__global__ void __launch_bounds__(kMaxExperts) plan_offsets_kernel(int32_t* __restrict__ job_counters,
-                                                                   const int32_t* __restrict__ counts, int n,
-                                                                   int32_t* __restrict__ offsets,
-                                                                   int32_t* __restrict__ pad_offsets) {
+__global__ void __launch_bounds__(kMaxExperts) plan_offsets_kernel(int32_t* job_counters, const int32_t* counts,
+                                                                   int n, int32_t* offsets, int32_t* pad_offsets) {
   chain_wait();
   chain_go();
   if (job_counters != nullptr && threadIdx.x < kJobCounters) job_counters[threadIdx.x] = 0;
@@ -885,11 +892,9 @@ __global__ void __launch_bounds__(kMaxExperts) plan_offsets_kernel(int32_t* __re
   }
 }
 
-__global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* __restrict__ idx,
-                                                                 int64_t T, int k, int lo, int n,
-                                                                 const int32_t* __restrict__ block_base,
-                                                                 const int32_t* __restrict__ pad_offsets,
-                                                                 int32_t* __restrict__ dst_row) {
+__global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* idx, int64_t T, int k, int lo, int n,
+                                                                 const int32_t* block_base, const int32_t* pad_offsets,
+                                                                 int32_t* dst_row) {
   chain_wait();
   chain_go();
   extern __shared__ int32_t sm[];
@@ -901,10 +906,10 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int64_t t = static_cast<int64_t>(blockIdx.x) * kPlanTokens + threadIdx.x;
   if (t < T) {
-    for (int j = 0; j < k; ++j) {
-      int e = idx[t * k + j] - lo;
+    for_each_pick(idx + t * k, k, [&](int, int32_t pick) {
+      const int e = pick - lo;
       if (e >= 0 && e < n) atomicOr(&bm[warp * n + e], 1u << lane);
-    }
+    });
   }
   __syncthreads();
   for (int e = threadIdx.x; e < n; e += blockDim.x) {
@@ -917,12 +922,10 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
   __syncthreads();
   if (t < T) {
     const uint32_t lt = (1u << lane) - 1u;
-    for (int j = 0; j < k; ++j) {
-      int e = idx[t * k + j] - lo;
-      int32_t dst = -1;
-      if (e >= 0 && e < n) dst = wbase[warp * n + e] + __popc(bm[warp * n + e] & lt);
-      dst_row[t * k + j] = dst;
-    }
+    for_each_pick(idx + t * k, k, [&](int j, int32_t pick) {
+      const int e = pick - lo;
+      dst_row[t * k + j] = e >= 0 && e < n ? wbase[warp * n + e] + __popc(bm[warp * n + e] & lt) : -1;
+    });
   }
 }
 
@@ -936,11 +939,9 @@ __host__ __device__ constexpr int plan_small_runs(int T) { return (T + kPlanToke
 constexpr size_t plan_small_smem(int T, int n) {
   return static_cast<size_t>(2 * ((T + 31) / 32) + plan_small_runs(T)) * n * sizeof(int32_t);
 }
-__global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restrict__ idx, int T, int k, int lo, int n,
-                                                          int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
-                                                          int32_t* __restrict__ pad_offsets,
-                                                          int32_t* __restrict__ dst_row,
-                                                          int32_t* __restrict__ job_counters) {
+__global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, int T, int k, int lo, int n,
+                                                          int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
+                                                          int32_t* dst_row, int32_t* job_counters) {
   chain_wait();
   chain_go();
   extern __shared__ int32_t sm[];
@@ -957,10 +958,10 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
   __syncthreads();
   if (tid < T) {
     const uint32_t bit = 1u << lane;
-    for (int j = 0; j < k; ++j) {
-      const int e = idx[tid * k + j] - lo;
+    for_each_pick(idx + tid * k, k, [&](int, int32_t pick) {
+      const int e = pick - lo;
       if (e >= 0 && e < n && (atomicOr(&bm[warp * n + e], bit) & bit)) atomicAdd(&again[warp / RUN_W * n + e], 1);
-    }
+    });
   }
   __syncthreads();
   int32_t c = 0;
@@ -993,10 +994,10 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* __restr
   __syncthreads();
   if (tid < T) {
     const uint32_t lt = (1u << lane) - 1u;
-    for (int j = 0; j < k; ++j) {
-      const int e = idx[tid * k + j] - lo;
+    for_each_pick(idx + tid * k, k, [&](int j, int32_t pick) {
+      const int e = pick - lo;
       dst_row[tid * k + j] = e >= 0 && e < n ? wbase[warp * n + e] + __popc(bm[warp * n + e] & lt) : -1;
-    }
+    });
   }
 }
 
@@ -1107,8 +1108,7 @@ int launch_permute_plan_static(const Handle* h, const int32_t* idx, int64_t T, i
 // BACK: every pick also leaves, in the destination rank's return table at the pick's row, where the
 // expert's output for that row has to go: source rank << kPeerShift | (token * k + slot).
 template <bool PEER, bool DEDUP, bool BACK>
-__global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restrict__ x,
-                                                           const int32_t* __restrict__ dst_row,
+__global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restrict__ x, const int32_t* dst_row,
                                                            int64_t T, int k, int vec_per_row,
                                                            PeerPtrs bufs, PeerPtrs dups, PeerPtrs backs, int my_rank,
                                                            Guard guard) {
@@ -1302,15 +1302,10 @@ __device__ __forceinline__ float round_bf16(float f) {
 // (token * k + slot) of this rank's return buffer (bufs.p[owner] all point at it), a pick of this rank's own
 // experts is read in place from its out_rows (bufs.p[rank]); 0 = rows as dst_row says.
 template <int MODE, bool PEER>
-__global__ void __launch_bounds__(256) combine_kernel(PeerPtrs bufs,
-                                                      const int32_t* __restrict__ dst_row,
-                                                      const int32_t* __restrict__ topk_idx,
-                                                      const float* __restrict__ topk_w,
-                                                      const uint4* __restrict__ shared,
-                                                      const uint4* residual,
+__global__ void __launch_bounds__(256) combine_kernel(PeerPtrs bufs, const int32_t* dst_row, const int32_t* topk_idx,
+                                                      const float* topk_w, const uint4* shared, const uint4* residual,
                                                       int64_t T, int k, int vec_per_row, int v_chunk,
-                                                      uint4* y, int by_slot, const int32_t* __restrict__ delta,
-                                                      Guard guard) {
+                                                      uint4* y, int by_slot, const int32_t* delta, Guard guard) {
   chain_wait();
   chain_go();
   const int lane = threadIdx.x & 31;
@@ -1376,8 +1371,8 @@ __global__ void __launch_bounds__(256) combine_kernel(PeerPtrs bufs,
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           val[u] = make_uint4(0u, 0u, 0u, 0u);
-          // peer rows are written by another GPU during this forward: plain (coherent) loads
-          if (base[s0 + u] != nullptr) val[u] = PEER ? base[s0 + u][v] : __ldg(base[s0 + u] + v);
+          // rows of the kernel before this one, or of another GPU during this forward: plain (coherent) loads
+          if (base[s0 + u] != nullptr) val[u] = base[s0 + u][v];
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -1397,7 +1392,7 @@ __global__ void __launch_bounds__(256) combine_kernel(PeerPtrs bufs,
     }
     if (shared != nullptr) {
       float f[8];
-      unpack8(__ldg(shared + t * vec_per_row + v), f);
+      unpack8(shared[t * vec_per_row + v], f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(round_bf16(acc[i]), f[i]);
     }

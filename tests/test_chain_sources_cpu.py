@@ -1,0 +1,66 @@
+"""Kernels launched by programmatic dependence (launch_chained) begin while the kernel before them still writes.  What they
+may then do is a matter of their source, which this looks at; a wrong order of a load would show as a wrong value at best
+once in a while."""
+import os
+import re
+
+import pytest
+
+from moe_gen_b200 import build as b
+
+# operands that are complete before the first kernel of a forward begins: the caller's, and the packed weights
+OLDER = {"x", "gate_w", "bias", "w", "weight", "b8"}
+# __ldg of: rows of x in the scatter, router operands, weight scales
+LDG_OLDER = ("src + v", "xr + v", "wr + v", "reinterpret_cast<const uint2*>(xr[j])", "reinterpret_cast<const uint2*>(w +",
+             "srow +", "row + i * 32", "weight + v")
+
+
+def _strip(text):
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _kernels():
+    """name -> (parameters, body) of every __global__ function"""
+    out = {}
+    for f in b.SOURCES:
+        text = _strip(open(os.path.join(b.CSRC, f)).read())
+        for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\s*\(", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"(": 1, ")": -1}.get(text[i], 0)
+                i += 1
+            params = text[m.end():i - 1]
+            j = text.index("{", i)
+            depth, i = 1, j + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+            out[m.group(1)] = (params, text[j + 1:i - 1])
+    return out
+
+
+KERNELS = _kernels()
+CHAINED = sorted(n for n, (_, body) in KERNELS.items() if "chain_wait()" in body)
+
+
+def test_every_kernel_launched_by_dependence_waits():
+    launched = set()
+    for f in b.SOURCES:
+        text = _strip(open(os.path.join(b.CSRC, f)).read())
+        launched |= set(re.findall(r"launch_chained\(\s*h,\s*(\w+)", text))
+        if "cudaLaunchAttributeProgrammaticStreamSerialization" in text:
+            launched |= set(re.findall(r"cudaLaunchKernelEx\(&cfg,\s*(\w+_kernel)", text))
+    assert len(launched) >= 8 and "combine_kernel" in launched
+    assert launched == set(CHAINED)
+
+
+@pytest.mark.parametrize("name", CHAINED)
+def test_no_read_only_path_for_what_a_predecessor_writes(name):
+    """__ldg, and __restrict__ on a pointer that is only read, promise memory that nothing writes while the kernel lives:
+    the load may come from the non-coherent path and may be moved ahead of the wait."""
+    params, body = KERNELS[name]
+    for p in params.split(","):
+        if "__restrict__" in p:
+            assert p.split()[-1] in OLDER, f"{name}: {p.strip()}"
+    for m in re.finditer(r"__ldg\(", body):
+        assert body[m.end():].startswith(LDG_OLDER), f"{name}: __ldg({body[m.end():m.end() + 40]}"
