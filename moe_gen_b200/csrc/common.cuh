@@ -131,12 +131,14 @@ constexpr uint32_t kMagic = 0x4d474232u;  // "MGB2"
 
 // Kernels of one forward follow one another by programmatic dependent launch: a kernel's blocks are placed as soon as
 // all blocks of the kernel before have begun and find room, set themselves up, and wait (chain_wait) until that kernel
-// has ended and its writes are visible.  Every kernel launched this way waits in every block, and lets the next one go
-// (chain_go) only after its own wait: what a kernel does before its wait may then rely on everything up to the kernel
-// before the last.  What an earlier kernel of the same forward writes is read by ordinary loads, through pointers without
-// __restrict__: the life of a chained kernel overlaps its predecessors', so it is not read-only memory, which __ldg and
-// const __restrict__ promise (the load may then be non-coherent, or be moved ahead of the wait).  The caller's operands and
-// the weights are older than the first kernel and may be read so.  Only inside a forward and behind a kernel of it: what precedes the first one is the caller's.
+// has ended and its writes are visible.  Every thread of a kernel launched this way waits before it reads memory: the
+// begin of a kernel makes nothing visible, older kernels' writes neither (the weight-lane GEMM peeks at the counts for
+// a guess, and reads them again).  Every block lets the next kernel go (chain_go).
+// What an earlier kernel of the same forward writes is read by ordinary loads, through pointers without __restrict__: the
+// life of a chained kernel overlaps its predecessors', so it is not read-only memory, which __ldg and const __restrict__
+// promise (the load may then be non-coherent, or be moved ahead of the wait).  The caller's operands and the weights are
+// older than the first kernel and may be read so.  Only inside a forward and behind a kernel of it: what precedes the first
+// one is the caller's.
 // Layer, ms, without and with: V2-Lite 8 tokens 0.160 and 0.142, 512 0.248 and 0.231, 2048 0.384 and 0.375, Mixtral 61
 // tokens 0.491 and 0.471, V2-236B 512 tokens 1.247 and 1.227; level from a few milliseconds on.
 template <typename... P, typename... A>

@@ -64,3 +64,21 @@ def test_no_read_only_path_for_what_a_predecessor_writes(name):
             assert p.split()[-1] in OLDER, f"{name}: {p.strip()}"
     for m in re.finditer(r"__ldg\(", body):
         assert body[m.end():].startswith(LDG_OLDER), f"{name}: __ldg({body[m.end():m.end() + 40]}"
+
+
+@pytest.mark.parametrize("name", CHAINED)
+def test_every_thread_waits_before_it_reads_memory(name):
+    """What a predecessor has written is visible to a thread behind its own wait; the begin of a kernel promises nothing,
+    about older kernels either.  A value may be peeked at before, as a guess, if it is read again behind the wait."""
+    params, body = KERNELS[name]
+    at = body.index("chain_wait()")
+    before, behind = body[:at], body[at:]
+    for m in re.findall(r"\bpeek\(([\w.]+)", before):
+        assert m in behind, f"{name}: {m} is only guessed"
+    assert "peek(" not in behind
+    before = re.sub(r"\bpeek\([\w.]+", "peek(", before)
+    assert before.count("{") == before.count("}"), f"{name}: only some threads reach the wait"
+    pointers = [p.split()[-1].lstrip("*") for p in params.split(",") if "*" in p]
+    used = [p for p in pointers if re.search(rf"\b{p}\b", before)]
+    used += re.findall(r"\bg\.(?:pad_offsets|counts|next_job|scales|out)\b", before)
+    assert not used, f"{name}: {used} before the wait"
