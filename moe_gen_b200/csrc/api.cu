@@ -552,7 +552,8 @@ static int join_return(Handle* h, cudaStream_t st) {
 
 static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const int32_t* counts, int64_t rows_padded,
                       const void* packed, void* h_buf, void* out_rows, void* deq, cudaStream_t st, int* launches,
-                      bool timed = false, const ReturnHook* hook = nullptr, int32_t* job_counters = nullptr) {
+                      bool timed = false, const ReturnHook* hook = nullptr, int32_t* job_counters = nullptr,
+                      bool chain_down = true) {
   if (hook != nullptr) {
     int rc0 = ensure_return_stream(h);
     if (rc0 != MG_OK) return rc0;
@@ -588,6 +589,7 @@ static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const i
     int rc = launch_grouped_gemm(h, p, st);
     if (rc != MG_OK) return rc;
     if (timed) mark(h, MG_STAGE_EXPERT_GEMM1, st);
+    if (!chain_down) h->chain = false;
     p.a = h_buf; p.b = base + L.w2; p.n_per_group = d.hidden; p.K = d.inter; p.out = out_rows; p.ldo = d.hidden;
     p.epilogue = EPI_PLAIN_BF16;
     p.next_job = job_counters != nullptr ? job_counters + 1 : nullptr;
@@ -757,6 +759,13 @@ int mg_workspace_ptr(mg_handle hh, void* d_ws, int64_t max_tokens, int64_t max_r
   return MG_OK;
 }
 
+// Up to here the down product is not chained while the shared expert runs on its own stream: chained, its blocks would stand
+// in line for every SM that the gate/up product leaves, ahead of the shared expert's second product, which then comes last
+// and alone.  Layer, us, chained and not: V2-236B 1 token 130 and 117 (without any chaining 126), V2-Lite 1 token 76 and 70, 8
+// 141 and 135, 64 215 and 210; above, where the experts are long against it, V2-Lite 256 tokens 217 and 219, V2-236B 512
+// 1191 and 1200.
+constexpr int64_t kUnchainedDownTokens = 64;
+
 // d_residual: nullptr, or [T,H] bf16 added to the block's bf16 output in the combine (may be d_y)
 // d_logits_in: nullptr, or caller-computed fp32 router logits [T,E] used in place of the router GEMM
 static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void* d_gate_w, const float* d_bias,
@@ -860,7 +869,7 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   mark(h, MG_STAGE_PERMUTE_ROWS, st);
   launches += 1;
   rc = expert_ffn(h, perm, pad, counts, padded_rows(h, T * d.top_k), d_packed, hbuf, orow, deq, st, &launches, true,
-                  nullptr, reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]));
+                  nullptr, reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]), !(shared_early && T <= kUnchainedDownTokens));
   if (rc != MG_OK) return rc;
   if (shared_early) {
     MG_CUDA(cudaStreamWaitEvent(st, h->ev_shared_out, 0));

@@ -139,8 +139,8 @@ constexpr uint32_t kMagic = 0x4d474232u;  // "MGB2"
 // promise (the load may then be non-coherent, or be moved ahead of the wait).  The caller's operands and the weights are
 // older than the first kernel and may be read so.  Only inside a forward and behind a kernel of it: what precedes the first
 // one is the caller's.
-// Layer, ms, without and with: V2-Lite 8 tokens 0.160 and 0.142, 512 0.248 and 0.231, 2048 0.384 and 0.375, Mixtral 61
-// tokens 0.491 and 0.471, V2-236B 512 tokens 1.247 and 1.227; level from a few milliseconds on.
+// Layer, us, without and with: V2-Lite 8 tokens 147 and 135, 512 248 and 232, 2048 364 and 360, Mixtral 61 tokens 487 and
+// 466, V2-236B 512 tokens 1217 and 1200; level from a few milliseconds on.
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(const Handle* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                   A&&... args) {
