@@ -550,6 +550,11 @@ static int join_return(Handle* h, cudaStream_t st) {
   return MG_OK;
 }
 
+static int zero_job_counters(Handle* h, cudaStream_t st) {
+  if (h->job_counters != nullptr) MG_CUDA(cudaMemsetAsync(h->job_counters, 0, kJobCounters * sizeof(int32_t), st));
+  return MG_OK;
+}
+
 static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const int32_t* counts, int64_t rows_padded,
                       const void* packed, void* h_buf, void* out_rows, void* deq, cudaStream_t st, int* launches,
                       bool timed = false, const ReturnHook* hook = nullptr, int32_t* job_counters = nullptr,
@@ -605,6 +610,7 @@ static int expert_ffn(Handle* h, const void* perm_x, const int32_t* pad, const i
         p.n_groups = n; p.pad_offsets = pad + lo; p.counts = counts + lo;
         p.b = base + L.w2 + lo * w2_expert;
         p.scales = fp8 ? reinterpret_cast<const float*>(base + L.s2) + lo * s2_expert : nullptr;
+        p.next_job = job_counters != nullptr ? job_counters + kDequantChunks + c : nullptr;
         rc = launch_grouped_gemm(h, p, st);
         if (rc != MG_OK) return rc;
         rc = push_part(h, hook, out_rows, pad, lo, n, c, st);
@@ -684,7 +690,10 @@ namespace mg {
 int expert_ffn_return(Handle* h, const void* perm_x, const int32_t* pad, const int32_t* counts, int64_t rows_padded,
                       const void* packed, void* h_buf, void* out_rows, void* deq, const ReturnHook& hook,
                       cudaStream_t st) {
-  return expert_ffn(h, perm_x, pad, counts, rows_padded, packed, h_buf, out_rows, deq, st, nullptr, false, &hook);
+  int rc = zero_job_counters(h, st);
+  if (rc != MG_OK) return rc;
+  return expert_ffn(h, perm_x, pad, counts, rows_padded, packed, h_buf, out_rows, deq, st, nullptr, false, &hook,
+                    h->job_counters);
 }
 }  // namespace mg
 extern "C" {
@@ -709,8 +718,17 @@ int mg_expert_ffn(mg_handle hh, const void* d_perm_x, const int32_t* d_pad, cons
              "mg_expert_ffn: null pointer");
   MG_REQUIRE(n_rows_padded >= 0 && n_rows_padded % kTileM == 0, MG_ERR_SHAPE,
              "n_rows_padded=%lld must be a multiple of %d", static_cast<long long>(n_rows_padded), kTileM);
+  int rc = zero_job_counters(h, static_cast<cudaStream_t>(stream));
+  if (rc != MG_OK) return rc;
   return expert_ffn(h, d_perm_x, d_pad, d_counts, n_rows_padded, d_packed, d_h_buf, d_out_rows, d_deq,
-                    static_cast<cudaStream_t>(stream), nullptr);
+                    static_cast<cudaStream_t>(stream), nullptr, false, nullptr, h->job_counters);
+}
+
+int mg_set_job_counters(mg_handle hh, int32_t* d_counters) {
+  Handle* h = check(hh);
+  if (!h) return MG_ERR_STATE;
+  h->job_counters = d_counters;
+  return MG_OK;
 }
 
 static int shared_ffn(Handle* h, const void* x, int64_t T, const void* packed, void* hs, void* out, cudaStream_t st,

@@ -18,7 +18,8 @@ constexpr int kPeerShift = 24;       // expert-parallel destinations: rank << 24
 constexpr int kPeerRowMask = (1 << kPeerShift) - 1;
 constexpr int kSkipRow = -(1 << 30); // stays negative after the in-segment rank is added
 constexpr int kDequantChunks = 8;    // expert chunks of the overlapped FP8 de-quantisation
-constexpr int kJobCounters = 2 * kDequantChunks;   // one per expert GEMM launch of a forward
+constexpr int kJobCounters = MG_JOB_COUNTERS;      // one per expert GEMM launch of a forward
+static_assert(kJobCounters >= 2 * kDequantChunks, "every part of the experts has a counter for either product");
 constexpr int kStageSlots = 32;      // forwards whose per-stage times are kept for averaging
 
 // thread-local error text -------------------------------------------------------------
@@ -123,6 +124,7 @@ struct Handle {
   bool stage_timing;      // record an event after every stage of mg_moe_forward
   int stage_calls;        // forwards recorded since timing was enabled
   cudaEvent_t stage_ev[kStageSlots][MG_STAGE_COUNT + 1];   // ring of event sets, one per forward
+  int32_t* job_counters = nullptr;   // the caller's (mg_set_job_counters)
   bool chain = false;     // launches follow one another inside one forward (launch_chained)
   mutable TensorMapCache tmaps;
   mutable WlMapCache wl_maps;

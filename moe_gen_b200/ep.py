@@ -191,6 +191,7 @@ class EPMoELayer:
                 mb.h_buf = torch.empty(cap, lay.I, dtype=torch.bfloat16, device=self.dev)
                 mb.flag = torch.zeros(1, dtype=torch.int32, device=self.dev)
                 mb.delta = torch.zeros(E, **i32)
+                mb.jobs = torch.zeros(L.JOB_COUNTERS, **i32)
                 mb.counts_host = torch.zeros(self.world, E, dtype=torch.int32).pin_memory()
                 mb.counts_event = torch.cuda.Event()
                 mb.stream = self._streams[i]
@@ -425,7 +426,7 @@ class EPMoELayer:
             # ---- experts, one micro-batch after the other on the tensor cores
             prev = None
             for mb in self._mbs:
-                with torch.cuda.stream(mb.stream):
+                with torch.cuda.stream(mb.stream), lay.job_counters(mb.jobs):
                     if prev is not None:
                         mb.stream.wait_event(prev)   # also orders the reuse of the de-quantised weights
                     if self.copy_return:

@@ -8,6 +8,7 @@ The staged methods mirror the steps of the reference's layer
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from typing import Optional, Tuple
 
@@ -325,6 +326,19 @@ class MoELayer:
             L.check(self.lib.mg_permute_rows(self._h, x.data_ptr(), dst_row.data_ptr(), x.shape[0],
                                              perm.data_ptr(), self._stream()))
         return perm
+
+    @contextlib.contextmanager
+    def job_counters(self, buf: torch.Tensor):
+        """The expert calls inside hand out their jobs by counters in buf (int32 [JOB_COUNTERS] on the layer's
+        device, theirs alone until they have run) instead of in fixed turns (mg_set_job_counters)."""
+        self._check_in(buf, torch.int32, "job counters")
+        if buf.numel() < L.JOB_COUNTERS:
+            raise ValueError(f"job counters: {buf.numel()} words, {L.JOB_COUNTERS} needed")
+        L.check(self.lib.mg_set_job_counters(self._h, buf.data_ptr()))
+        try:
+            yield
+        finally:
+            L.check(self.lib.mg_set_job_counters(self._h, None))
 
     def expert_ffn(self, perm_x: torch.Tensor, pad_offsets: torch.Tensor, counts: torch.Tensor,
                    predequant: bool = False):

@@ -27,6 +27,7 @@ OPT_RING_BYTES = 7
 OPT_RING_PERSIST = 8
 OPT_ROWS_BOUND = 9
 OPT_ROUTE_FIXUP = 10
+JOB_COUNTERS = 16
 FP8_AUTO, FP8_PREDEQUANT, FP8_IN_KERNEL, FP8_RING = 0, 1, 2, 3
 
 
@@ -65,6 +66,7 @@ SIGNATURES = {
     "mg_dequant_ws_bytes": [_vp, _P(_sz)],
     "mg_dequant_start": [_vp, _vp, _vp, _vp],
     "mg_expert_ffn": [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp],
+    "mg_set_job_counters": [_vp, _vp],
     "mg_shared_ffn": [_vp, _vp, _i64, _vp, _vp, _vp, _vp],
     "mg_combine": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp],
     "mg_moe_forward": [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _sz, _vp, _vp],

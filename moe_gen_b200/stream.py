@@ -131,12 +131,14 @@ class StreamedMoELayer:
             self.copy_stream.wait_stream(comp)
             for j, g in enumerate(todo[:self.slots]):
                 self._copy_group(g, j)
+            jobs = torch.empty(L.JOB_COUNTERS, dtype=torch.int32, device=dev)    # the groups follow one another on `comp`
             for j, g in enumerate(todo):
                 b = j % self.slots
                 comp.wait_event(self.ready[b])
-                L.check(lib.mg_expert_ffn(lay._h, perm.data_ptr(), pad.data_ptr() + 4 * g * n,
-                                          counts.data_ptr() + 4 * g * n, rows, self.slot[b].data_ptr(),
-                                          hbuf.data_ptr(), outr.data_ptr(), _ptr(deq), st))
+                with lay.job_counters(jobs):
+                    L.check(lib.mg_expert_ffn(lay._h, perm.data_ptr(), pad.data_ptr() + 4 * g * n,
+                                              counts.data_ptr() + 4 * g * n, rows, self.slot[b].data_ptr(),
+                                              hbuf.data_ptr(), outr.data_ptr(), _ptr(deq), st))
                 self.free[b].record(comp)
                 if j + self.slots < len(todo):
                     self.copy_stream.wait_event(self.free[b])

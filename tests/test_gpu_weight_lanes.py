@@ -227,3 +227,46 @@ def test_jobs_handed_out_by_the_counter_equal_fixed_turns(built_lib, T, fp8):
         torch.cuda.synchronize()
         assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     assert layer.device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("pattern", sorted(PATTERNS))
+def test_stage_call_by_counters_equals_fixed_turns(built_lib, pattern, fp8):
+    """mg_expert_ffn with the caller's job counters, whose words hold anything before: the bits of fixed turns, also
+    with FP8 weights converted first (a counter per part and product)."""
+    from moe_gen_b200 import MoELayer
+    from moe_gen_b200 import lib as L
+    hidden, inter, n_experts = 2304, 2176, 24
+    if fp8:
+        layer = _random_fp8_layer(hidden, inter, n_experts, 6)
+    else:
+        layer = MoELayer(hidden=hidden, inter=inter, n_experts=n_experts, top_k=2, device="cuda:0")
+        layer.set_router(torch.zeros(n_experts, hidden))
+        g = torch.Generator(device="cuda").manual_seed(6)
+        for e in range(n_experts):
+            layer.load_expert(e, *((torch.randn(*shape, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+                                   for shape in ((inter, hidden), (inter, hidden), (hidden, inter))))
+    cnt = torch.tensor((PATTERNS[pattern] * n_experts)[:n_experts])
+    pad = torch.zeros(n_experts + 1, dtype=torch.int64)
+    pad[1:] = ((cnt + 127) // 128 * 128).cumsum(0)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = (torch.randn(int(pad[-1]), hidden, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    live = torch.zeros(x.shape[0], dtype=torch.bool, device="cuda")
+    for e, c in enumerate(cnt.tolist()):
+        live[pad[e]:pad[e] + c] = True
+    pad_d, cnt_d = pad.int().cuda(), cnt.int().cuda()
+    want = layer.expert_ffn(x, pad_d, cnt_d)
+    buf = torch.full((L.JOB_COUNTERS + 1,), 12345, dtype=torch.int32, device="cuda")
+    with layer.job_counters(buf[:L.JOB_COUNTERS]):
+        got = [layer.expert_ffn(x, pad_d, cnt_d) for _ in range(3)]
+        if fp8:
+            got.append(layer.expert_ffn(x, pad_d, cnt_d, predequant=True))
+    used = buf.clone()
+    got.append(layer.expert_ffn(x, pad_d, cnt_d))
+    torch.cuda.synchronize()
+    assert layer.device_status() == (0, 0)
+    assert int(used[L.JOB_COUNTERS]) == 12345 and bool((used[:L.JOB_COUNTERS] != 12345).all())
+    assert torch.equal(used, buf)                          # not touched once they are no longer set
+    for out in got:
+        for a, b in zip(out, want):
+            assert torch.equal(a[live].view(torch.int16), b[live].view(torch.int16))
