@@ -772,7 +772,7 @@ int mg_workspace_ptr(mg_handle hh, void* d_ws, int64_t max_tokens, int64_t max_r
   Handle* h = check(hh);
   if (!h) return MG_ERR_STATE;
   MG_REQUIRE(d_ws && ptr, MG_ERR_NULL, "null argument");
-  MG_REQUIRE(which >= 0 && which < WS_N, MG_ERR_SHAPE, "which=%d out of range", which);
+  MG_REQUIRE(which >= 0 && which < WS_JOBS, MG_ERR_SHAPE, "which=%d out of range", which);
   *ptr = static_cast<uint8_t*>(d_ws) + ws_layout(h, max_tokens, max_rows).off[which];
   return MG_OK;
 }

@@ -37,3 +37,15 @@ def test_back_to_back_forwards_equal_single_launches(built_lib, name, T):
         assert torch.equal(y.view(torch.int16), want[i % 3].view(torch.int16)), i
     for i, y in enumerate(got_block):
         assert torch.equal(y.view(torch.int16), want_block[i % 3].view(torch.int16)), i
+
+
+def test_workspace_sections_that_may_be_asked_for(built_lib):
+    """The section behind the last of them, the job counters, is the library's own."""
+    import ctypes as C
+    from moe_gen_b200 import lib as L
+    layer = make_layer(SPECS["bf16_renorm"], O.make_inputs(SPECS["bf16_renorm"], 1, 3)[1])
+    ws = layer._workspace(64)
+    p, got = C.c_void_p(), []
+    for which in range(-1, 18):
+        got.append(layer.lib.mg_workspace_ptr(layer._h, ws.data_ptr(), 64, 0, which, C.byref(p)))
+    assert got == [-2] + [0] * 15 + [-2] * 3
