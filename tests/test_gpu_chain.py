@@ -49,3 +49,22 @@ def test_workspace_sections_that_may_be_asked_for(built_lib):
     for which in range(-1, 18):
         got.append(layer.lib.mg_workspace_ptr(layer._h, ws.data_ptr(), 64, 0, which, C.byref(p)))
     assert got == [-2] + [0] * 15 + [-2] * 3
+
+
+@pytest.mark.parametrize("fill", [0, 0x7f, 0xff])
+@pytest.mark.parametrize("T", [3, 200, 1500])
+@pytest.mark.parametrize("name", sorted(SPECS))
+def test_what_a_workspace_held_before_does_not_matter(built_lib, name, T, fill):
+    """The expert GEMMs peek at the workspace's counts before the plan is known to be there; the peek may show anything,
+    such as zeros, large numbers or negative ones, and decides nothing."""
+    x, W = O.make_inputs(SPECS[name], T, 80 + T)
+    layer = make_layer(SPECS[name], W)
+    x = x.cuda()
+    layer.set_stage_timing(True)
+    want = layer.forward(x).clone()
+    torch.cuda.synchronize()
+    layer.set_stage_timing(False)
+    for _ in range(3):
+        layer._ws.fill_(fill)
+        assert torch.equal(layer.forward(x).view(torch.int16), want.view(torch.int16))
+    assert layer.device_status() == (0, 0)

@@ -270,3 +270,26 @@ def test_stage_call_by_counters_equals_fixed_turns(built_lib, pattern, fp8):
     for out in got:
         for a, b in zip(out, want):
             assert torch.equal(a[live].view(torch.int16), b[live].view(torch.int16))
+
+
+def test_auto_converts_first_where_the_kernels_that_convert_refuse(built_lib):
+    """Inner sizes beyond 16384: MG_FP8_AUTO de-quantises first from 1024 rows per expert of the call on, or of the batch
+    the caller says it belongs to; below, the call is refused."""
+    from moe_gen_b200 import lib as L
+    layer = _random_fp8_layer(256, 16512, 4, 9)
+    g = torch.Generator(device="cuda").manual_seed(10)
+    layer.set_router(torch.randn(4, 256, generator=g, device="cuda") * 0.05)
+    x = (torch.randn(2048, 256, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    got = layer.forward(x)
+    with pytest.raises(L.MoeGenError, match="K a multiple of 128 up to 16384"):
+        layer.forward(x[:2047])
+    layer.set_option(L.OPT_BATCH_TOKENS, 2048)
+    part = layer.forward(x[:3])
+    layer.set_option(L.OPT_BATCH_TOKENS, 0)
+    layer.set_option(L.OPT_FP8_MODE, L.FP8_PREDEQUANT)
+    want, want_part = layer.forward(x), layer.forward(x[:3])
+    torch.cuda.synchronize()
+    assert layer.device_status() == (0, 0)
+    assert bool(torch.isfinite(want.float()).all()) and bool((want != 0).any())
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert torch.equal(part.view(torch.int16), want_part.view(torch.int16))
