@@ -1381,7 +1381,7 @@ static EncodeTiledFn get_encode_fn() {
 // are kept in the handle: a forward at decode sizes is short enough for ~60 driver calls to show.
 int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
               TensorMapKind kind) {
-  const bool fp8 = kind == TM_FP8_ROWS || kind == TM_FP8_SW128;
+  const bool fp8 = kind == TM_FP8_ROWS;
   TensorMapCache& c = h->tmaps;
   for (int i = 0; i < c.used; ++i) {
     const TensorMapCache::Entry& e = c.e[i];
@@ -1394,7 +1394,7 @@ int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64_t rows
   MG_REQUIRE(fn != nullptr, MG_ERR_DRIVER, "cuTensorMapEncodeTiled not available from the driver");
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * (fp8 ? 1 : 2)};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(kind == TM_OUT_PIECE ? 32 : kind == TM_OUT_16 ? 16 : kind == TM_FP8_SW128 ? 128 : BK), box_rows};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(kind == TM_OUT_PIECE ? 32 : kind == TM_OUT_16 ? 16 : BK), box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -272,8 +272,7 @@ enum TensorMapKind : uint32_t {
   TM_BF16 = 0,        // boxes of 64 bf16, SWIZZLE_128B: MMA operand tiles
   TM_FP8_ROWS = 1,    // boxes of 64 bytes, unswizzled
   TM_OUT_PIECE = 2,   // boxes of 32 bf16, SWIZZLE_64B: the epilogue's stores
-  TM_OUT_16 = 4,      // boxes of 16 bf16, unswizzled: the SwiGLU stores of the weight-lane kernel
-  TM_FP8_SW128 = 3,   // boxes of 128 bytes, SWIZZLE_128B: one row per converter thread, no bank conflicts
+  TM_OUT_16 = 3,      // boxes of 16 bf16, unswizzled: the SwiGLU stores of the weight-lane kernel
 };
 
 int encode_2d(const Handle* h, CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,

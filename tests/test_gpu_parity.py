@@ -312,7 +312,7 @@ def test_fp8_weights_converted_in_the_gemm_equal_dequantise_first(built_lib, H, 
     worst, _ = _check_expert_rows(spec, W, xd, layer, idx)
     assert worst < 5e-3
     ys = []
-    for pair in (0, 1):                                # one CTA per SM / SM pairs
+    for pair in (0, 1):                                # weights on the lanes / tokens on an SM pair's lanes
         layer.set_option(2, pair)
         for mode in (0, 1, 2, 3, 1):                   # auto, pre-dequantise, in-kernel, ring, again
             layer.set_option(1, mode)
@@ -328,7 +328,9 @@ def test_fp8_weights_converted_in_the_gemm_equal_dequantise_first(built_lib, H, 
 
 @pytest.mark.parametrize("T", [3, 130, 700, 3000])
 def test_sm_pair_gemm_equals_single_cta_gemm(built_lib, T):
-    """The 2-CTA (cta_group::2) kernel computes the same sums in the same order as the 1-CTA one."""
+    """The kernel with 256 tokens on an SM pair's lanes computes the same sums in the same order as the default ones: the
+    weight-lane kernel for the experts, the one-CTA kernel for the shared expert.  (Experts on the one-CTA kernel: FP8
+    layers with 128-row tiles, above.)"""
     spec = O.LayerSpec(512, 256, 16, 4, 256, combine_mode=O.COMBINE_FP32)
     x, W = O.make_inputs(spec, T, 60 + T)
     layer = make_layer(spec, W, DEV)
