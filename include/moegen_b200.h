@@ -478,11 +478,14 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
  *                      a separate pass on a side stream one chunk of experts ahead of the bf16 GEMMs;
  *   MG_FP8_RING        the GEMM kernel's CTAs convert every weight once per expert into a bf16 ring of
  *                      MG_OPT_RING_BYTES and fetch their B tiles from it by TMA: no bf16 copy of the weights,
- *                      58 MB of scratch; measured 5 % slower than MG_FP8_PREDEQUANT at 65536 tokens of the
- *                      DeepSeek-V3 layer (the ring does not stay in L2), so only on request;
- *   MG_FP8_AUTO        (default) in-kernel (DeepSeek-V3 shape, in-kernel against pre-dequantise: 22.5 and 29.2 ms
- *                      at 1024 rows per expert, 43.9 and 50.9 ms at 2048); inner sizes beyond 16384, which the kernels
- *                      that convert refuse, pre-dequantise from 1024 rows per expert on.
+ *                      58 MB of scratch; measured slower than the others at 65536 tokens of the DeepSeek-V3 layer
+ *                      (56 ms; pre-dequantise 51, in-kernel 44: the ring does not stay in L2), so only on request;
+ *   MG_FP8_AUTO        (default) in mg_moe_forward and its host, block and from-logits forms in-kernel (DeepSeek-V3
+ *                      shape, in-kernel against pre-dequantise: 22.7 and 29.2 ms at 1024 rows per expert, 44.2 and
+ *                      51.3 ms at 2048; 65536 tokens from host memory in chunks of 4096: 62 and 81); inner sizes beyond
+ *                      16384, which the kernels that convert refuse, pre-dequantise from 1024 rows per expert on.
+ *                      mg_expert_ffn and the expert-parallel expert calls pre-dequantise where they are given scratch
+ *                      and convert in the kernel where not.
  * All give bit-identical results.  Set before asking mg_workspace_bytes / mg_dequant_ws_bytes. */
 #define MG_OPT_FP8_MODE    1
 #define MG_FP8_AUTO        0

@@ -1588,14 +1588,16 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   }
   // FP8 weights converted in the kernel, by default with the weights on the lanes: one conversion per 384 tokens of
   // an expert and MMAs as wide as its rows.  V3 layer, ms, 128-row tiles / 256-row tiles / weights on the lanes: 64
-  // tokens 3.7 / 4.5 / 2.6, 4096 skewed tokens 8.0 / 7.7 / 5.5, 16384 tokens 20.5 / 16.3 / 14.1, 32768 tokens 37.4 /
-  // 30.1 / 27.3.  MG_OPT_FP8_M256 = 0 or 2 asks for the tiles with tokens on the lanes.
+  // tokens 3.5 / 4.1 / 2.1, 4096 skewed tokens 8.2 / 7.7 / 4.8, 16384 tokens 20.6 / 16.4 / 12.0, 32768 tokens 38.9 /
+  // 30.1 / 22.7.  MG_OPT_FP8_M256 = 0 or 2 asks for the tiles with tokens on the lanes: checks of this one, no use else.
   const bool convert = p.b_fp8 && !dense && !f32_out && !pair;
   if (convert && h->opt_fp8_m256 == 1) return launch_gemm_wl(h, p, st);
   // bf16 weights of experts as well: MMAs as wide as an expert's rows and not 128 or 256 of them, and fewer operand bytes
   // per SM (40 KiB per 128 x 384 x 64 instead of 48 per 128 x 256 x 64).  Layer, ms, 128x256 tiles on one CTA per SM and
   // weights on the lanes: Mixtral 61 tokens 0.545 and 0.491, 16384 9.32 and 8.91; V2-236B 512 tokens 1.36 and 1.25, 32768
   // 11.58 and 11.58 (power cap); V2-Lite 8 tokens 0.170 and 0.160, 512 0.255 and 0.248, 2048 0.402 and 0.384.
+  // Behind it by 2 % where 512 rows of an expert are two jobs and the last turn of the pairs is nearly empty (Mixtral 2048
+  // tokens 1.48 and 1.50).
   // Shared experts (dense) stay with the tokens on the lanes: beside the routing kernels on another stream a pair's CTAs,
   // with all of the SM's shared memory, keep those waiting (V2-Lite, 4096 tokens 0.63 and 0.68 ms), and later they are
   // level.

@@ -14,8 +14,9 @@
 // What bounds it.  Decode: the weights' bytes and the conversion, which share the step.  DeepSeek-V3 shape, 64 tokens,
 // gate/up + down products: 2.30 ms before and 1.80 ms with the changes below, 5.6 TB/s of the measured 6.5 (without
 // the conversion 1.49 ms, the HBM rate).  From a few thousand tokens on: the 1000 W cap (SM clock 1.1-1.3 GHz), where
-// every weight byte moved and converted once more costs time: 16384 tokens 11.4 and 10.5 ms.  Jobs of at most 320, 256
-// and 192 tokens were 1, 9 and 14 % slower there; prefetching tokens or weights into L2 ahead of the rings 2 to 15 %.
+// every weight byte moved and converted once more costs time: 16384 tokens 11.4 and 10.5 ms (10.0 by the counter).  Jobs of at
+// most 320, 256 and 192 tokens were 1, 9 and 14 % slower there; prefetching tokens or weights into L2 ahead of the rings 2 to
+// 15 %.
 //   * two products by one packed multiplication (convert16): the converters are bound by issue slots, 2.8 instructions
 //     per element of which 2.5 are conversions and the product: 64 tokens 2.30 and 2.10 ms;
 //   * 128 K elements per hand-over: half as many waits, votes and commits per element, on both sides;
@@ -27,9 +28,10 @@
 //     or 16 tokens (4096 skewed tokens 4.89 and 4.77 ms);
 //   * jobs alternate between the two ends of the accumulator columns and the next one starts as soon as the columns that
 //     both need have been read (3.85 and 3.80 ms; the clock falls as the tensor cores idle less).
-//   * jobs are handed out by a counter (next_job), not in fixed turns: pairs that start late or get long jobs take fewer,
-//     and the jobs under way stay neighbours in the list, whose weights and tokens L2 then holds: V3 layer 16384 tokens
-//     13.1 and 11.9 ms, 65536 tokens 51 and 44, 4096 skewed 4.94 and 4.79.
+//   * jobs are handed out by a counter (next_job, where the caller has memory for one), not in fixed turns: pairs that
+//     start late or get long jobs take fewer, and the jobs under way stay neighbours in the list, whose weights and tokens
+//     L2 then holds: V3 layer 16384 tokens 13.1 and 11.9 ms, 65536 tokens 51 and 44, 4096 skewed 4.94 and 4.79; both
+//     products alone, V2-236B 11000 tokens 3.97 and 3.31.
 // Direct stores of the output from registers were slower than pieces staged for TMA (down product, 16384 tokens 4.5
 // against 4.0 ms).
 //
@@ -676,8 +678,8 @@ int launch_kernel(const Handle* h, const WlMaps& maps, const WlArgs& a, int grid
   return MG_OK;
 }
 
-// From the handle's cache, by what the maps are made of: a forward's launches are few and the same ones again, and fourteen
-// driver calls a launch are 10 us that a decode step would see.
+// From the handle's cache, by what the maps are made of: a forward's launches are few and the same ones again.  Encoding the
+// maps anew, as for a batch size not seen lately, takes a forward 3 us more on the host (V2-Lite 36 and 39 us).
 template <bool FP8>
 int wl_maps(const Handle* h, const GemmProblem& p, bool swiglu, const WlMaps** out) {
   WlMapCache& cache = h->wl_maps;

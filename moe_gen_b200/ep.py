@@ -218,8 +218,8 @@ class EPMoELayer:
             self.shared_out = torch.empty(T, lay.H, dtype=torch.bfloat16, device=self.dev) if lay.Is else None
             nd = C.c_size_t()
             L.check(self.lib.mg_dequant_ws_bytes(lay._h, C.byref(nd)))
-            # FP8: scratch for the library's FP8 mode (the L2-resident ring from 1024 rows per expert on, or
-            # the bf16 copy of pre-dequantise mode); below that the GEMMs convert in the kernel
+            # FP8: scratch for the library's FP8 mode (the ring, or the bf16 copy of pre-dequantise mode; the automatic
+            # mode makes the copy from 1024 rows per expert on); without it the GEMMs convert in the kernel
             mode = lay.options.get(L.OPT_FP8_MODE, 0)
             Tb = max(T, self._batch_tokens)    # parts of one batch share the de-quantised copy
             use_deq = nd.value > 0 and (mode in (L.FP8_PREDEQUANT, L.FP8_RING) or
