@@ -97,6 +97,7 @@ struct WlArgs {
   int scale_cols;
   int32_t* next_job;            // counts the jobs handed out beyond each pair's first; nullptr: every n_pairs-th job
   int32_t* status;
+  int rows;                     // of the token matrix: the first row number behind it
   int chained;                  // launched while the kernel before may still run (launch_chained)
 };
 
@@ -390,6 +391,24 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
         const int h1 = min(j.n_tok, 256) >> 1, h2 = (j.n_tok >> 1) - h1;
         const int row1 = j.row0 + static_cast<int>(rank) * h1, row2 = j.row0 + 256 + static_cast<int>(rank) * h2;
         const int kpt = steps_per_stage<FP8>(j.n_tok >> 1);
+        if (j.n_tok == 32) {
+          // Two groups of eight rows, each with all steps of the stage, or zeros for a group without a live one: a box
+          // that begins behind the last row reads nothing.  Rows that nobody wrote cost their bytes and, at the power cap,
+          // the multipliers' work on whatever they hold: layer, us, all 32 rows and this, workspace full of random values:
+          // V3 16 tokens 1112 and 1064, 64 tokens 2244 and 2139, 256 tokens 2659 and 2555; zeros there already: 2152 and
+          // 2146; Mixtral 61 tokens 476 and 472, V2-236B 512 tokens 1238 and 1229.
+          const int live = j.left - 16 * static_cast<int>(rank);
+          const int g0 = live > 0 ? row1 : g.rows, g1 = live > 8 ? row1 + 8 : g.rows;
+          for (int kb = 0; kb < g.k_steps; kb += kpt, r.next(C::ST)) {
+            if (!mbar_wait(smem_u32(&tempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 52)) break;
+            const uint32_t fb = smem_u32(&tfull[r.i]);
+            const uint32_t dst = t_base + r.i * C::T_STAGE;
+            if (rank == 0) mbar_expect_tx(fb, kpt * 32 * 128);
+            tma_load_3d_pair(dst, &maps.t8, 0, g0, kb, fb);
+            tma_load_3d_pair(dst + kpt * 1024, &maps.t8, 0, g1, kb, fb);
+          }
+          continue;
+        }
         const CUtensorMap* m1 = &maps.t[(h1 >> 4) - 1];
         const CUtensorMap* m2 = &maps.t2[(max(h2, 16) >> 4) - 1];
         for (int kb = 0; kb < g.k_steps; kb += kpt, r.next(C::ST)) {
@@ -423,7 +442,8 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
         const int n1 = min(j.n_tok, 256), n2 = j.n_tok - n1;
         const uint32_t id1 = id0 | (static_cast<uint32_t>(n1 >> 3) << 17), id2 = id0 | (static_cast<uint32_t>(n2 >> 3) << 17);
         const uint32_t d = tmem_base + (h ? C::ACC_COLS - j.n_tok : 0);
-        const int kpt = steps_per_stage<FP8>(j.n_tok >> 1), step_bytes = j.n_tok * 64;
+        const int kpt = steps_per_stage<FP8>(j.n_tok >> 1), step_bytes = j.n_tok == 32 ? 1024 : j.n_tok * 64;
+        const uint32_t group_bytes = j.n_tok == 32 ? kpt * 1024 : 1024;      // see the token role
         int in_stage = 0;
         if (FP8) {
           for (int kb = 0; kb < g.k_steps; kb += 2) {
@@ -438,7 +458,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
                 tc_fence_after();
               }
               const uint32_t tb = t_base + rt.i * C::T_STAGE + in_stage * step_bytes;
-              const uint64_t db = make_smem_desc(tb);
+              const uint64_t db = make_smem_desc(tb, group_bytes);
               const uint64_t db2 = make_smem_desc(tb + n1 * 64);
               const uint32_t a = tmem_base + C::ACC_COLS + ra.i * WL_A_COLS + half * (WL_A_COLS / 2);
 #pragma unroll
@@ -466,7 +486,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
             tc_fence_after();
             const uint32_t tb = t_base + rt.i * C::T_STAGE + in_stage * step_bytes;
             const uint64_t da = make_smem_desc(w_base + ra.i * WL_W_STAGE);
-            const uint64_t db = make_smem_desc(tb), db2 = make_smem_desc(tb + n1 * 64);
+            const uint64_t db = make_smem_desc(tb, group_bytes), db2 = make_smem_desc(tb + n1 * 64);
 #pragma unroll
             for (int k = 0; k < WL_K / 16; ++k) {
               const uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
@@ -698,6 +718,8 @@ int wl_maps(const Handle* h, const GemmProblem& p, bool swiglu, const WlMaps** o
                     {WL_K, n, i < 8 ? static_cast<uint32_t>(steps_per_stage<FP8>(n)) : 1u});
   }
   if (rc == MG_OK)
+    rc = encode_map(&m.t8, p.a, false, 3, {WL_K, rows, steps}, {2 * K, 2 * WL_K}, {WL_K, 8, steps_per_stage<FP8>(16)});
+  if (rc == MG_OK)
     rc = encode_2d(h, &m.c, p.out, rows, static_cast<uint64_t>(p.ldo), swiglu ? 32 : 16, swiglu ? TM_OUT_16 : TM_OUT_PIECE);
   if (rc != MG_OK) return rc;
   WlMapCache::Entry& e = cache.e[cache.next];
@@ -731,6 +753,7 @@ int launch_gemm_wl(const Handle* h, const GemmProblem& p, cudaStream_t st) {
   a.scale_cols = p.K / 128;
   a.next_job = p.next_job;
   a.status = h->d_status;
+  a.rows = static_cast<int>(p.a_rows);
   a.chained = h->chain ? 1 : 0;
   const int max_tokens = p.b_fp8 ? WlCfg<true>::MAX_TOKENS : WlCfg<false>::MAX_TOKENS;
   const int64_t tiles = (p.a_rows + max_tokens - 1) / max_tokens + p.n_groups;

@@ -186,12 +186,12 @@ __device__ __forceinline__ void tc_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// K-major, 128B-swizzled operand tile: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
+// K-major, 128B-swizzled operand tile: rows of 128 bytes, 8-row groups group_bytes apart.
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t group_bytes = 1024) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);        // start address, 16-byte units
   d |= static_cast<uint64_t>(1) << 16;                        // leading byte offset (unused here)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                // stride byte offset between 8-row groups
+  d |= static_cast<uint64_t>(group_bytes >> 4) << 32;         // stride byte offset between 8-row groups
   d |= static_cast<uint64_t>(1) << 46;                        // descriptor version (Blackwell)
   d |= static_cast<uint64_t>(2) << 61;                        // SWIZZLE_128B
   return d;

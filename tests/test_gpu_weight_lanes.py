@@ -67,6 +67,15 @@ def test_expert_products_at_job_edges(built_lib, counts, fp8):
         _close(out[s], ro, mo, ("out", e, c))
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("counts", [
+    [7, 8, 9, 15, 16, 17, 23, 24],         # jobs of 32 tokens leave out groups of eight without a live row
+    [25, 1, 0, 41, 8, 392, 16, 400],
+])
+def test_expert_products_at_the_edges_of_token_groups(built_lib, counts, fp8):
+    test_expert_products_at_job_edges(built_lib, counts, fp8)
+
+
 @pytest.mark.parametrize("T", [1, 31, 32, 33, 256, 257, 384, 385, 1000, 3500])
 def test_shared_expert_at_job_edges(built_lib, T):
     spec = O.LayerSpec(512, 128, 8, 2, 384, 1, 1, O.GATE_SOFTMAX_GREEDY, False, 1.0, O.WEIGHT_BF16, O.COMBINE_FP32)
