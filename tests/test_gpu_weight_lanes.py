@@ -71,6 +71,8 @@ def test_expert_products_at_job_edges(built_lib, counts, fp8):
 @pytest.mark.parametrize("counts", [
     [7, 8, 9, 15, 16, 17, 23, 24],         # jobs of 32 tokens leave out groups of eight without a live row
     [25, 1, 0, 41, 8, 392, 16, 400],
+    [258, 287, 288, 289, 319, 320, 321, 0],     # jobs of 288, 320, 352 and 384 tokens are two MMAs per K step
+    [351, 352, 353, 290, 0, 383, 700, 2],
 ])
 def test_expert_products_at_the_edges_of_token_groups(built_lib, counts, fp8):
     test_expert_products_at_job_edges(built_lib, counts, fp8)
