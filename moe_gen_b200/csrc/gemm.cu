@@ -1568,10 +1568,12 @@ int launch_grouped_gemm(const Handle* h, const GemmProblem& p, cudaStream_t st) 
   // 49 and 23, at the rule's upper end, where the rows are read by 8 CTAs, 2304 tokens 53 and 27; V2-236B 512 tokens 37
   // and 20, 3712 tokens 40 and 23; 64 experts of 7168 columns 9472 tokens 55 and 39.  Wide tiles with the elected
   // issue: V3 2305 tokens 52.
-  const bool narrow = f32_out && dense && p.n_per_group > BN_NARROW &&
+  // 8 experts (16 columns) of 4096: 61 tokens 20 and 12, 16384 tokens 35 and 32, for the deeper ring.
+  const bool narrow = f32_out && dense &&
                       (p.dense_rows + BM - 1) / BM * ((p.n_per_group + BN_NARROW - 1) / BN_NARROW) <= h->sm_count;
   if (f32_out) {
-    bn = narrow ? BN_NARROW : static_cast<int>(round_up(p.n_per_group, 16));
+    bn = static_cast<int>(round_up(p.n_per_group, 16));
+    if (narrow && bn > BN_NARROW) bn = BN_NARROW;
     MG_REQUIRE(p.n_per_group <= BN_MAX && p.n_groups == 1 && p.n_per_group % 4 == 0, MG_ERR_SHAPE,
                "fp32-output GEMM needs one group of <=256 columns (multiple of 4), got %d", p.n_per_group);
   } else {
