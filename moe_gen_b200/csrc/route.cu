@@ -1098,8 +1098,13 @@ int launch_permute_plan_static(const Handle* h, const int32_t* idx, int64_t T, i
 }
 
 // ---------------------------------------------------------------------------------------
-// row scatter: one warp per token, x row read once, written to each destination row
+// row scatter: a warp per token, or per slice of one, x row read once, written to each destination row
 // ---------------------------------------------------------------------------------------
+// Few tokens: a warp that copies 14 KB to 8 places is a chain of stores; cut into slices of at least 128 vectors while there
+// are fewer than 16 warps per SM.  Neighbouring slices share a block: where a block of this kernel runs, the GEMM behind it
+// cannot be placed early (slices of 32 vectors, a block each: V3 1 token 151 and 157 us).  Kernel, us, a warp per token and
+// this: V3 64 tokens 21 and 6, V2-236B 512 tokens 25 and 15; layer: V3 8 tokens 621 and 616, V2-236B 8 tokens 350 and 344, 512
+// tokens 1228 and 1221.
 // PEER: dst_row packs (destination rank << kPeerShift | row) and rows are written to that
 // rank's buffer through its peer mapping (plain stores over NVLink).
 // DEDUP: when several picks of a token go to the same rank, only the first one's row travels; for
@@ -1109,13 +1114,16 @@ int launch_permute_plan_static(const Handle* h, const int32_t* idx, int64_t T, i
 // expert's output for that row has to go: source rank << kPeerShift | (token * k + slot).
 template <bool PEER, bool DEDUP, bool BACK>
 __global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restrict__ x, const int32_t* dst_row,
-                                                           int64_t T, int k, int vec_per_row,
+                                                           int64_t T, int k, int vec_per_row, int slices, int v_chunk,
                                                            PeerPtrs bufs, PeerPtrs dups, PeerPtrs backs, int my_rank,
                                                            Guard guard) {
   chain_wait();
   chain_go();
   const int lane = threadIdx.x & 31;
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t t = PEER ? item : item / slices;
+  const int v_begin = PEER ? 0 : static_cast<int>(item - t * slices) * v_chunk;
+  const int v_end = PEER ? vec_per_row : min(vec_per_row, v_begin + v_chunk);
   if (t >= T) return;
   int32_t my_dst = lane < k ? dst_row[t * k + lane] : -1;
   if (my_dst >= 0 && !MG_GUARD((PEER ? (my_dst & kPeerRowMask) : my_dst) < guard.rows_bound &&
@@ -1138,12 +1146,12 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restri
     skip = __ballot_sync(0xFFFFFFFFu, my_first >= 0);
   }
   const uint4* src = x + t * vec_per_row;
-  for (int v0 = 0; v0 < vec_per_row; v0 += 128) {
+  for (int v0 = v_begin; v0 < v_end; v0 += 128) {
     uint4 val[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       int v = v0 + u * 32 + lane;
-      if (v < vec_per_row) val[u] = __ldg(src + v);
+      if (v < v_end) val[u] = __ldg(src + v);
     }
     for (int j = 0; j < k; ++j) {
       int32_t d = __shfl_sync(0xFFFFFFFFu, my_dst, j);
@@ -1153,7 +1161,7 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restri
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         int v = v0 + u * 32 + lane;
-        if (v < vec_per_row) dst[v] = val[u];
+        if (v < v_end) dst[v] = val[u];
       }
     }
   }
@@ -1191,12 +1199,15 @@ __global__ void __launch_bounds__(256) fill_duplicate_rows_kernel(uint4* __restr
 int launch_permute_rows(const Handle* h, const void* x, const int32_t* dst_row, int64_t T,
                         void* perm_x, cudaStream_t st) {
   if (T == 0) return MG_OK;
-  const int warps = 8;
-  dim3 grid(static_cast<unsigned>((T + warps - 1) / warps)), block(warps * 32);
+  const int warps = 8, vpr = h->d.hidden / 8, steps = (vpr + 127) / 128;
+  int64_t want = (static_cast<int64_t>(h->sm_count) * 16 + T - 1) / T;
+  if (want > steps) want = steps;
+  const int v_chunk = static_cast<int>((steps + want - 1) / want) * 128, slices = (vpr + v_chunk - 1) / v_chunk;
+  dim3 grid(static_cast<unsigned>((T * slices + warps - 1) / warps)), block(warps * 32);
   PeerPtrs bufs{};
   bufs.p[0] = perm_x;
   MG_CUDA(launch_chained(h, permute_rows_kernel<false, false, false>, grid, block, 0, st, static_cast<const uint4*>(x), dst_row,
-                         T, h->d.top_k, h->d.hidden / 8, bufs, bufs, bufs, 0, Guard{h->d_status, h->guard_rows, 1}));
+                         T, h->d.top_k, vpr, slices, v_chunk, bufs, bufs, bufs, 0, Guard{h->d_status, h->guard_rows, 1}));
   return MG_OK;
 }
 
@@ -1211,13 +1222,13 @@ int launch_dispatch_rows(const Handle* h, const void* x, const int32_t* dst, int
   const PeerPtrs& b = backs ? *backs : peers;
   const Guard guard{h->d_status, h->guard_rows, h->d.ep_size};
   if (dups != nullptr && backs != nullptr)
-    permute_rows_kernel<true, true, true><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, peers, d, b, me, guard);
+    permute_rows_kernel<true, true, true><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, 1, vpr, peers, d, b, me, guard);
   else if (dups != nullptr)
-    permute_rows_kernel<true, true, false><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, peers, d, b, me, guard);
+    permute_rows_kernel<true, true, false><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, 1, vpr, peers, d, b, me, guard);
   else if (backs != nullptr)
-    permute_rows_kernel<true, false, true><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, peers, d, b, me, guard);
+    permute_rows_kernel<true, false, true><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, 1, vpr, peers, d, b, me, guard);
   else
-    permute_rows_kernel<true, false, false><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, peers, d, b, me, guard);
+    permute_rows_kernel<true, false, false><<<grid, block, 0, st>>>(xs, dst, T, k, vpr, 1, vpr, peers, d, b, me, guard);
   MG_CUDA(cudaGetLastError());
   return MG_OK;
 }
