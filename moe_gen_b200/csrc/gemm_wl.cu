@@ -36,14 +36,16 @@
 // against 4.0 ms).
 //
 // Roles per CTA: warp 0 = weight TMA, warp 1 = token TMA, warp 2 = MMA issuer (leader CTA), warp 3 = job list and
-// TMEM owner, warps 4-11 = epilogue (two per lane quarter, alternate 32-token chunks), warps 12-19 = converters: a
-// thread owns one lane = one weight row; warps 12-15 take the even stages of 128 K elements, 16-19 the odd ones.
+// TMEM owner, warps 4-11 = epilogue (two per lane quarter, alternate 32-token chunks), warps 12-27 = converters: a
+// thread owns one lane = one weight row and 64 K elements of a stage; warps 12-19 take the even stages of 128 K elements,
+// 20-27 the odd ones.  Eight warps with all 128 elements each had less to issue while one of two per scheduler waits: V3, us,
+// 64 tokens 2116 and 2107, 1024 tokens 2873 and 2844, 333 skewed 1608 and 1595; level from 4096 tokens on.
 //
 // Barriers (per CTA unless said otherwise):
-//   wfull/wempty   weight ring, stages of 128 rows x 128 K bytes, released by the four converter warps that read it
+//   wfull/wempty   weight ring, stages of 128 rows x 128 K bytes, released by the eight converter warps that read it
 //   tfull/tempty   token ring; leader's tfull counts both CTAs' bytes, tempty by commit to both
 //   aready/afree   the two 64-column slots of converted weights in TMEM, one per converter group; aready on the leader
-//                  counts the four warps of both CTAs, afree by commit to both
+//                  counts the eight warps of both CTAs, afree by commit to both
 //   dfull/dempty   accumulators of even and odd jobs, dempty once an epilogue has read all of one
 //   dpart          an epilogue has read the columns that the next job's accumulator shares with its own
 //   jfull/jempty   the next job, for the roles of a CTA; mfull: its number, from the leader's list to the other CTA's
@@ -61,9 +63,9 @@ namespace {
 constexpr int WL_GROUP_T = 8;                  // token tiles per L2 reuse group (weight tiles vary slower inside)
 constexpr int WL_K = 64;                       // K elements per MMA step (one 128-byte swizzle row of bf16)
 constexpr int WL_W_STAGE = 128 * 128;          // 16 KiB: 128 rows of 64 bf16 or of 128 FP8
-constexpr int WL_A_SLOTS = 2;                  // FP8: converted weights, one slot per converter group
+constexpr int WL_A_SLOTS = 2;                  // FP8: converted weights, one slot per converter group of eight warps
 constexpr int WL_A_COLS = 64;                  // 128 bf16 per lane
-constexpr int WL_EPI_WARPS = 8, WL_CONV_WARPS = 8;
+constexpr int WL_EPI_WARPS = 8, WL_CONV_WARPS = 16;
 constexpr int WL_PIECE = 1024;                 // epilogue staging: 32 tokens x 16 outputs or 16 tokens x 32 outputs
 constexpr int WL_JOBS = 1;                     // announced ahead: few, so that the last jobs go to whoever is free
 constexpr int WL_AHEAD = 8;                     // weight stages brought into L2 while the kernel before still runs
@@ -266,7 +268,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
     for (int s = 0; s < C::SW; ++s) { mbar_init(smem_u32(&wfull[s]), 1); mbar_init(smem_u32(&wempty[s]), FP8 ? WL_CONV_WARPS / 2 : 1); }
     for (int s = 0; s < C::ST; ++s) { mbar_init(smem_u32(&tfull[s]), 1); mbar_init(smem_u32(&tempty[s]), 1); }
     if (FP8)
-      for (int s = 0; s < WL_A_SLOTS; ++s) { mbar_init(smem_u32(&aready[s]), 8); mbar_init(smem_u32(&afree[s]), 1); }
+      for (int s = 0; s < WL_A_SLOTS; ++s) { mbar_init(smem_u32(&aready[s]), WL_CONV_WARPS); mbar_init(smem_u32(&afree[s]), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&dfull[s]), 1); mbar_init(smem_u32(&dempty[s]), 2 * WL_EPI_WARPS); }
     mbar_init(smem_u32(dpart), 2 * WL_EPI_WARPS);
     for (int s = 0; s < WL_JOBS; ++s) {
@@ -631,10 +633,12 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
   } else if (FP8 && warp >= 4 + WL_EPI_WARPS) {
     // ---------------- FP8 -> bf16 converters: shared -> registers -> tensor memory ----------------
     const int quarter = warp & 3;
-    const uint32_t grp = (warp - 4 - WL_EPI_WARPS) >> 2;   // even / odd stages, counted over all jobs
+    const uint32_t grp = (warp - 4 - WL_EPI_WARPS) >> 3;   // even / odd stages, counted over all jobs
+    const uint32_t half = (warp - 4 - WL_EPI_WARPS) >> 2 & 1u;          // 64 K elements of a stage
     const int row = !SWIGLU ? quarter * 32 + lane : quarter * 16 + (lane & 15) + (lane & 16) * 4;
     const int block = SWIGLU ? lane >> 4 : static_cast<int>(rank);      // scale block row of this lane's weights
-    const uint32_t a_slot = tmem_base + C::ACC_COLS + grp * WL_A_COLS + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t a_slot = tmem_base + C::ACC_COLS + grp * WL_A_COLS + half * (WL_A_COLS / 2) +
+                            (static_cast<uint32_t>(quarter * 32) << 16);
     const int stages = g.k_steps / 2;
     Ring rw, rj;
     rw.i = grp;
@@ -653,23 +657,19 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
         ok = wait_warp(smem_u32(&wfull[rw.i]), rw.ph, abort_flag, g.status, 57);
         if (!ok) break;
         const uint8_t* src = smem + rw.i * WL_W_STAGE + row * 128;
-        uint4 q[8];
+        uint4 q[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const uint4*>(src + ((i ^ (row & 7)) << 4));
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const uint4*>(src + (((half * 4 + i) ^ (row & 7)) << 4));
         uint32_t o[32];
         convert32(q[0], q[1], s, o);
         convert32(q[2], q[3], s, o + 16);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&wempty[rw.i]));
         ok = wait_warp(smem_u32(&afree[grp]), ph ^ 1u, abort_flag, g.status, 58);
         if (!ok) break;
         ph ^= 1u;
         tc_fence_after();
         tc_st32(a_slot, o);
-        uint32_t o2[32];
-        convert32(q[4], q[5], s, o2);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&wempty[rw.i]));
-        convert32(q[6], q[7], s, o2 + 16);
-        tc_st32(a_slot + WL_A_COLS / 2, o2);
         rw.i += 2;
         if (rw.i >= C::SW) { rw.i -= C::SW; rw.ph ^= 1u; }
         tc_st_wait();
