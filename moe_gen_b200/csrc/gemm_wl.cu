@@ -131,7 +131,9 @@ __host__ __device__ constexpr int steps_per_stage(int h) {
 // few tokens with A in shared memory is bound by reading A (M256 K16, cycles at N = 32, 64, 96, 128: 39, 43, 50, 64, where
 // the flop rate is N / 2), so that 256 + 32 tokens took 167 cycles, where 160 + 128 take 144.
 // V2-236B (320 tokens per job), layer, ms, 256 + rest and this: 32768 tokens 11.51 and 11.36, 8192 tokens 3.31 and 3.26.
-__device__ __forceinline__ int first_part(int n_tok) { return n_tok <= 256 ? n_tok : ((n_tok >> 1) + 31) & ~31; }
+// FP8 weights come from tensor memory, where an MMA takes N / 2 at any width: as wide as it goes, then the rest.
+template <bool FP8>
+__device__ __forceinline__ int first_part(int n_tok) { return n_tok <= 256 ? n_tok : FP8 ? 256 : ((n_tok >> 1) + 31) & ~31; }
 
 // s_jp[e] = token tiles of the experts before e
 __device__ __forceinline__ Job locate_job(int job, const int* s_pad, const int* s_cnt, const int* s_jp, const WlArgs& g) {
@@ -396,7 +398,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
       Ring r, rj;
       Job j;
       while (take_job(j, rj)) {
-        const int h1 = first_part(j.n_tok) >> 1, h2 = (j.n_tok >> 1) - h1;
+        const int h1 = first_part<FP8>(j.n_tok) >> 1, h2 = (j.n_tok >> 1) - h1;
         const int row1 = j.row0 + static_cast<int>(rank) * h1, row2 = j.row0 + 2 * h1 + static_cast<int>(rank) * h2;
         const int kpt = steps_per_stage<FP8>(j.n_tok >> 1);
         if (j.n_tok == 32) {
@@ -417,8 +419,8 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
           }
           continue;
         }
-        const CUtensorMap* m1 = h2 > 0 ? &maps.t2[(h1 >> 4) - 4] : &maps.t[(h1 >> 4) - 1];
-        const CUtensorMap* m2 = &maps.t2[(max(h2, 64) >> 4) - 4];
+        const CUtensorMap* m1 = h2 > 0 && h1 < 128 ? &maps.t2[(h1 >> 4) - 1] : &maps.t[(h1 >> 4) - 1];
+        const CUtensorMap* m2 = &maps.t2[(max(h2, 16) >> 4) - 1];
         for (int kb = 0; kb < g.k_steps; kb += kpt, r.next(C::ST)) {
           if (!mbar_wait(smem_u32(&tempty[r.i]), r.ph ^ 1u, abort_flag, g.status, 52)) break;
           const uint32_t fb = smem_u32(&tfull[r.i]);
@@ -447,7 +449,7 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
         ++seq;
         n_before = j.n_tok;
         tc_fence_after();
-        const int n1 = first_part(j.n_tok), n2 = j.n_tok - n1;
+        const int n1 = first_part<FP8>(j.n_tok), n2 = j.n_tok - n1;
         const uint32_t id1 = id0 | (static_cast<uint32_t>(n1 >> 3) << 17), id2 = id0 | (static_cast<uint32_t>(n2 >> 3) << 17);
         const uint32_t d = tmem_base + (h ? C::ACC_COLS - j.n_tok : 0);
         const int kpt = steps_per_stage<FP8>(j.n_tok >> 1), step_bytes = j.n_tok == 32 ? 1024 : j.n_tok * 64;
@@ -718,8 +720,8 @@ int wl_maps(const Handle* h, const GemmProblem& p, bool swiglu, const WlMaps** o
   int rc = FP8 ? encode_map(&m.w, p.b, true, 3, {K, 128, blocks}, {K, 128 * K}, {128, 128 / both, both})
                : encode_map(&m.w, p.b, false, 4, {K, 16, blocks, 8}, {2 * K, 256 * K, 32 * K}, {WL_K, 16, both, 8 / both});
   const uint64_t rows = static_cast<uint64_t>(p.a_rows), steps = K / WL_K;
-  for (int i = 0; i < 11 && rc == MG_OK; ++i) {
-    const uint32_t n = 16 * (i < 8 ? i + 1 : i - 4);
+  for (int i = 0; i < 14 && rc == MG_OK; ++i) {
+    const uint32_t n = 16 * (i < 8 ? i + 1 : i - 7);
     rc = encode_map(i < 8 ? &m.t[i] : &m.t2[i - 8], p.a, false, 3, {WL_K, rows, steps}, {2 * K, 2 * WL_K},
                     {WL_K, n, i < 8 ? static_cast<uint32_t>(steps_per_stage<FP8>(n)) : 1u});
   }
