@@ -525,8 +525,7 @@ int mg_last_launch_count(mg_handle h, int32_t* launches);
 /* MG_OPT_SHARED_EARLY: 1 = mg_moe_forward runs the shared expert's two GEMMs on a library
  * stream beside the top-k, plan and scatter kernels (ordered after the router GEMM by an event,
  * joined before the combine); 0 = on the caller's stream after the routed experts; 2 (default) = 1 for
- * calls of at most 4096 tokens, where the kernels are short enough to gain from running side by
- * side, else 0.  When the shared expert runs early the
+ * calls of at most 16384 tokens (4096 while stage times are recorded), else 0.  When the shared expert runs early the
  * stage times of the shared expert (mg_stage_times) read as the wait at the join, not as its GEMMs. */
 #define MG_OPT_SHARED_EARLY 6
 /* MG_OPT_KEEP_DEQUANT: 1 = in pre-dequantise mode, a call may reuse the bf16 copy the previous

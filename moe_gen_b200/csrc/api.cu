@@ -847,9 +847,12 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   mark(h, MG_STAGE_GATE_LOGITS, st);
   // The shared expert needs only x: its GEMMs (tensor-bound) run on a second stream beside the
   // top-k, plan and scatter kernels (HBM- and latency-bound) instead of after the routed experts.
-  // pays only while the kernels are short (measured: V2-Lite at 2048 tokens 0.428 -> 0.383 ms; at
-  // 32768 / 65536 tokens of V2-236B / V3 the step got 1-2 % slower), hence the automatic setting
-  const bool shared_early = d.inter_shared && (h->opt_shared_early == 1 || (h->opt_shared_early == 2 && T <= 4096));
+  // Layer, ms, after the experts and so: V2-Lite 1024 tokens 0.304 and 0.280, 2048 0.414 and 0.385, 6000 0.867 and 0.847,
+  // 12000 1.572 and 1.541, 16384 2.175 and 2.159; V2-236B 2048 1.59 and 1.61, 6000 2.61 and 2.55, 12000 4.67 and 4.64, 32768
+  // 11.70 and 11.71; V3 8192 6.37 and 6.34, 16384 11.83 and 11.85, 65536 43.46 and 43.57.  While stage times are recorded,
+  // long kernels keep a time of their own.
+  const bool shared_early = d.inter_shared && (h->opt_shared_early == 1 ||
+                                               (h->opt_shared_early == 2 && T <= (h->stage_timing ? 4096 : 16384)));
   if (shared_early) {
     if (!h->side2) {
       MG_CUDA(cudaStreamCreateWithFlags(&h->side2, cudaStreamNonBlocking));
