@@ -881,11 +881,15 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   if (rc != MG_OK) return rc;
   h->chain = chain;
   mark(h, MG_STAGE_ROUTE_TOPK, st);
-  rc = launch_permute_plan(h, idx, T, 0, d.n_experts, counts, offsets, pad, dst, plan, st, &launches,
-                           reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]));
-  if (rc != MG_OK) return rc;
-  mark(h, MG_STAGE_PERMUTE_PLAN, st);
-  rc = launch_permute_rows(h, d_x, dst, T, perm, st);
+  int32_t* jobs = reinterpret_cast<int32_t*>(ws + L.off[WS_JOBS]);
+  if (plan_copies(h, T) && !h->stage_timing) {      // while stage times are recorded each has its own
+    rc = launch_plan_and_rows(h, idx, T, counts, offsets, pad, dst, jobs, d_x, perm, st);
+  } else {
+    rc = launch_permute_plan(h, idx, T, 0, d.n_experts, counts, offsets, pad, dst, plan, st, &launches, jobs);
+    if (rc != MG_OK) return rc;
+    mark(h, MG_STAGE_PERMUTE_PLAN, st);
+    rc = launch_permute_rows(h, d_x, dst, T, perm, st);
+  }
   if (rc != MG_OK) return rc;
   mark(h, MG_STAGE_PERMUTE_ROWS, st);
   launches += 1;

@@ -183,6 +183,9 @@ size_t plan_ws_bytes(const Handle* h, int64_t T);
 int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expert_lo, int n_exp,
                         int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,
                         void* ws, cudaStream_t st, int* launches, int32_t* job_counters = nullptr);
+bool plan_copies(const Handle* h, int64_t T);      // the forward's plan and scatter are one launch, launch_plan_and_rows
+int launch_plan_and_rows(const Handle* h, const int32_t* idx, int64_t T, int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
+                         int32_t* dst_row, int32_t* job_counters, const void* x, void* perm_x, cudaStream_t st);
 int launch_permute_plan_static(const Handle* h, const int32_t* idx, int64_t T, int expert_lo, int n_exp,
                                int32_t* counts, int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row,
                                cudaStream_t st);

@@ -929,6 +929,29 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
   }
 }
 
+// vectors [v, v_end) of a row, read once, to every destination row; lane j holds pick j's row (negative: none)
+__device__ __forceinline__ void copy_row(const uint4* src, uint4* rows, int32_t my_dst, int k, int v, int v_end, int vec_per_row,
+                                         int lane) {
+  for (int v0 = v; v0 < v_end; v0 += 128) {
+    uint4 val[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      int v = v0 + u * 32 + lane;
+      if (v < v_end) val[u] = __ldg(src + v);
+    }
+    for (int j = 0; j < k; ++j) {
+      const int32_t d = __shfl_sync(0xFFFFFFFFu, my_dst, j);
+      if (d < 0) continue;
+      uint4* dst = rows + static_cast<int64_t>(d) * vec_per_row;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        int v = v0 + u * 32 + lane;
+        if (v < v_end) dst[v] = val[u];
+      }
+    }
+  }
+}
+
 // The whole plan in one block, for batches of up to kPlanSmallTokens tokens: a bitmap per (32 tokens, expert) gives
 // the counts and the stable ranks, one block scan the offsets.  Same results as the four kernels above, which cost a
 // launch each: 20 -> 8 us at 8 tokens, 23 -> 10 us at 512.  The limit is one token per thread of the block.
@@ -939,9 +962,17 @@ __host__ __device__ constexpr int plan_small_runs(int T) { return (T + kPlanToke
 constexpr size_t plan_small_smem(int T, int n) {
   return static_cast<size_t>(2 * ((T + 31) / 32) + plan_small_runs(T)) * n * sizeof(int32_t);
 }
+// COPY: the scatter as well.  Every block makes the plan for itself, the first one stores it, and all of them copy rows (a warp
+// per token or slice of one): one launch and one trip through memory less (plan_copies).
+struct PlanCopy {
+  const uint4* x;
+  uint4* rows;
+  int vec_per_row, slices, v_chunk;
+};
+template <bool COPY>
 __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, int T, int k, int lo, int n,
                                                           int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
-                                                          int32_t* dst_row, int32_t* job_counters) {
+                                                          int32_t* dst_row, int32_t* job_counters, PlanCopy copy, Guard guard) {
   chain_wait();
   chain_go();
   extern __shared__ int32_t sm[];
@@ -952,7 +983,8 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, in
   int32_t* again = wbase + W * n;                  // [plan_small_runs(T)][n] repeated picks of e
   constexpr int RUN_W = kPlanTokens / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (job_counters != nullptr && tid < kJobCounters) job_counters[tid] = 0;
+  const bool stores = !COPY || blockIdx.x == 0;
+  if (stores && job_counters != nullptr && tid < kJobCounters) job_counters[tid] = 0;
   for (int i = tid; i < W * n; i += blockDim.x) bm[i] = 0u;
   for (int i = tid; i < plan_small_runs(T) * n; i += blockDim.x) again[i] = 0;
   __syncthreads();
@@ -985,36 +1017,82 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, in
     int32_t bo = 0, bp = 0;
     for (int i = 0; i < warp; ++i) { bo += warp_o[i]; bp += warp_p[i]; }
     const int32_t first = bp + ip - cp;
-    counts[tid] = c;
-    offsets[tid] = bo + io - c;
-    pad_offsets[tid] = first;
-    if (tid == n - 1) { offsets[n] = bo + io; pad_offsets[n] = bp + ip; }
+    if (stores) {
+      counts[tid] = c;
+      offsets[tid] = bo + io - c;
+      pad_offsets[tid] = first;
+      if (tid == n - 1) { offsets[n] = bo + io; pad_offsets[n] = bp + ip; }
+    }
     for (int w = 0; w < W; ++w) wbase[w * n + tid] += first;
   }
   __syncthreads();
-  if (tid < T) {
+  if (stores && tid < T) {
     const uint32_t lt = (1u << lane) - 1u;
     for_each_pick(idx + tid * k, k, [&](int j, int32_t pick) {
       const int e = pick - lo;
       dst_row[tid * k + j] = e >= 0 && e < n ? wbase[warp * n + e] + __popc(bm[warp * n + e] & lt) : -1;
     });
   }
+  if constexpr (COPY) {
+    const int item = blockIdx.x * (blockDim.x >> 5) + warp;
+    const int t = item / copy.slices, v = (item - t * copy.slices) * copy.v_chunk;
+    if (t >= T) return;
+    const int e = lane < k ? idx[t * k + lane] - lo : -1, at = (t >> 5) * n + e;
+    int32_t dst = e >= 0 && e < n ? wbase[at] + __popc(bm[at] & ((1u << (t & 31)) - 1u)) : -1;
+    if (dst >= 0 && !MG_GUARD(dst < guard.rows_bound, guard, 103)) dst = -1;
+    copy_row(copy.x + static_cast<int64_t>(t) * copy.vec_per_row, copy.rows, dst, k, v, min(copy.vec_per_row, v + copy.v_chunk),
+             copy.vec_per_row, lane);
+  }
 }
 
+// slices a token's row is cut into by the scatter: of at least 128 vectors, while there are fewer than 16 warps per SM
+struct RowSlices { int n, v_chunk; };
+static RowSlices row_slices(const Handle* h, int64_t T) {
+  const int vpr = h->d.hidden / 8, steps = (vpr + 127) / 128;
+  int64_t want = (static_cast<int64_t>(h->sm_count) * 16 + T - 1) / T;
+  if (want > steps) want = steps;
+  const int v_chunk = static_cast<int>((steps + want - 1) / want) * 128;
+  return {(vpr + v_chunk - 1) / v_chunk, v_chunk};
+}
+
+// x == nullptr: the plan alone
 static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo, int n, int32_t* counts,
                              int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row, int32_t* job_counters,
-                             cudaStream_t st) {
+                             const void* x, void* perm_x, cudaStream_t st) {
   const size_t smem = plan_small_smem(T, n);
-  static bool done[64];
-  if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[h->device])) {
-    MG_CUDA(cudaFuncSetAttribute(plan_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  static bool done[2][64];
+  if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[x != nullptr][h->device])) {
+    MG_CUDA(cudaFuncSetAttribute(x != nullptr ? plan_small_kernel<true> : plan_small_kernel<false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(plan_small_smem(kPlanSmallTokens, kMaxExperts))));
-    if (h->device >= 0 && h->device < 64) done[h->device] = true;
+    if (h->device >= 0 && h->device < 64) done[x != nullptr][h->device] = true;
   }
-  const int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;
-  MG_CUDA(launch_chained(h, plan_small_kernel, 1, threads, smem, st, idx, T, h->d.top_k, lo, n, counts, offsets, pad_offsets,
-                         dst_row, job_counters));
+  int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;
+  const Guard guard{h->d_status, h->guard_rows, 1};
+  if (x == nullptr) {
+    MG_CUDA(launch_chained(h, plan_small_kernel<false>, 1, threads, smem, st, idx, T, h->d.top_k, lo, n, counts, offsets,
+                           pad_offsets, dst_row, job_counters, PlanCopy{}, guard));
+    return MG_OK;
+  }
+  if (threads < 256) threads = 256;
+  const RowSlices rs = row_slices(h, T);
+  const int warps = threads / 32;
+  MG_CUDA(launch_chained(h, plan_small_kernel<true>, (T * rs.n + warps - 1) / warps, threads, smem, st, idx, T, h->d.top_k, lo, n,
+                         counts, offsets, pad_offsets, dst_row, job_counters,
+                         PlanCopy{static_cast<const uint4*>(x), static_cast<uint4*>(perm_x), h->d.hidden / 8, rs.n, rs.v_chunk},
+                         guard));
   return MG_OK;
+}
+
+// From some 200 tokens on every block's own plan costs more than the launch it saves, and a single short row gains nothing
+// either.  Layer, us, two launches and one: V2-Lite 1 token 67.8 and 68.3, 8 140 and 138.7, 64 210 and 207.8, 256 220.3 and
+// 221.6; Mixtral 61 tokens 470.5 and 465; V2-236B 8 tokens 343.6 and 341, 128 1159 and 1157, 512 1223 and 1230; V3 1 token
+// 147.8 and 144.8.
+bool plan_copies(const Handle* h, int64_t T) { return T > 0 && T <= 128 && T * h->d.hidden >= 4096; }
+int launch_plan_and_rows(const Handle* h, const int32_t* idx, int64_t T, int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
+                         int32_t* dst_row, int32_t* job_counters, const void* x, void* perm_x, cudaStream_t st) {
+  return launch_plan_small(h, idx, static_cast<int>(T), 0, h->d.n_experts, counts, offsets, pad_offsets, dst_row, job_counters, x,
+                           perm_x, st);
 }
 
 size_t plan_ws_bytes(const Handle* h, int64_t T) {
@@ -1031,7 +1109,7 @@ int launch_permute_plan(const Handle* h, const int32_t* idx, int64_t T, int expe
   if (T > 0 && T <= kPlanSmallTokens) {
     if (launches) *launches += 1;
     return launch_plan_small(h, idx, static_cast<int>(T), expert_lo, n_exp, counts, offsets, pad_offsets, dst_row,
-                             job_counters, st);
+                             job_counters, nullptr, nullptr, st);
   }
   int nblk = static_cast<int>((T + kPlanTokens - 1) / kPlanTokens);
   int32_t* bc = static_cast<int32_t*>(ws);
@@ -1199,15 +1277,13 @@ __global__ void __launch_bounds__(256) fill_duplicate_rows_kernel(uint4* __restr
 int launch_permute_rows(const Handle* h, const void* x, const int32_t* dst_row, int64_t T,
                         void* perm_x, cudaStream_t st) {
   if (T == 0) return MG_OK;
-  const int warps = 8, vpr = h->d.hidden / 8, steps = (vpr + 127) / 128;
-  int64_t want = (static_cast<int64_t>(h->sm_count) * 16 + T - 1) / T;
-  if (want > steps) want = steps;
-  const int v_chunk = static_cast<int>((steps + want - 1) / want) * 128, slices = (vpr + v_chunk - 1) / v_chunk;
-  dim3 grid(static_cast<unsigned>((T * slices + warps - 1) / warps)), block(warps * 32);
+  const int warps = 8;
+  const RowSlices rs = row_slices(h, T);
+  dim3 grid(static_cast<unsigned>((T * rs.n + warps - 1) / warps)), block(warps * 32);
   PeerPtrs bufs{};
   bufs.p[0] = perm_x;
   MG_CUDA(launch_chained(h, permute_rows_kernel<false, false, false>, grid, block, 0, st, static_cast<const uint4*>(x), dst_row,
-                         T, h->d.top_k, vpr, slices, v_chunk, bufs, bufs, bufs, 0, Guard{h->d_status, h->guard_rows, 1}));
+                         T, h->d.top_k, h->d.hidden / 8, rs.n, rs.v_chunk, bufs, bufs, bufs, 0, Guard{h->d_status, h->guard_rows, 1}));
   return MG_OK;
 }
 

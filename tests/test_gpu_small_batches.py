@@ -1,5 +1,7 @@
-"""GPU: kernels whose split of the work depends on how few tokens there are: the scatter's slices of a row, and the router
-product of few experts in narrow tiles."""
+"""GPU: kernels whose split of the work depends on how few tokens there are: the scatter's slices of a row, the plan and the
+scatter in one launch, and the router product of few experts in narrow tiles."""
+import ctypes as C
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -51,3 +53,42 @@ def test_router_product_of_few_experts(built_lib, n_experts, T, gating):
     if gating == 3:
         err = err + 2.0 ** -8 * (ref.abs() + err)
     assert bool(((got.double() - ref).abs() <= err).all())
+
+
+@pytest.mark.parametrize("hidden", [1280, 2304, 4096])                   # 160, 288 and 512 vectors
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 31, 33, 64, 65, 127, 128, 129])
+@pytest.mark.parametrize("n_experts", [8, 260])
+def test_plan_and_scatter_in_one_launch(built_lib, hidden, T, n_experts):
+    """Up to 128 tokens, from 4096 elements on, the forward plans and scatters in one launch: its tables, its rows and its
+    result are those of the stages."""
+    k = 3
+    layer = _layer(hidden, n_experts, k)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    layer.set_router(torch.randn(n_experts, hidden, generator=g, device="cuda") * 0.02)
+    for e in range(n_experts):
+        layer.load_expert(e, *((torch.randn(*s, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+                               for s in ((128, hidden), (128, hidden), (hidden, 128))))
+    x = torch.randn(T, hidden, generator=g, device="cuda").to(torch.bfloat16)
+    logits = torch.randn(T, n_experts, generator=g, device="cuda")
+    idx, w = layer.route_topk(logits)
+    plan = layer.permute_plan(idx)
+    counts, offsets, pad, dst = plan
+    rows = layer.permute_rows(x, dst, layer.padded_rows(T * k))
+    want = layer.combine(layer.expert_ffn(rows, pad, counts)[1], dst, idx, w, None)
+    ws = layer._workspace(T)
+    ws.fill_(0xff)
+    got = layer.forward_from_logits(x, logits)
+    torch.cuda.synchronize()
+    assert layer.device_status() == (0, 0)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+    def section(which, like):
+        p = C.c_void_p()
+        assert layer.lib.mg_workspace_ptr(layer._h, ws.data_ptr(), T, 0, which, C.byref(p)) == 0
+        at = p.value - ws.data_ptr()
+        return ws[at:at + like.numel() * like.element_size()].view(like.dtype).view(like.shape)
+
+    for which, t in zip((3, 4, 5, 6), plan):
+        assert torch.equal(section(which, t), t), which
+    live = dst.flatten().long()
+    assert torch.equal(section(7, rows)[live].view(torch.int16), rows[live].view(torch.int16))
