@@ -57,7 +57,7 @@ struct WlMaps {
   CUtensorMap w;                // FP8: weights [blocks of 128 rows][128][K]; bf16: [8][blocks][16][K]
   CUtensorMap t[8];             // 16 .. 128 tokens
   CUtensorMap t8;               // 8 tokens: jobs of up to 32 leave out groups of eight without a live one
-  CUtensorMap t2[6];            // 16 .. 96 tokens, one step: the parts of a job of more than 256
+  CUtensorMap t2[5];            // 16 .. 80 tokens, one step: the parts of a job of more than 256
   CUtensorMap c;                // output pieces
 };
 struct WlMapCache {

@@ -127,13 +127,13 @@ __host__ __device__ constexpr int steps_per_stage(int h) {
   return fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
 }
 
-// Tokens of a job's first MMA per K step; the second takes the rest.  Two MMAs of about one width, multiples of 32: an MMA of
-// few tokens with A in shared memory is bound by reading A (M256 K16, cycles at N = 32, 64, 96, 128: 39, 43, 50, 64, where
-// the flop rate is N / 2), so that 256 + 32 tokens took 167 cycles, where 160 + 128 take 144.
-// V2-236B (320 tokens per job), layer, ms, 256 + rest and this: 32768 tokens 11.51 and 11.36, 8192 tokens 3.31 and 3.26.
-// FP8 weights come from tensor memory, where an MMA takes N / 2 at any width: as wide as it goes, then the rest.
+// Tokens of a job's first MMA per K step; the second takes the rest.  256, but 160 where 32 or 64 would be left: an MMA of few
+// tokens with A in shared memory is bound by reading A (M256 K16, cycles at N = 32, 64, 96, 128: 39, 43, 50, 64, where the
+// flop rate is N / 2), so that 256 + 32 tokens took 167 cycles, where 160 + 128 take 144.  V2-236B (320 tokens per job), layer,
+// ms, 256 + rest and this: 32768 tokens 11.51 and 11.36, 8192 tokens 3.35 and 3.31.
+// FP8 weights come from tensor memory, where an MMA takes N / 2 at any width.
 template <bool FP8>
-__device__ __forceinline__ int first_part(int n_tok) { return n_tok <= 256 ? n_tok : FP8 ? 256 : ((n_tok >> 1) + 31) & ~31; }
+__device__ __forceinline__ int first_part(int n_tok) { return n_tok <= 256 ? n_tok : FP8 || n_tok >= 352 ? 256 : 160; }
 
 // s_jp[e] = token tiles of the experts before e
 __device__ __forceinline__ Job locate_job(int job, const int* s_pad, const int* s_cnt, const int* s_jp, const WlArgs& g) {
@@ -720,7 +720,7 @@ int wl_maps(const Handle* h, const GemmProblem& p, bool swiglu, const WlMaps** o
   int rc = FP8 ? encode_map(&m.w, p.b, true, 3, {K, 128, blocks}, {K, 128 * K}, {128, 128 / both, both})
                : encode_map(&m.w, p.b, false, 4, {K, 16, blocks, 8}, {2 * K, 256 * K, 32 * K}, {WL_K, 16, both, 8 / both});
   const uint64_t rows = static_cast<uint64_t>(p.a_rows), steps = K / WL_K;
-  for (int i = 0; i < 14 && rc == MG_OK; ++i) {
+  for (int i = 0; i < 13 && rc == MG_OK; ++i) {
     const uint32_t n = 16 * (i < 8 ? i + 1 : i - 7);
     rc = encode_map(i < 8 ? &m.t[i] : &m.t2[i - 8], p.a, false, 3, {WL_K, rows, steps}, {2 * K, 2 * WL_K},
                     {WL_K, n, i < 8 ? static_cast<uint32_t>(steps_per_stage<FP8>(n)) : 1u});
