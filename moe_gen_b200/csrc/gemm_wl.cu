@@ -305,8 +305,6 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
       }
     }
   };
-  if (g.chained)
-    for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) s_cnt[i] = min(max(peek(g.counts + i), 0), 1 << 16);
   if (warp == 3) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
                  : "memory");
@@ -314,13 +312,20 @@ grouped_gemm_wl_kernel(const __grid_constant__ WlMaps maps, const WlArgs g) {
   }
   tc_fence_before();
   __syncthreads();
-  if (g.chained && warp == 3) { count_tiles(); __syncwarp(); }
   cluster_sync_all();      // barriers of both CTAs initialised, TMEM allocated on both SMs
   tc_fence_after();
-  // Until the wait, nothing that an earlier kernel of the forward wrote is known to be visible.  The counts seen before it
-  // say which weights this pair will most likely read first, and these are brought into L2 meanwhile; whatever the counts
-  // hold, the job they give is one of the layer's.  Layer, us, without this, with 4, 8 and 16 stages: V2-Lite 8 tokens 152,
-  // 144.4, 144.2 and 144.8, 64 tokens 226, 218, 217.7 and 217; V2-236B 8 tokens 393, 378, 377 and 379.
+  // Until the wait, nothing that an earlier kernel of the forward wrote is known to be visible.  The counts seen just before it
+  // (last of all here: the plan may still be storing them when this kernel begins) say which weights this pair will most likely
+  // read first, and these are brought into L2 meanwhile; whatever the counts hold, the job they give is one of the layer's.
+  // Layer, us, routing changing from call to call, without this, with 4, 8 and 16 stages: V2-Lite 8 tokens 137.7, 136.5, 136.5
+  // and 137.0, 512 tokens 257, 237, 237 and 239; Mixtral 61 tokens 469, 465, 465 and 465; V2-236B 512 tokens 1241, 1228, 1225
+  // and 1228; V3, where converting bounds it, 8 tokens 591, 595, 595 and 596, 64 tokens 2124, 2143, 2149 and 2143.
+  if (g.chained) {
+    for (int i = threadIdx.x; i < g.n_groups; i += blockDim.x) s_cnt[i] = min(max(peek(g.counts + i), 0), 1 << 16);
+    __syncthreads();
+    if (warp == 3) count_tiles();
+    __syncthreads();
+  }
   if (g.chained && warp == 0 && pair < s_jp[g.n_groups] * g.n_tiles && elect_one()) {
     const int blk = locate_job(pair, s_cnt, s_cnt, s_jp, g).b_row >> 7, r0 = static_cast<int>(rank);
     const int steps = min(g.k_steps / (FP8 ? 2 : 1), WL_AHEAD);

@@ -963,7 +963,10 @@ constexpr size_t plan_small_smem(int T, int n) {
   return static_cast<size_t>(2 * ((T + 31) / 32) + plan_small_runs(T)) * n * sizeof(int32_t);
 }
 // COPY: the scatter as well.  Every block makes the plan for itself, the first one stores it, and all of them copy rows (a warp
-// per token or slice of one): one launch and one trip through memory less (plan_copies).
+// per token or slice of one): one launch and one trip through memory less (plan_copies).  The GEMM behind it peeks at the counts
+// while it sets itself up, so the block that stores them lets it go when they are in shared memory: let go at the top, as by the
+// other blocks, that peek found an earlier call's counts in half of the blocks or more where calls differ (V3 8 tokens, both
+// products: 70 % of the blocks; so none of 48 calls).
 struct PlanCopy {
   const uint4* x;
   uint4* rows;
@@ -974,7 +977,8 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, in
                                                           int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
                                                           int32_t* dst_row, int32_t* job_counters, PlanCopy copy, Guard guard) {
   chain_wait();
-  chain_go();
+  const bool stores = !COPY || blockIdx.x == 0;
+  if (!COPY || !stores) chain_go();
   extern __shared__ int32_t sm[];
   __shared__ int32_t warp_o[32], warp_p[32];
   const int W = (T + 31) >> 5;
@@ -983,7 +987,6 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, in
   int32_t* again = wbase + W * n;                  // [plan_small_runs(T)][n] repeated picks of e
   constexpr int RUN_W = kPlanTokens / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool stores = !COPY || blockIdx.x == 0;
   if (stores && job_counters != nullptr && tid < kJobCounters) job_counters[tid] = 0;
   for (int i = tid; i < W * n; i += blockDim.x) bm[i] = 0u;
   for (int i = tid; i < plan_small_runs(T) * n; i += blockDim.x) again[i] = 0;
@@ -996,6 +999,7 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, in
     });
   }
   __syncthreads();
+  if (COPY && stores) chain_go();
   int32_t c = 0;
   if (tid < n) {
     for (int w = 0; w < W; ++w) {
@@ -1084,10 +1088,10 @@ static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo,
   return MG_OK;
 }
 
-// From some 200 tokens on every block's own plan costs more than the launch it saves, and a single short row gains nothing
-// either.  Layer, us, two launches and one: V2-Lite 1 token 67.8 and 68.3, 8 140 and 138.7, 64 210 and 207.8, 256 220.3 and
-// 221.6; Mixtral 61 tokens 470.5 and 465; V2-236B 8 tokens 343.6 and 341, 128 1159 and 1157, 512 1223 and 1230; V3 1 token
-// 147.8 and 144.8.
+// From some 200 tokens on every block's own plan costs as much as the launch it saves or more, and a single short row gains
+// nothing either.  Layer, us, two launches and one, routing changing from call to call: V2-Lite 1 token 68.7 and 70.1, 2 83.8 and
+// 81.3, 8 135.5 and 133.7, 64 210.9 and 208.8, 128 213.6 and 212.0, 256 219.1 and 219.3; Mixtral 1 token 161.0 and 155.9, 61 468.8
+// and 467.7; V2-236B 8 tokens 359 and 357, 128 1170 and 1171, 512 1230 and 1239; V3 1 token 149.7 and 146.5, 256 2562 and 2570.
 bool plan_copies(const Handle* h, int64_t T) { return T > 0 && T <= 128 && T * h->d.hidden >= 4096; }
 int launch_plan_and_rows(const Handle* h, const int32_t* idx, int64_t T, int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
                          int32_t* dst_row, int32_t* job_counters, const void* x, void* perm_x, cudaStream_t st) {

@@ -82,3 +82,16 @@ def test_every_thread_waits_before_it_reads_memory(name):
     used = [p for p in pointers if re.search(rf"\b{p}\b", before)]
     used += re.findall(r"\bg\.(?:pad_offsets|counts|next_job|scales|out)\b", before)
     assert not used, f"{name}: {used} before the wait"
+
+
+def test_the_plan_that_copies_lets_the_gemm_go_behind_its_counting():
+    """Where the plan copies the rows too, the weight-lane GEMM comes straight behind it, begins as soon as every block has let it
+    go, and peeks at the counts: the block that stores them lets it go when it has counted, and the peek comes last in the GEMM's
+    own preparation, so that it shows this call's counts and not what an earlier call left there."""
+    _, body = KERNELS["plan_small_kernel"]
+    assert re.findall(r"([^\n;]*)chain_go\(\)", body) == ["  if (!COPY || !stores) ", "  if (COPY && stores) "]
+    assert "stores = !COPY || blockIdx.x == 0" in body[:body.index("chain_go()")]
+    counted = body[body.index("atomicOr(&bm"):body.rindex("chain_go()")]
+    assert "__syncthreads();" in counted and "counts[tid] =" not in counted
+    _, body = KERNELS["grouped_gemm_wl_kernel"]
+    assert body.index("tcgen05.alloc") < body.index("cluster_sync_all()") < body.index("peek(") < body.index("chain_wait()")
