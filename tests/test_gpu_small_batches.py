@@ -9,15 +9,19 @@ import torch.nn.functional as F
 pytestmark = pytest.mark.gpu
 
 
+def _sm_count():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
 def _layer(hidden, n_experts, top_k, gating=0):
     from moe_gen_b200 import MoELayer
     return MoELayer(hidden=hidden, inter=128, n_experts=n_experts, top_k=top_k, gating=gating, device="cuda:0")
 
 
 @pytest.mark.parametrize("hidden", [256, 1024, 1280, 2304, 7168])       # 32 to 896 vectors, slices of 128 with and without a rest
-@pytest.mark.parametrize("T", [1, 2, 7, 64, 333, 2367, 2369])           # 2368 = 16 warps on each of 148 SMs: one slice from there on
-def test_scatter_copies_whole_rows(built_lib, hidden, T):
-    k = 3
+@pytest.mark.parametrize("per_sm,T", [(0, 1), (0, 2), (0, 7), (0, 64), (0, 333), (16, -1), (16, 1)])     # 16 warps per SM: one slice from there on
+def test_scatter_copies_whole_rows(built_lib, hidden, per_sm, T):
+    k, T = 3, T + per_sm * _sm_count()
     layer = _layer(hidden, 16, k)
     g = torch.Generator(device="cuda").manual_seed(T)
     x = torch.randn(T, hidden, generator=g, device="cuda").to(torch.bfloat16)
@@ -38,7 +42,7 @@ def test_scatter_copies_whole_rows(built_lib, hidden, T):
 def test_router_product_of_few_experts(built_lib, n_experts, T, gating):
     """The same bits whatever the tile: those of a call of so many tokens that no wave of narrow tiles takes them.  And within
     fp32 sums of H products (truncated partial sums: H / 16 steps of 2^-23 of the terms' magnitude), or one bf16 rounding."""
-    H, many = 512, 148 * 128 + 1
+    H, many = 512, _sm_count() * 128 + 1
     layer = _layer(H, n_experts, 2, gating)
     g = torch.Generator(device="cuda").manual_seed(n_experts)
     w = (torch.randn(n_experts, H, generator=g, device="cuda") * 0.05).to(torch.bfloat16).float()
