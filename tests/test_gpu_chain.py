@@ -15,11 +15,11 @@ SPECS = {
 }
 
 
-@pytest.mark.parametrize("T", [1, 60, 1024, 1100, 5000])
+@pytest.mark.parametrize("T", [1, 60, 1024, 1100, 5000, 16500])
 @pytest.mark.parametrize("name", sorted(SPECS))
 def test_back_to_back_forwards_equal_single_launches(built_lib, name, T):
-    """Up to 1024 tokens the plan is one kernel, above four; the shared expert joins from its own stream up to 4096
-    tokens and follows in the same stream above."""
+    """Up to 128 tokens plan and scatter are one kernel, up to 1024 the plan, above it is four; the shared expert joins from
+    its own stream up to 16384 tokens and follows in the same stream above, where every kernel behind the first is chained."""
     x, W = O.make_inputs(SPECS[name], T, 70 + T)
     layer = make_layer(SPECS[name], W)
     xs = [x.cuda(), x.flip(0).contiguous().cuda(), (x * 0.5).cuda()]
