@@ -847,10 +847,11 @@ static int moe_forward_impl(mg_handle hh, const void* d_x, int64_t T, const void
   mark(h, MG_STAGE_GATE_LOGITS, st);
   // The shared expert needs only x: its GEMMs (tensor-bound) run on a second stream beside the
   // top-k, plan and scatter kernels (HBM- and latency-bound) instead of after the routed experts.
-  // Layer, ms, after the experts and so: V2-Lite 1024 tokens 0.304 and 0.280, 2048 0.414 and 0.385, 6000 0.867 and 0.847,
-  // 12000 1.572 and 1.541, 16384 2.175 and 2.159; V2-236B 2048 1.59 and 1.61, 6000 2.61 and 2.55, 12000 4.67 and 4.64, 32768
-  // 11.70 and 11.71; V3 8192 6.37 and 6.34, 16384 11.83 and 11.85, 65536 43.46 and 43.57.  While stage times are recorded,
-  // long kernels keep a time of their own.
+  // Layer, ms, after the experts and so: V2-Lite 512 tokens 0.259 and 0.232, 2048 0.426 and 0.382, 8192 1.16 and 1.09, 16384
+  // 2.13 and 2.07; V2-236B 512 1.270 and 1.228, 2048 1.61 and 1.57, 8192 3.33 and 3.20, 12000 4.86 and 4.80, 16384 5.92 and 5.93;
+  // V3 512 2.67 and 2.65, 8192 6.64 and 6.63, 16384 11.99 and 12.01.  So the line lies where the largest layers are level
+  // (beyond it V2-236B 32768 11.70 and 11.71, V3 65536 43.46 and 43.57).  While stage times are recorded, long kernels keep a
+  // time of their own.
   const bool shared_early = d.inter_shared && (h->opt_shared_early == 1 ||
                                                (h->opt_shared_early == 2 && T <= (h->stage_timing ? 4096 : 16384)));
   if (shared_early) {

@@ -480,6 +480,27 @@ def test_shared_expert_beside_the_routing_kernels_equals_after_the_experts(built
         assert torch.equal(ys[0].view(torch.int16), y.view(torch.int16))
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("T", [4096, 4097, 16384, 16385])
+def test_shared_expert_on_either_side_of_the_automatic_line(built_lib, T, fp8):
+    """By itself the shared expert runs beside the routing kernels up to 16384 tokens (4096 while stage times are recorded):
+    the bits of both fixed settings, and of forwards whose stages are timed."""
+    spec = O.LayerSpec(512, 128, 16, 2, 256, 1, 1, O.GATE_SOFTMAX_GREEDY, False, 1.0,
+                       O.WEIGHT_FP8_BLOCK128 if fp8 else O.WEIGHT_BF16, O.COMBINE_BF16_PROD)
+    x, W = O.make_inputs(spec, T, 52)
+    layer = make_layer(spec, W, DEV)
+    xs = [x.to(DEV), x.flip(0).contiguous().to(DEV)]
+    ys = []
+    for mode, timed in ((0, False), (1, False), (2, False), (2, True)):
+        layer.set_option(6, mode)
+        layer.set_stage_timing(timed)
+        ys.append([layer.forward(xs[i % 2]).clone() for i in range(4)])
+        _status_ok(layer)
+    for got in ys:
+        for i, y in enumerate(got):
+            assert torch.equal(ys[0][i % 2].view(torch.int16), y.view(torch.int16)), i
+
+
 @pytest.mark.parametrize("T", [0, 1, 127, 129])
 def test_layer_edge_token_counts(built_lib, T):
     spec = O.LayerSpec(256, 128, 64, 6, 256, 1, 1, O.GATE_SOFTMAX_GREEDY, False, 1.0, O.WEIGHT_BF16,
