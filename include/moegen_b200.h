@@ -543,7 +543,10 @@ int mg_set_option(mg_handle h, int32_t option, int32_t value);
  * forward records a CUDA event on `stream` after every stage; after the caller has
  * synchronised, mg_stage_times() returns the milliseconds per MG_STAGE_* (0 for stages
  * the layer does not have), averaged over the forwards since timing was enabled (the
- * last 32 if there were more). */
+ * last 32 if there were more).  While it is enabled the forward gives the same bits by another
+ * schedule: its kernels are launched one after the other, without overlap; up to 128 tokens the plan and the
+ * scatter are two launches (else one); and the shared expert runs beside the routing kernels up to
+ * 4096 tokens by itself (else 16384, MG_OPT_SHARED_EARLY).  The stages' sum is not the time of a forward without it. */
 int mg_set_stage_timing(mg_handle h, int32_t enable);
 int mg_stage_times(mg_handle h, float* ms, int32_t n);
 

@@ -136,6 +136,7 @@ class MoELayer:
             self._hws = None
 
     def set_stage_timing(self, enable: bool):
+        """Record the stages' times; forwards then follow another schedule (mg_set_stage_timing), with the same bits."""
         L.check(self.lib.mg_set_stage_timing(self._h, int(enable)))
 
     def stage_times(self) -> dict:
