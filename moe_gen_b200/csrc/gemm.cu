@@ -34,8 +34,8 @@ constexpr int GEMM_THREADS = 192;
 constexpr int CONVERT_THREADS = 256;
 constexpr int NUM_BARS = 2 * STAGES + 4 + 2 * B_SLOTS;
 
-// NARROW: tiles of 32 columns for the router product of few tokens, which is a chain of load latencies: more CTAs
-// and a deeper ring of smaller stages.
+// NARROW: tiles of at most 32 columns for the router product while they fit one wave (few tokens, or few experts at any
+// number of tokens up to 128 per SM), which is a chain of load latencies: more CTAs and a deeper ring of smaller stages.
 constexpr int BN_NARROW = 32;
 template <bool F8B, bool NARROW = false>
 struct Cfg {

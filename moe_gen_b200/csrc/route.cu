@@ -929,23 +929,23 @@ __global__ void __launch_bounds__(kPlanTokens) plan_place_kernel(const int32_t* 
   }
 }
 
-// vectors [v, v_end) of a row, read once, to every destination row; lane j holds pick j's row (negative: none)
-__device__ __forceinline__ void copy_row(const uint4* src, uint4* rows, int32_t my_dst, int k, int v, int v_end, int vec_per_row,
-                                         int lane) {
-  for (int v0 = v; v0 < v_end; v0 += 128) {
+// vectors [v_begin, v_end) of a row, read once, to the k places row_of(pick, entry of the pick) names (nullptr: none); lane j
+// holds pick j's entry
+template <typename RowOf>
+__device__ __forceinline__ void copy_row(const uint4* src, int32_t my_dst, int k, int v_begin, int v_end, int lane, RowOf row_of) {
+  for (int v0 = v_begin; v0 < v_end; v0 += 128) {
     uint4 val[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      int v = v0 + u * 32 + lane;
+      const int v = v0 + u * 32 + lane;
       if (v < v_end) val[u] = __ldg(src + v);
     }
     for (int j = 0; j < k; ++j) {
-      const int32_t d = __shfl_sync(0xFFFFFFFFu, my_dst, j);
-      if (d < 0) continue;
-      uint4* dst = rows + static_cast<int64_t>(d) * vec_per_row;
+      uint4* dst = row_of(j, __shfl_sync(0xFFFFFFFFu, my_dst, j));
+      if (dst == nullptr) continue;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        int v = v0 + u * 32 + lane;
+        const int v = v0 + u * 32 + lane;
         if (v < v_end) dst[v] = val[u];
       }
     }
@@ -1044,12 +1044,13 @@ __global__ void __launch_bounds__(1024) plan_small_kernel(const int32_t* idx, in
     const int e = lane < k ? idx[t * k + lane] - lo : -1, at = (t >> 5) * n + e;
     int32_t dst = e >= 0 && e < n ? wbase[at] + __popc(bm[at] & ((1u << (t & 31)) - 1u)) : -1;
     if (dst >= 0 && !MG_GUARD(dst < guard.rows_bound, guard, 103)) dst = -1;
-    copy_row(copy.x + static_cast<int64_t>(t) * copy.vec_per_row, copy.rows, dst, k, v, min(copy.vec_per_row, v + copy.v_chunk),
-             copy.vec_per_row, lane);
+    copy_row(copy.x + static_cast<int64_t>(t) * copy.vec_per_row, dst, k, v, min(copy.vec_per_row, v + copy.v_chunk), lane,
+             [&](int, int32_t d) { return d < 0 ? nullptr : copy.rows + static_cast<int64_t>(d) * copy.vec_per_row; });
   }
 }
 
-// slices a token's row is cut into by the scatter: of at least 128 vectors, while there are fewer than 16 warps per SM
+// slices a token's row is cut into by the scatter while there are fewer than 16 warps per SM: 128 vectors or a multiple, the last
+// one what is left
 struct RowSlices { int n, v_chunk; };
 static RowSlices row_slices(const Handle* h, int64_t T) {
   const int vpr = h->d.hidden / 8, steps = (vpr + 127) / 128;
@@ -1059,17 +1060,19 @@ static RowSlices row_slices(const Handle* h, int64_t T) {
   return {(vpr + v_chunk - 1) / v_chunk, v_chunk};
 }
 
+constexpr int kPlanCopyTokens = 128;        // most tokens of the copying form (plan_copies)
+static_assert(plan_small_smem(kPlanCopyTokens, kMaxExperts) <= 48 * 1024, "the copying form sets no shared-memory limit");
+
 // x == nullptr: the plan alone
 static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo, int n, int32_t* counts,
                              int32_t* offsets, int32_t* pad_offsets, int32_t* dst_row, int32_t* job_counters,
                              const void* x, void* perm_x, cudaStream_t st) {
   const size_t smem = plan_small_smem(T, n);
-  static bool done[2][64];
-  if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[x != nullptr][h->device])) {
-    MG_CUDA(cudaFuncSetAttribute(x != nullptr ? plan_small_kernel<true> : plan_small_kernel<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+  static bool done[64];
+  if (smem > 48 * 1024 && !(h->device >= 0 && h->device < 64 && done[h->device])) {
+    MG_CUDA(cudaFuncSetAttribute(plan_small_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(plan_small_smem(kPlanSmallTokens, kMaxExperts))));
-    if (h->device >= 0 && h->device < 64) done[x != nullptr][h->device] = true;
+    if (h->device >= 0 && h->device < 64) done[h->device] = true;
   }
   int threads = T > n ? (T + 31) / 32 * 32 : (n + 31) / 32 * 32;
   const Guard guard{h->d_status, h->guard_rows, 1};
@@ -1092,7 +1095,7 @@ static int launch_plan_small(const Handle* h, const int32_t* idx, int T, int lo,
 // nothing either.  Layer, us, two launches and one, routing changing from call to call: V2-Lite 1 token 68.7 and 70.1, 2 83.8 and
 // 81.3, 8 135.5 and 133.7, 64 210.9 and 208.8, 128 213.6 and 212.0, 256 219.1 and 219.3; Mixtral 1 token 161.0 and 155.9, 61 468.8
 // and 467.7; V2-236B 8 tokens 359 and 357, 128 1170 and 1171, 512 1230 and 1239; V3 1 token 149.7 and 146.5, 256 2562 and 2570.
-bool plan_copies(const Handle* h, int64_t T) { return T > 0 && T <= 128 && T * h->d.hidden >= 4096; }
+bool plan_copies(const Handle* h, int64_t T) { return T > 0 && T <= kPlanCopyTokens && T * h->d.hidden >= 4096; }
 int launch_plan_and_rows(const Handle* h, const int32_t* idx, int64_t T, int32_t* counts, int32_t* offsets, int32_t* pad_offsets,
                          int32_t* dst_row, int32_t* job_counters, const void* x, void* perm_x, cudaStream_t st) {
   return launch_plan_small(h, idx, static_cast<int>(T), 0, h->d.n_experts, counts, offsets, pad_offsets, dst_row, job_counters, x,
@@ -1182,11 +1185,10 @@ int launch_permute_plan_static(const Handle* h, const int32_t* idx, int64_t T, i
 // ---------------------------------------------------------------------------------------
 // row scatter: a warp per token, or per slice of one, x row read once, written to each destination row
 // ---------------------------------------------------------------------------------------
-// Few tokens: a warp that copies 14 KB to 8 places is a chain of stores; cut into slices of at least 128 vectors while there
-// are fewer than 16 warps per SM.  Neighbouring slices share a block: where a block of this kernel runs, the GEMM behind it
-// cannot be placed early (slices of 32 vectors, a block each: V3 1 token 151 and 157 us).  Kernel, us, a warp per token and
-// this: V3 64 tokens 21 and 6, V2-236B 512 tokens 25 and 15; layer: V3 8 tokens 621 and 616, V2-236B 8 tokens 350 and 344, 512
-// tokens 1228 and 1221.
+// Few tokens: a warp that copies 14 KB to 8 places is a chain of stores; cut into slices (row_slices) while there are fewer than
+// 16 warps per SM.  Neighbouring slices share a block: where a block of this kernel runs, the GEMM behind it cannot be placed
+// early (slices of 32 vectors, a block each: V3 1 token 151 and 157 us).  Kernel, us, a warp per token and this: V3 64 tokens
+// 21 and 6, V2-236B 512 tokens 25 and 15; layer: V3 8 tokens 621 and 616, V2-236B 8 tokens 350 and 344, 512 tokens 1228 and 1221.
 // PEER: dst_row packs (destination rank << kPeerShift | row) and rows are written to that
 // rank's buffer through its peer mapping (plain stores over NVLink).
 // DEDUP: when several picks of a token go to the same rank, only the first one's row travels; for
@@ -1227,26 +1229,11 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(const uint4* __restri
       static_cast<int32_t*>(dups.p[my_dst >> kPeerShift])[my_dst & kPeerRowMask] = first_dst & kPeerRowMask;
     skip = __ballot_sync(0xFFFFFFFFu, my_first >= 0);
   }
-  const uint4* src = x + t * vec_per_row;
-  for (int v0 = v_begin; v0 < v_end; v0 += 128) {
-    uint4 val[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      int v = v0 + u * 32 + lane;
-      if (v < v_end) val[u] = __ldg(src + v);
-    }
-    for (int j = 0; j < k; ++j) {
-      int32_t d = __shfl_sync(0xFFFFFFFFu, my_dst, j);
-      if (d < 0 || ((skip >> j) & 1u)) continue;
-      uint4* dst = static_cast<uint4*>(PEER ? bufs.p[d >> kPeerShift] : bufs.p[0]) +
-                   static_cast<int64_t>(PEER ? (d & kPeerRowMask) : d) * vec_per_row;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int v = v0 + u * 32 + lane;
-        if (v < v_end) dst[v] = val[u];
-      }
-    }
-  }
+  copy_row(x + t * vec_per_row, my_dst, k, v_begin, v_end, lane, [&](int j, int32_t d) -> uint4* {
+    if (d < 0 || ((skip >> j) & 1u)) return nullptr;
+    return static_cast<uint4*>(PEER ? bufs.p[d >> kPeerShift] : bufs.p[0]) +
+           static_cast<int64_t>(PEER ? (d & kPeerRowMask) : d) * vec_per_row;
+  });
 }
 
 // Owner side of the de-duplicated dispatch: row r with dup[r] >= 0 becomes a copy of row dup[r]

@@ -19,27 +19,31 @@ def _strip(text):
     return re.sub(r"//[^\n]*", "", text)
 
 
-def _kernels():
-    """name -> (parameters, body) of every __global__ function"""
+def _functions(files, head):
+    """name -> (parameters, body) of every function whose head matches; bodies of one name together"""
     out = {}
-    for f in b.SOURCES:
+    for f in files:
         text = _strip(open(os.path.join(b.CSRC, f)).read())
-        for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\s*\(", text):
+        for m in re.finditer(head, text):
             depth, i = 1, m.end()
             while depth:
                 depth += {"(": 1, ")": -1}.get(text[i], 0)
                 i += 1
             params = text[m.end():i - 1]
             j = text.index("{", i)
+            if ";" in text[i:j]:
+                continue                  # declared here, defined elsewhere
             depth, i = 1, j + 1
             while depth:
                 depth += {"{": 1, "}": -1}.get(text[i], 0)
                 i += 1
-            out[m.group(1)] = (params, text[j + 1:i - 1])
+            old = out.get(m.group(1), ("", ""))
+            out[m.group(1)] = (old[0] + ", " * bool(old[0]) + params, old[1] + text[j + 1:i - 1])
     return out
 
 
-KERNELS = _kernels()
+KERNELS = _functions(b.SOURCES, r"__global__[^;{]*?(\w+_kernel)\s*\(")
+HELPERS = _functions(b.SOURCES + ["common.cuh", "tc.cuh"], r"__device__ __forceinline__ [^;{(]*?(\w+)\s*\(")
 CHAINED = sorted(n for n, (_, body) in KERNELS.items() if "chain_wait()" in body)
 
 
@@ -57,13 +61,19 @@ def test_every_kernel_launched_by_dependence_waits():
 @pytest.mark.parametrize("name", CHAINED)
 def test_no_read_only_path_for_what_a_predecessor_writes(name):
     """__ldg, and __restrict__ on a pointer that is only read, promise memory that nothing writes while the kernel lives:
-    the load may come from the non-coherent path and may be moved ahead of the wait."""
-    params, body = KERNELS[name]
-    for p in params.split(","):
-        if "__restrict__" in p:
-            assert p.split()[-1] in OLDER, f"{name}: {p.strip()}"
-    for m in re.finditer(r"__ldg\(", body):
-        assert body[m.end():].startswith(LDG_OLDER), f"{name}: __ldg({body[m.end():m.end() + 40]}"
+    the load may come from the non-coherent path and may be moved ahead of the wait.  The same for what the kernel calls."""
+    todo, seen = [name], {}
+    while todo:
+        f = todo.pop()
+        seen[f] = KERNELS[f] if f in KERNELS else HELPERS[f]
+        todo += [g for g in set(re.findall(r"\b(\w+)\s*(?:<[^<>;(){}]*>)?\(", seen[f][1])) if g in HELPERS and g not in seen]
+    for f, (params, body) in seen.items():
+        for p in params.split(","):
+            if "__restrict__" in p:
+                assert p.split()[-1] in OLDER, f"{f}: {p.strip()}"
+        for m in re.finditer(r"__ldg\(", body):
+            assert body[m.end():].startswith(LDG_OLDER), f"{f}: __ldg({body[m.end():m.end() + 40]}"
+    assert "copy_row" in seen or name not in ("permute_rows_kernel", "plan_small_kernel")
 
 
 @pytest.mark.parametrize("name", CHAINED)
